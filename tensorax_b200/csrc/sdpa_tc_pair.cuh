@@ -223,25 +223,26 @@ sdpa_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         if (run) {
             const bool leader = ptx::elect_one();
             bool ok = true;
-            for (int j = 0; j < n_max && ok; ++j) {
+            // Key tile 0 went out before the meeting, and nothing is waited for on its behalf: with one live query tile
+            // its QK^T can complete, and release the stage, before this warp gets here, and a wait for the barrier's
+            // initial phase would then wait for the NEXT release, which needs a tile this warp has not loaded.
+            for (int j = 1; j < n_max && ok; ++j) {
                 const int s = j % NS;
                 const uint32_t ph = (uint32_t)(j / NS) & 1u;
                 ok = ptx::mbar_wait(k_empty + 8 * s, ph ^ 1u, abort_flag, Cfg::WAIT_NS);
                 if (!ok) break;
                 const bool left_out = Cfg::FAULT_TEST && j == p.skip_k_tile;     // self-test: this tile never arrives
-                if (leader && j > 0) {                                           // key tile 0 went out before the meeting
-                    if (!left_out) {
-                        ptx::mbar_arrive_expect_tx(k_full + 8 * s, Cfg::K_BYTES);
+                if (leader && !left_out) {
+                    ptx::mbar_arrive_expect_tx(k_full + 8 * s, Cfg::K_BYTES);
 #pragma unroll
-                        for (int pn = 0; pn < Cfg::KP; ++pn)
-                            ptx::tma_load_3d(k_s + s * Cfg::K_BYTES + pn * Cfg::KV_PANEL, &tm_k, k_full + 8 * s,
-                                             pn * 64, j * BN, kvh);
-                    }
+                    for (int pn = 0; pn < Cfg::KP; ++pn)
+                        ptx::tma_load_3d(k_s + s * Cfg::K_BYTES + pn * Cfg::KV_PANEL, &tm_k, k_full + 8 * s,
+                                         pn * 64, j * BN, kvh);
                 }
                 __syncwarp();
                 ok = ptx::mbar_wait(v_empty + 8 * s, ph ^ 1u, abort_flag, Cfg::WAIT_NS);
                 if (!ok) break;
-                if (leader && j > 0) {
+                if (leader) {
                     ptx::mbar_arrive_expect_tx(v_full + 8 * s, Cfg::V_BYTES);
 #pragma unroll
                     for (int pn = 0; pn < Cfg::KP; ++pn)
