@@ -53,6 +53,8 @@ enum {
                                 tensor-core kernel where its shapes apply -- what the reference's `_mma` variant does inside
                                 its kernel (fp32 in/out, fp16 MMA operands, csrc/cuda/kernels/attn.cu:441-603); fp16
                                 tolerances then apply.  Without the flag fp32 inputs always get exact fp32 arithmetic. */
+    TX_SDPA_KV_LENS_HOST = 16, /* `kv_lens` is a HOST array, read during the call: up to 32 lengths travel with the launch,
+                                 longer arrays are copied to the device first (forward and backward descriptors) */
     TX_SDPA_P_IN_SMEM = 2    /* tensor-core kernel: stage P in shared memory instead of tensor memory
                                 (ignored for d = 512, where shared memory has no room for it) */
 };
@@ -266,7 +268,7 @@ typedef struct tx_sdpa_bwd_desc {
     float *dq, *dk, *dv;      /* fp32 [batch, q_heads, seq_q, d], [batch, kv_heads, seq_k, d] x 2 */
     int64_t batch, q_heads, kv_heads, seq_q, seq_k, d;
     int32_t causal;
-    int32_t flags;            /* TX_SDPA_OUT_F16: dtype of `out` */
+    int32_t flags;            /* TX_SDPA_OUT_F16: dtype of `out`; TX_SDPA_KV_LENS_HOST */
     void *stream;
 } tx_sdpa_bwd_desc;
 TX_API int tx_sdpa_backward(const tx_sdpa_bwd_desc *desc);

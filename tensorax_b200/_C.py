@@ -16,6 +16,7 @@ dispatchers (csrc/tensor_ops.cpp:830-1181).  What is different, on purpose:
 from __future__ import annotations
 
 import ctypes
+import math
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -37,7 +38,7 @@ class TensorImpl:
         if device not in ("cpu", "cuda"):
             raise RuntimeError(f"Unknown device: {device}")
         self._shape = [int(s) for s in shape]
-        self._size = int(np.prod(self._shape, dtype=np.int64)) if len(self._shape) else 1
+        self._size = math.prod(self._shape)
         self._dtype = dtype
         self._device = device
         self._host = host
@@ -219,6 +220,14 @@ def _validate(query, key, value, mask, who="SDPA"):
     return B, H, Hkv, Sq, Sk, dk, dv
 
 
+def _host_lens(kv_lens, B, who):
+    """The key lengths as a host array of int32, handed to the library as they are (TX_SDPA_KV_LENS_HOST)."""
+    lens = np.ascontiguousarray(kv_lens, dtype=np.int32)
+    if lens.shape != (B,):
+        raise RuntimeError(f"{who}: kv_lens must hold one length per batch element")
+    return (ctypes.c_int32 * B).from_buffer_copy(lens)
+
+
 def synchronize() -> None:
     """Wait for everything enqueued with ``sync=False`` and raise if a kernel reported a failure."""
     _lib.check(_lib.load().tx_sdpa_finish(None))
@@ -244,16 +253,14 @@ def _forward(query, key, value, mask, causal=False, kv_lens=None, flags=0, who="
     if out_dtype == "float16":
         flags = int(flags) | _lib.TX_SDPA_OUT_F16
     lse = TensorImpl([B, H, Sq], "float32", "cuda") if want_lse else None
-    lens_buf = None
+    lens = None
     if kv_lens is not None:
-        lens = np.ascontiguousarray(kv_lens, dtype=np.int32)
-        if lens.shape != (B,):
-            raise RuntimeError(f"{who}: kv_lens must hold one length per batch element")
-        lens_buf = _lib.to_device(lens)
+        lens = _host_lens(kv_lens, B, who)
+        flags = int(flags) | _lib.TX_SDPA_KV_LENS_HOST
     desc = _lib.SdpaDesc(
         q=query.data_ptr, k=key.data_ptr, v=value.data_ptr,
         mask=mask.data_ptr if mask is not None else None,
-        kv_lens=lens_buf.ptr if lens_buf is not None else None, out=out.data_ptr,
+        kv_lens=ctypes.addressof(lens) if lens is not None else None, out=out.data_ptr,
         batch=B, q_heads=H, kv_heads=Hkv, seq_q=Sq, seq_k=Sk, d_k=dk, d_v=dv,
         dtype=_lib.TX_DTYPE_F16 if f16 else _lib.TX_DTYPE_F32, causal=int(bool(causal)),
         flags=int(flags), stream=None, lse=lse.data_ptr if lse is not None else None)
@@ -261,8 +268,7 @@ def _forward(query, key, value, mask, causal=False, kv_lens=None, flags=0, who="
     _lib.check(lib.tx_sdpa_forward(ctypes.byref(desc)))
     if sync:
         _lib.check(lib.tx_sdpa_finish(None))   # the reference launchers return a finished result
-    # sync=False: the launch is stream-ordered; buffers freed meanwhile (the key lengths above) go back to
-    # the pool in stream order, so nothing is reused before the kernel has read it
+    # sync=False: the launch is stream-ordered and has taken the key lengths with it
     return (out, lse) if want_lse else out
 
 
@@ -290,17 +296,15 @@ def scaled_dot_product_attention_backward(query, key, value, out, lse, grad, cau
     dq = TensorImpl([B, H, Sq, dk], "float32", "cuda")
     dkk = TensorImpl([B, Hkv, Sk, dk], "float32", "cuda")
     dvv = TensorImpl([B, Hkv, Sk, dv], "float32", "cuda")
-    lens_buf = None
+    lens, flags = None, _lib.TX_SDPA_OUT_F16 if out.dtype == "float16" else 0
     if kv_lens is not None:
-        lens = np.ascontiguousarray(kv_lens, dtype=np.int32)
-        if lens.shape != (B,):
-            raise RuntimeError("SDPA backward: kv_lens must hold one length per batch element")
-        lens_buf = _lib.to_device(lens)
+        lens = _host_lens(kv_lens, B, "SDPA backward")
+        flags |= _lib.TX_SDPA_KV_LENS_HOST
     desc = _lib.SdpaBwdDesc(
         q=query.data_ptr, k=key.data_ptr, v=value.data_ptr, out=out.data_ptr, dout=grad.data_ptr,
-        lse=lse.data_ptr, kv_lens=lens_buf.ptr if lens_buf is not None else None,
+        lse=lse.data_ptr, kv_lens=ctypes.addressof(lens) if lens is not None else None,
         dq=dq.data_ptr, dk=dkk.data_ptr, dv=dvv.data_ptr, batch=B, q_heads=H, kv_heads=Hkv, seq_q=Sq, seq_k=Sk,
-        d=dk, causal=int(bool(causal)), flags=_lib.TX_SDPA_OUT_F16 if out.dtype == "float16" else 0, stream=None)
+        d=dk, causal=int(bool(causal)), flags=flags, stream=None)
     lib = _lib.load()
     _lib.check(lib.tx_sdpa_backward(ctypes.byref(desc)))
     _lib.check(lib.tx_sdpa_finish(None))

@@ -20,6 +20,7 @@ TX_SDPA_FORCE_SIMT = 1
 TX_SDPA_P_IN_SMEM = 2
 TX_SDPA_OUT_F16 = 4
 TX_SDPA_F32_VIA_F16 = 8
+TX_SDPA_KV_LENS_HOST = 16
 
 # every symbol include/tensorax_b200.h declares
 EXPORTED_SYMBOLS = (
@@ -135,12 +136,12 @@ class DeviceBuffer:
     ownership rule of the reference's TensorImpl (csrc/tensor_ops.cpp:64-76)."""
 
     def __init__(self, nbytes: int):
-        lib = load()
-        if not lib.tx_cuda_is_available():
-            raise BackendError("CUDA device not available: tensorax_b200 has no CPU fallback")
+        lib = _lib or load()
         self.nbytes = int(nbytes)
         self.ptr = lib.tx_cuda_malloc(self.nbytes)
         if not self.ptr:
+            if not lib.tx_cuda_is_available():
+                raise BackendError("CUDA device not available: tensorax_b200 has no CPU fallback")
             check(3)
 
     def __del__(self):

@@ -1,0 +1,25 @@
+// Valid keys per batch element, as a kernel parameter: a device array, or up to 32 lengths inside the parameter block
+// itself.  The second form is for callers that have the lengths on the host (a serving loop, the Python layer): they
+// travel with the launch instead of in a buffer of their own that is allocated, filled by a copy the host waits for,
+// and freed on every call.
+#pragma once
+#include <cstdint>
+
+namespace txb {
+
+struct KvLens {
+    static constexpr int kInline = 32;
+    const int32_t *ptr = nullptr;      // optional device array [B]
+    int32_t n_inline = 0;              // B when the lengths are in `val`
+    int32_t val[kInline];
+
+    // `all`, or the batch element's length where one was given and is smaller (a negative one counts as 0)
+    __device__ __forceinline__ int limit(int b, int all) const
+    {
+        if (n_inline > 0) return min(all, max(val[b], 0));
+        if (ptr) return min(all, max(ptr[b], 0));
+        return all;
+    }
+};
+
+}  // namespace txb

@@ -106,7 +106,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
                 }
                 __syncwarp();
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, LTC_ERR_PRODUCER); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, LTC_ERR_PRODUCER); }
         }
     } else if (warp == 1) {
         if (run) {
@@ -140,7 +140,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
                 }
                 __syncwarp();
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, LTC_ERR_MMA); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, LTC_ERR_MMA); }
         }
     } else {
         const int t = tid - 64;                       // 0..127
@@ -212,7 +212,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
                 }
             }
         }
-        if (run && !ok) { *abort_flag = 1; atomicCAS(p.status, 0, LTC_ERR_SPLIT); }
+        if (run && !ok) { *abort_flag = 1; ptx::report(p.status, LTC_ERR_SPLIT); }
     }
 
     ptx::tc_fence_before_sync();

@@ -8,6 +8,8 @@
 #include <cuda_fp16.h>
 #include <cstdint>
 
+#include "kv_lens.cuh"
+
 #include "bounded_wait.h"
 
 namespace txb {
@@ -92,6 +94,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 {
     return bounded_wait([&] { return mbar_test_wait(bar, parity); }, [&] { return mbar_try_wait(bar, parity); },
                         [] { return global_timer_ns(); }, abort_flag, limit_ns);
+}
+
+// Record that a wait ran out: the first code stays in the device status word (asked by the launch's later CTAs), and
+// whoever set it also writes it to the host's mirror, whose device address is kept 8 bytes behind the word (null: none).
+// The mirror is what lets the host learn of a failure after a synchronise without a copy from the device.
+__device__ __forceinline__ void report(int *status, int code)
+{
+    if (atomicCAS(status, 0, code) == 0) {
+        volatile int *mirror = *reinterpret_cast<volatile int *volatile *>(status + 2);
+        if (mirror) {
+            *mirror = code;
+            __threadfence_system();
+        }
+    }
 }
 
 // ---------------------------------------------------------------- fences

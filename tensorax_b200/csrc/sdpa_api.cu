@@ -15,6 +15,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 // NVTX ranges around the entry points, as the reference's launchers have them
@@ -73,7 +74,17 @@ int ensure_device()
 }
 
 constexpr int kMaxDevices = 64;
+
+int current_device(int *dev)
+{
+    TX_CUDA(cudaGetDevice(dev));
+    if (*dev < 0 || *dev >= kMaxDevices) return fail(TX_ERR_INVALID, "device index %d out of range", *dev);
+    return TX_OK;
+}
+
 int pool_ready();
+void pool_took(void *ptr, size_t bytes);
+void pool_gave(void *ptr);
 
 // Workspace of one call from the device's stream-ordered pool.  pool_ready() first: with the pool's default release
 // threshold of zero every synchronisation hands the freed workspace back to the driver, and the next call pays for
@@ -82,26 +93,48 @@ int pool_alloc(char **p, size_t bytes, cudaStream_t st)
 {
     if (int rc = pool_ready()) return rc;
     TX_CUDA(cudaMallocAsync(reinterpret_cast<void **>(p), bytes, st));
+    pool_took(*p, bytes);
     return TX_OK;
 }
 
-// One status word per device, written by kernels whose bounded waits run out.
-int *g_status[kMaxDevices] = {};
+void pool_free(char *p, cudaStream_t st)
+{
+    pool_gave(p);
+    (void)cudaFreeAsync(p, st);
+}
+
+// One status word per device, written by kernels whose bounded waits run out, and its mirror in pinned host memory
+// (the device address of the mirror sits behind the word, see ptx::report): asking for it after a synchronise is a
+// load, where copying the word back was a second trip to the device on every call (7 us of a 47 us call).
+struct Status {
+    int *word = nullptr;
+    volatile int *mirror = nullptr;
+};
+Status g_status[kMaxDevices];
+std::atomic<bool> g_status_ready[kMaxDevices] = {};
 std::mutex g_status_mu;
 
 int status_word(int **out)
 {
     int dev = 0;
-    TX_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDevices) return fail(TX_ERR_INVALID, "device index %d out of range", dev);
-    std::lock_guard<std::mutex> lk(g_status_mu);
-    if (!g_status[dev]) {
-        int *w = nullptr;
-        TX_CUDA(cudaMalloc(&w, 256));
-        TX_CUDA(cudaMemset(w, 0, 256));
-        g_status[dev] = w;
+    if (int rc = current_device(&dev)) return rc;
+    if (!g_status_ready[dev].load(std::memory_order_acquire)) {
+        std::lock_guard<std::mutex> lk(g_status_mu);
+        if (!g_status_ready[dev].load(std::memory_order_relaxed)) {
+            Status s;
+            int *mirror = nullptr, *mirror_dev = nullptr;
+            TX_CUDA(cudaMalloc(&s.word, 256));
+            TX_CUDA(cudaHostAlloc(&mirror, 64, cudaHostAllocMapped));
+            *mirror = 0;
+            s.mirror = mirror;
+            TX_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&mirror_dev), mirror, 0));
+            TX_CUDA(cudaMemset(s.word, 0, 256));
+            TX_CUDA(cudaMemcpy(s.word + 2, &mirror_dev, sizeof mirror_dev, cudaMemcpyHostToDevice));
+            g_status[dev] = s;
+            g_status_ready[dev].store(true, std::memory_order_release);
+        }
     }
-    *out = g_status[dev];
+    *out = g_status[dev].word;
     return TX_OK;
 }
 
@@ -178,35 +211,31 @@ int make_map(CUtensorMap *m, const void *base, int64_t slabs, int64_t rows, int6
     return TX_OK;
 }
 
-// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per kernel (by entry address) and device.
-std::mutex g_smem_mu;
-std::vector<std::pair<const void *, int>> g_smem_done;
-template <class Kernel>
-int allow_smem(Kernel kernel, int bytes)
+// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per kernel and device: one bit per device beside each kernel.
+template <auto Kernel>
+int allow_smem(int bytes)
 {
+    static std::atomic<uint64_t> done{0};
+    static_assert(kMaxDevices <= 64, "one bit per device");
     int dev = 0;
-    TX_CUDA(cudaGetDevice(&dev));
-    const std::pair<const void *, int> key(reinterpret_cast<const void *>(kernel), dev);
-    std::lock_guard<std::mutex> lk(g_smem_mu);
-    if (std::find(g_smem_done.begin(), g_smem_done.end(), key) != g_smem_done.end()) return TX_OK;
-    TX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    g_smem_done.push_back(key);
+    if (int rc = current_device(&dev)) return rc;
+    if (done.load(std::memory_order_acquire) >> dev & 1u) return TX_OK;
+    TX_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    done.fetch_or(uint64_t{1} << dev, std::memory_order_release);
     return TX_OK;
 }
 
 // Multiprocessors of the current device (asked once per device).
 int sm_count(int *n)
 {
-    static std::mutex mu;
-    static std::vector<std::pair<int, int>> seen;
+    static std::atomic<int> seen[kMaxDevices] = {};
     int dev = 0;
-    TX_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lk(mu);
-    for (const auto &e : seen)
-        if (e.first == dev) { *n = e.second; return TX_OK; }
-    int v = 0;
-    TX_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
-    seen.emplace_back(dev, v);
+    if (int rc = current_device(&dev)) return rc;
+    int v = seen[dev].load(std::memory_order_relaxed);
+    if (v == 0) {
+        TX_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
+        seen[dev].store(v, std::memory_order_relaxed);
+    }
     *n = v;
     return TX_OK;
 }
@@ -263,6 +292,42 @@ bool tc_eligible(const tx_sdpa_desc *d)
 }
 
 // ------------------------------------------------------------------ launches
+// Key lengths as a kernel parameter.  Host arrays of more than KvLens::kInline lengths never get here (with_device_lens).
+txb::KvLens lens_of(const int32_t *lens, int flags, int64_t batch)
+{
+    txb::KvLens k;
+    if (lens && (flags & TX_SDPA_KV_LENS_HOST)) {
+        k.n_inline = (int)batch;
+        std::copy(lens, lens + batch, k.val);
+    } else {
+        k.ptr = lens;
+    }
+    return k;
+}
+
+void pool_free(char *p, cudaStream_t st);
+
+// `call(desc)` with the key lengths where the kernels can read them: a host array too long for the parameter block is
+// copied to the device first (the copy has read it when the call returns).
+template <class Desc, class Call>
+int with_device_lens(const Desc *d, Call call)
+{
+    if (!d->kv_lens || !(d->flags & TX_SDPA_KV_LENS_HOST) || d->batch <= txb::KvLens::kInline) return call(d);
+    cudaStream_t st = static_cast<cudaStream_t>(d->stream);
+    char *ws = nullptr;
+    if (int rc = pool_alloc(&ws, (size_t)d->batch * 4, st)) return rc;
+    Desc on_device = *d;
+    on_device.kv_lens = reinterpret_cast<const int32_t *>(ws);
+    on_device.flags &= ~TX_SDPA_KV_LENS_HOST;
+    int rc = TX_OK;
+    if (cudaMemcpyAsync(ws, d->kv_lens, (size_t)d->batch * 4, cudaMemcpyHostToDevice, st) != cudaSuccess)
+        rc = fail(TX_ERR_CUDA, "SDPA: copying the key lengths failed");
+    else
+        rc = call(&on_device);
+    pool_free(ws, st);
+    return rc;
+}
+
 template <typename T, int DVC, bool PROF>
 int launch_simt_t(const txb::SimtParams &p, cudaStream_t st)
 {
@@ -309,7 +374,7 @@ int launch_tc_t(const tx_sdpa_desc *d, cudaStream_t st, int *status, long long *
     p.out = d->out;
     p.out_f16 = out_f16 ? 1 : 0;
     p.lse = d->lse;
-    p.kv_lens = d->kv_lens;
+    p.kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
     p.status = status;
     p.Hq = (int)d->q_heads;
     p.Hkv = (int)d->kv_heads;
@@ -325,7 +390,7 @@ int launch_tc_t(const tx_sdpa_desc *d, cudaStream_t st, int *status, long long *
     if (int rc = causal_group(d, n_tiles * zparts, &group)) return rc;
     p.group = (int)group; p.n_pairs = (int)n_tiles; p.BH = (int)slabs;
     if (n_tiles * slabs * zparts > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA: more than 2^31 work items");
-    if (int rc = allow_smem(txb::sdpa_tc_kernel<Cfg>, (int)Cfg::SMEM_BYTES)) return rc;
+    if (int rc = allow_smem<txb::sdpa_tc_kernel<Cfg>>((int)Cfg::SMEM_BYTES)) return rc;
     dim3 grid((unsigned)(n_tiles * slabs * zparts), 1, 1);
     txb::sdpa_tc_kernel<Cfg><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(tq, tk, tv, to, p);
     g_launches++;
@@ -375,7 +440,7 @@ int launch_pair_t(const tx_sdpa_desc *d, cudaStream_t st, int *status, long long
     p.out = d->out;
     p.out_f16 = out_f16 ? 1 : 0;
     p.lse = d->lse;
-    p.kv_lens = d->kv_lens;
+    p.kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
     p.status = status;
     p.Hq = (int)d->q_heads;
     p.Hkv = (int)d->kv_heads;
@@ -403,7 +468,7 @@ int launch_pair_t(const tx_sdpa_desc *d, cudaStream_t st, int *status, long long
     p.n_pairs = (int)n_pairs;
     p.BH = (int)slabs;
     if (n_pairs * slabs > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA: more than 2^31 work items");
-    if (int rc = allow_smem(txb::sdpa_tc_pair_kernel<Cfg>, (int)Cfg::SMEM_BYTES)) return rc;
+    if (int rc = allow_smem<txb::sdpa_tc_pair_kernel<Cfg>>((int)Cfg::SMEM_BYTES)) return rc;
     dim3 grid((unsigned)(n_pairs * slabs), 1, 1);
     txb::sdpa_tc_pair_kernel<Cfg><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(tq, tk, tv, to, p);
     g_launches++;
@@ -453,7 +518,7 @@ template <int D, class DqCfg, class DkvCfg>
 int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __half *dout_h, const float *delta)
 {
     txb::BwdParams p;
-    p.lse = d->lse; p.delta = delta; p.kv_lens = d->kv_lens;
+    p.lse = d->lse; p.delta = delta; p.kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
     p.dq = d->dq; p.dk = d->dk; p.dv = d->dv;
     p.status = status;
     p.Hq = (int)d->q_heads; p.Hkv = (int)d->kv_heads; p.Sq = (int)d->seq_q; p.Sk = (int)d->seq_k;
@@ -468,8 +533,7 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
         if (int rc = make_map(&tdo, dout_h, d->batch * d->q_heads, d->seq_q, D, DqCfg::BM)) return rc;
         if (int rc = make_map(&tk, d->k, d->batch * d->kv_heads, d->seq_k, D, DqCfg::BN)) return rc;
         if (int rc = make_map(&tv, d->v, d->batch * d->kv_heads, d->seq_k, D, DqCfg::BN)) return rc;
-        TX_CUDA(cudaFuncSetAttribute(txb::sdpa_bwd_dq_kernel<DqCfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)DqCfg::SMEM_BYTES));
+        if (int rc = allow_smem<txb::sdpa_bwd_dq_kernel<DqCfg>>((int)DqCfg::SMEM_BYTES)) return rc;
         // 1-D grid, grouped longest-first order for causal calls (a slab's CTAs stream its K and V)
         const int64_t items = (d->seq_q + DqCfg::BM - 1) / DqCfg::BM, slabs = d->batch * d->q_heads;
         const int64_t ratio = d->q_heads / d->kv_heads;
@@ -490,8 +554,7 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
         if (int rc = make_map(&tdo, dout_h, d->batch * d->q_heads, d->seq_q, D, DkvCfg::BQ)) return rc;
         if (int rc = make_map(&tk, d->k, d->batch * d->kv_heads, d->seq_k, D, DkvCfg::BMK)) return rc;
         if (int rc = make_map(&tv, d->v, d->batch * d->kv_heads, d->seq_k, D, DkvCfg::BMK)) return rc;
-        TX_CUDA(cudaFuncSetAttribute(txb::sdpa_bwd_dkv_kernel<DkvCfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)DkvCfg::SMEM_BYTES));
+        if (int rc = allow_smem<txb::sdpa_bwd_dkv_kernel<DkvCfg>>((int)DkvCfg::SMEM_BYTES)) return rc;
         // 1-D grid: (slab of (batch, K/V head)) x key tile x column part; a slab's CTAs stream the Q and dO of its
         // query heads
         const int64_t items = (d->seq_k + DkvCfg::BMK - 1) / DkvCfg::BMK, slabs = d->batch * d->kv_heads;
@@ -541,7 +604,7 @@ int forward_f32_via_f16(const tx_sdpa_desc *d, cudaStream_t st)
         rc = status_word(&status);
         if (rc == TX_OK) rc = launch_tc(&h, st, status);
     }
-    (void)cudaFreeAsync(ws, st);
+    pool_free(ws, st);
     return rc;
 }
 
@@ -562,7 +625,7 @@ void fill_simt_params(txb::SimtParams *p, const tx_sdpa_desc *d)
 {
     p->q = d->q; p->k = d->k; p->v = d->v;
     p->mask = d->mask;
-    p->kv_lens = d->kv_lens;
+    p->kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
     p->out = d->out;
     p->out_f16 = (d->flags & TX_SDPA_OUT_F16) ? 1 : 0;
     p->B = d->batch; p->Hq = d->q_heads; p->Hkv = d->kv_heads;
@@ -608,7 +671,7 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
         if (int r = make_map(&to, d->out, sq, d->seq_q, d->d_v, 32, 4)) return r;
         txb::X3Params p;
         p.out = static_cast<float *>(d->out);
-        p.kv_lens = d->kv_lens;
+        p.kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
         p.out_of_range = flag;
         p.status = status;
         p.Hq = (int)d->q_heads; p.Hkv = (int)d->kv_heads; p.Sq = (int)d->seq_q; p.Sk = (int)d->seq_k;
@@ -619,7 +682,7 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
         if (int r = causal_group(d, n_tiles, &group)) return r;
         p.group = (int)group; p.n_tiles_q = (int)n_tiles; p.BH = (int)sq;
         if (n_tiles * sq > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA: more than 2^31 work items");
-        if (int r = allow_smem(txb::sdpa_tc_x3_kernel<Cfg>, (int)Cfg::SMEM_BYTES)) return r;
+        if (int r = allow_smem<txb::sdpa_tc_x3_kernel<Cfg>>((int)Cfg::SMEM_BYTES)) return r;
         txb::sdpa_tc_x3_kernel<Cfg><<<(unsigned)(n_tiles * sq), Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(qh, ql, kh, kl, vh, vl, to, p);
         g_launches++;
         TX_CUDA(cudaGetLastError());
@@ -630,7 +693,7 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
         return launch_simt<float>(sp2, st);
     };
     rc = body();
-    (void)cudaFreeAsync(ws, st);
+    pool_free(ws, st);
     return rc;
 }
 
@@ -640,10 +703,8 @@ int launch_x3(const tx_sdpa_desc *d, cudaStream_t st, int *status)
     return launch_x3_t<txb::X3Cfg<128, 2>>(d, st, status);
 }
 
-int forward(const tx_sdpa_desc *d)
+int forward_launch(const tx_sdpa_desc *d)
 {
-    if (int rc = validate(d)) return rc;
-    if (int rc = ensure_device()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(d->stream);
     if (d->dtype == TX_DTYPE_F32 && (d->flags & TX_SDPA_F32_VIA_F16)) {
         tx_sdpa_desc probe = *d;
@@ -665,19 +726,23 @@ int forward(const tx_sdpa_desc *d)
     return d->dtype == TX_DTYPE_F16 ? launch_simt<__half>(p, st) : launch_simt<float>(p, st);
 }
 
+int forward(const tx_sdpa_desc *d)
+{
+    if (int rc = validate(d)) return rc;
+    if (int rc = ensure_device()) return rc;
+    return with_device_lens(d, forward_launch);
+}
+
 int finish(cudaStream_t st)
 {
     TX_CUDA(cudaStreamSynchronize(st));
     int dev = 0;
-    TX_CUDA(cudaGetDevice(&dev));
-    int *w = (dev >= 0 && dev < kMaxDevices) ? g_status[dev] : nullptr;
-    if (w) {
-        int code = 0;
-        TX_CUDA(cudaMemcpy(&code, w, sizeof code, cudaMemcpyDeviceToHost));
-        if (code != 0) {
-            (void)cudaMemset(w, 0, sizeof code);
-            return fail(TX_ERR_KERNEL, "SDPA kernel gave up on a bounded wait (stage code %d); output is not valid", code);
-        }
+    if (int rc = current_device(&dev)) return rc;
+    if (g_status_ready[dev].load(std::memory_order_acquire) && *g_status[dev].mirror != 0) {
+        const int code = *g_status[dev].mirror;
+        (void)cudaMemset(g_status[dev].word, 0, sizeof code);      // the word only: the mirror's address stays
+        *g_status[dev].mirror = 0;
+        return fail(TX_ERR_KERNEL, "SDPA kernel gave up on a bounded wait (stage code %d); output is not valid", code);
     }
     return TX_OK;
 }
@@ -713,7 +778,7 @@ int profile_f32(const float *Q, const float *K, const float *V, const float *mas
     int rc = cudaMemset(dev, 0, 32 * sizeof(long long)) == cudaSuccess ? TX_OK : fail(TX_ERR_CUDA, "cudaMemset failed");
     if (rc == TX_OK) {
         txb::SimtParams p;
-        p.q = Q; p.k = K; p.v = V; p.mask = mask; p.kv_lens = nullptr; p.out = out; p.out_f16 = 0;
+        p.q = Q; p.k = K; p.v = V; p.mask = mask; p.out = out; p.out_f16 = 0;
         p.B = B; p.Hq = H; p.Hkv = H; p.Sq = Sq; p.Sk = Sk; p.dk = dk; p.dv = dv;
         p.causal = 0;
         p.scale = 1.0f / std::sqrt((float)dk);
@@ -854,20 +919,70 @@ int static_scratch(unsigned char **out)
 // dominate short calls (docs/profiling/RESULTS.md:149-152).  Here the pair goes through the device's
 // stream-ordered memory pool with a release threshold that keeps freed blocks cached, so a steady
 // sequence of calls stops touching the driver's allocator after the first one.
-int pool_ready()
+// Freed blocks stay cached up to kPoolKeep bytes BEYOND what the program holds; more goes back to the driver at the
+// next synchronisation, so a process on a shared GPU does not sit on everything it ever touched.  CUDA's release
+// threshold counts the blocks in use too, so it follows them: with a fixed 4 GiB a program that held more than that
+// in tensors had every freed block unmapped at each synchronisation and mapped again by the next call (a 1 GiB result:
+// 4.6 ms to 24 ms per call around 3.7 ms of kernel).
+constexpr unsigned long long kPoolKeep = 4ull << 30, kPoolStep = 1ull << 30;
+struct PoolBooks {
+    std::mutex mu;
+    std::unordered_map<void *, std::pair<int, size_t>> blocks;     // pointer -> (device, bytes)
+    unsigned long long live[kMaxDevices] = {}, steps[kMaxDevices] = {};
+    cudaMemPool_t pool[kMaxDevices] = {};
+};
+PoolBooks &books()
+{
+    static PoolBooks *b = new PoolBooks;     // never destroyed: tensors may be freed while the process ends
+    return *b;
+}
+
+// Called with the books locked: the release threshold in whole steps, so that it is set only now and then.
+void pool_threshold(PoolBooks &bk, int dev)
+{
+    const unsigned long long steps = bk.live[dev] / kPoolStep + 1;
+    if (steps == bk.steps[dev]) return;
+    unsigned long long keep = steps * kPoolStep + kPoolKeep;
+    if (cudaMemPoolSetAttribute(bk.pool[dev], cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) bk.steps[dev] = steps;
+    else (void)cudaGetLastError();
+}
+
+void pool_took(void *ptr, size_t bytes)
 {
     int dev = 0;
-    TX_CUDA(cudaGetDevice(&dev));
-    static bool ready[kMaxDevices] = {};
-    if (dev < 0 || dev >= kMaxDevices) return fail(TX_ERR_INVALID, "device index %d out of range", dev);
-    if (!ready[dev]) {
-        cudaMemPool_t pool;
-        TX_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
-        // Freed blocks stay cached up to this much; beyond it the pool gives memory back to the driver at the
-        // next synchronisation, so a process on a shared GPU does not sit on everything it ever touched.
-        unsigned long long keep = 4ull << 30;
-        TX_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-        ready[dev] = true;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
+    PoolBooks &bk = books();
+    std::lock_guard<std::mutex> lk(bk.mu);
+    bk.blocks[ptr] = {dev, bytes};
+    bk.live[dev] += bytes;
+    pool_threshold(bk, dev);
+}
+
+void pool_gave(void *ptr)
+{
+    PoolBooks &bk = books();
+    std::lock_guard<std::mutex> lk(bk.mu);
+    const auto it = bk.blocks.find(ptr);
+    if (it == bk.blocks.end()) return;
+    const int dev = it->second.first;
+    bk.live[dev] -= it->second.second;
+    bk.blocks.erase(it);
+    pool_threshold(bk, dev);
+}
+
+int pool_ready()
+{
+    static std::atomic<bool> ready[kMaxDevices] = {};
+    int dev = 0;
+    if (int rc = current_device(&dev)) return rc;
+    if (!ready[dev].load(std::memory_order_acquire)) {
+        PoolBooks &bk = books();
+        std::lock_guard<std::mutex> lk(bk.mu);
+        TX_CUDA(cudaDeviceGetDefaultMemPool(&bk.pool[dev], dev));
+        unsigned long long keep = kPoolStep + kPoolKeep;
+        TX_CUDA(cudaMemPoolSetAttribute(bk.pool[dev], cudaMemPoolAttrReleaseThreshold, &keep));
+        bk.steps[dev] = 1;
+        ready[dev].store(true, std::memory_order_release);
     }
     return TX_OK;
 }
@@ -915,12 +1030,14 @@ void *tx_cuda_malloc(size_t bytes)
         (void)cudaGetLastError();
         return nullptr;
     }
+    pool_took(p, bytes ? bytes : 1);
     return p;
 }
 
 int tx_cuda_free(void *ptr)
 {
     if (!ptr) return TX_OK;
+    pool_gave(ptr);
     TX_CUDA(cudaFreeAsync(ptr, (cudaStream_t)0));
     return TX_OK;
 }
@@ -928,6 +1045,7 @@ int tx_cuda_free(void *ptr)
 int tx_cuda_free_on(void *ptr, void *stream)
 {
     if (!ptr) return TX_OK;
+    pool_gave(ptr);
     TX_CUDA(cudaFreeAsync(ptr, static_cast<cudaStream_t>(stream)));
     return TX_OK;
 }
@@ -1147,7 +1265,7 @@ int tx_linear_f32_cuda(const float *x, const float *w, const float *bias, float 
         lp.bias = bias; lp.out = out; lp.status = status;
         lp.S = (int)seq; lp.N = (int)out_features; lp.K = (int)in_features;
         lp.dh_in = (int)dh_in; lp.heads_out = heads_out;
-        TX_CUDA(cudaFuncSetAttribute(txb::linear_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)txb::LTC_SMEM));
+        if (int rc = allow_smem<txb::linear_tc_kernel>((int)txb::LTC_SMEM)) return rc;
         dim3 grid((unsigned)((out_features + txb::LTC_BN - 1) / txb::LTC_BN), (unsigned)((seq + txb::LTC_BM - 1) / txb::LTC_BM),
                   (unsigned)batch);
         txb::linear_tc_kernel<<<grid, txb::LTC_THREADS, txb::LTC_SMEM>>>(tx_map, tw_map, lp);
@@ -1190,7 +1308,7 @@ int tx_profile_sections_sdpa(const tx_sdpa_desc *d, long long *ticks64)
     cudaStream_t st = static_cast<cudaStream_t>(d->stream);
     int rc = TX_OK;
     if (cudaMemsetAsync(dev, 0, 64 * sizeof(long long), st) != cudaSuccess) rc = fail(TX_ERR_CUDA, "cudaMemsetAsync failed");
-    if (rc == TX_OK) rc = launch_tc(d, st, status, dev);
+    if (rc == TX_OK) rc = with_device_lens(d, [&](const tx_sdpa_desc *e) { return launch_tc(e, st, status, dev); });
     if (rc == TX_OK) rc = finish(st);
     if (rc == TX_OK && cudaMemcpy(ticks64, dev, 64 * sizeof(long long), cudaMemcpyDeviceToHost) != cudaSuccess)
         rc = fail(TX_ERR_CUDA, "cudaMemcpy of the section profile failed");
@@ -1207,10 +1325,14 @@ int tx_selftest_wait_timeout(const tx_sdpa_desc *d, int32_t skip_k_tile)
     int *status = nullptr;
     if (int rc = status_word(&status)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(d->stream);
-    if (int rc = launch_pair_t<txb::PairCfg<64, 128, 4, kPolyPairsD64, false, false, true>>(d, st, status, nullptr, skip_k_tile))
+    if (int rc = with_device_lens(d, [&](const tx_sdpa_desc *e) {
+            return launch_pair_t<txb::PairCfg<64, 128, 4, kPolyPairsD64, false, false, true>>(e, st, status, nullptr, skip_k_tile);
+        }))
         return rc;
     return finish(st);
 }
+
+static int backward_launch(const tx_sdpa_bwd_desc *d);
 
 int tx_sdpa_backward(const tx_sdpa_bwd_desc *d)
 {
@@ -1230,6 +1352,11 @@ int tx_sdpa_backward(const tx_sdpa_bwd_desc *d)
     if (!al(d->q) || !al(d->k) || !al(d->v) || !al(d->out) || !al(d->dout) || !al(d->dq) || !al(d->dk) || !al(d->dv))
         return fail(TX_ERR_INVALID, "SDPA backward: pointers must be 16-byte aligned");
     if (int rc = ensure_device()) return rc;
+    return with_device_lens(d, backward_launch);
+}
+
+static int backward_launch(const tx_sdpa_bwd_desc *d)
+{
     int *status = nullptr;
     if (int rc = status_word(&status)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(d->stream);
@@ -1265,7 +1392,7 @@ int tx_sdpa_backward(const tx_sdpa_bwd_desc *d)
             // read to its second, so one stage per ring would deadlock the MMA warp).
             rc = launch_bwd<256, txb::BwdDqCfg<256, 64, 2, 1, 1>, txb::BwdDkvCfg<256, 32, 2, 1, false, 2, 2>>(d, st, status, dout_h, delta);
     }
-    (void)cudaFreeAsync(ws, st);        // ordered after the kernels on `st`
+    pool_free(ws, st);        // ordered after the kernels on `st`
     return rc;
 }
 
@@ -1374,6 +1501,7 @@ static int forward_host(const tx_sdpa_desc *h, bool with_kernel)
             d.q = w + oq + uq * u0; d.k = w + ok + uk * u0; d.v = w + ov + uv * u0;
             d.out = w + oo + uo * u0;
             d.kv_lens = nl ? reinterpret_cast<const int32_t *>(w + ol) + u0 : nullptr;
+            d.flags &= ~TX_SDPA_KV_LENS_HOST;
             d.batch = nu; d.q_heads = group; d.kv_heads = 1;
             if (int rc = forward(&d)) return rc;
         }

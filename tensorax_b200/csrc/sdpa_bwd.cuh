@@ -33,7 +33,7 @@ enum : int { BWD_ERR_PRODUCER = 22, BWD_ERR_MMA = 23, BWD_ERR_ROWS = 24 };
 struct BwdParams {
     const float *lse;         // [B,Hq,Sq] log2-domain row statistic written by the forward
     const float *delta;       // [B,Hq,Sq] rowsum(dO o O)
-    const int32_t *kv_lens;   // optional [B]
+    KvLens kv_lens;           // optional [B]
     float *dq, *dk, *dv;      // [B,Hq,Sq,D], [B,Hkv,Sk,D], [B,Hkv,Sk,D] fp32
     int *status;
     int Hq, Hkv, Sq, Sk;
@@ -138,7 +138,7 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const int b = bh / p.Hq, h = bh % p.Hq;
     const int kvh = b * p.Hkv + h / (p.Hq / p.Hkv);
     int kv_limit = p.Sk;
-    if (p.kv_lens) kv_limit = min(kv_limit, max(p.kv_lens[b], 0));
+    kv_limit = p.kv_lens.limit(b, kv_limit);
     int kv_end = kv_limit;
     if (p.causal) kv_end = min(kv_end, q0 + BM);
     const int n_tiles = (kv_end + BN - 1) / BN;
@@ -160,7 +160,7 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             ptx::mbar_init(v_empty + 8 * s, 1);
         }
         ptx::fence_mbar_init();
-        if (sbase & 1023u) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_ALIGN); }
+        if (sbase & 1023u) { *abort_flag = 1; ptx::report(p.status, TC_ERR_ALIGN); }
         if (*reinterpret_cast<volatile int *>(p.status) != 0) *abort_flag = 1;
     }
     if (warp == 1) {
@@ -216,7 +216,7 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
                 __syncwarp();
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, BWD_ERR_PRODUCER); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, BWD_ERR_PRODUCER); }
         }
     } else if (warp == 1) {
         if (run) {
@@ -292,7 +292,7 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
                 __syncwarp();
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, BWD_ERR_MMA); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, BWD_ERR_MMA); }
         }
     } else {
         constexpr int CW = Cfg::CW;
@@ -378,7 +378,7 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
             }
         }
-        if (run && !ok) { *abort_flag = 1; atomicCAS(p.status, 0, BWD_ERR_ROWS); }
+        if (run && !ok) { *abort_flag = 1; ptx::report(p.status, BWD_ERR_ROWS); }
         if (!run && *abort_flag == 0 && row_ok) {
             // no visible key: the forward row is 0/0, and so is its gradient
             float *grow = p.dq + ((size_t)bh * p.Sq + row) * D;
@@ -471,7 +471,7 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int group = p.Hq / p.Hkv;
     const int bh0 = b * p.Hq + (kvh % p.Hkv) * group;           // first query head of the group
     int kv_limit = p.Sk;
-    if (p.kv_lens) kv_limit = min(kv_limit, max(p.kv_lens[b], 0));
+    kv_limit = p.kv_lens.limit(b, kv_limit);
     const int nq = (p.Sq + BQ - 1) / BQ;
     // causal: query rows below the tile's first key see none of its keys
     const int i_start = p.causal ? min(key0 / BQ, nq) : 0;
@@ -495,7 +495,7 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             ptx::mbar_init(do_empty + 8 * s, 1);
         }
         ptx::fence_mbar_init();
-        if (sbase & 1023u) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_ALIGN); }
+        if (sbase & 1023u) { *abort_flag = 1; ptx::report(p.status, TC_ERR_ALIGN); }
         if (*reinterpret_cast<volatile int *>(p.status) != 0) *abort_flag = 1;
     }
     if (warp == 1) {
@@ -552,7 +552,7 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 }
                 __syncwarp();
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, BWD_ERR_PRODUCER); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, BWD_ERR_PRODUCER); }
         }
     } else if (warp == 1) {
         if (run) {
@@ -647,7 +647,7 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 }
                 __syncwarp();
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, BWD_ERR_MMA); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, BWD_ERR_MMA); }
         }
     } else {
         constexpr int CW = Cfg::CW;
@@ -774,7 +774,7 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 }
             }
         }
-        if (run && !ok) { *abort_flag = 1; atomicCAS(p.status, 0, BWD_ERR_ROWS); }
+        if (run && !ok) { *abort_flag = 1; ptx::report(p.status, BWD_ERR_ROWS); }
         if (!run && *abort_flag == 0 && key < p.Sk) {
             // no query sees these keys: zero gradients -- unless the batch element has no valid key at
             // all, where the forward rows are 0/0 and the reference's rule propagates NaN to every gradient

@@ -26,12 +26,14 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "kv_lens.cuh"
+
 namespace txb {
 
 struct SimtParams {
     const void *q, *k, *v;   // [B,Hq,Sq,dk], [B,Hkv,Sk,dk], [B,Hkv,Sk,dv]
     const float *mask;       // optional dense additive [B,Hq,Sq,Sk]
-    const int32_t *kv_lens;  // optional [B]
+    KvLens kv_lens;           // optional [B]
     void *out;               // [B,Hq,Sq,dv] fp32, or fp16 when out_f16
     int64_t B, Hq, Hkv, Sq, Sk, dk, dv;
     int causal;
@@ -97,7 +99,7 @@ sdpa_simt_kernel(const SimtParams p)
     const float *M = p.mask ? p.mask + bh * p.Sq * p.Sk : nullptr;
 
     int64_t key_end = p.Sk;
-    if (p.kv_lens) key_end = min(key_end, (int64_t)max(p.kv_lens[b], 0));
+    key_end = p.kv_lens.limit((int)b, (int)key_end);
     const int64_t len_b = key_end;
     if (p.causal) key_end = min(key_end, q0 + SIMT_BR);   // keys past the last row's diagonal
 

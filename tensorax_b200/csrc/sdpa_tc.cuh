@@ -43,7 +43,7 @@ namespace txb {
 struct TcParams {
     void *out;                // [B,Hq,Sq,dv_total] fp32, or fp16 when out_f16
     float *lse;               // optional [B,Hq,Sq]: log2 of the row's sum of 2^(score*scale_log2)
-    const int32_t *kv_lens;   // optional [B]
+    KvLens kv_lens;           // optional [B]
     int *status;              // device word: 0 = ok, else first failing wait's code
     int Hq, Hkv, Sq, Sk;
     int dv_total;             // row length of `out` (= DV * the CTAs per query tile)
@@ -200,7 +200,7 @@ sdpa_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const int kvh = b * p.Hkv + h / (p.Hq / p.Hkv);
 
     int kv_limit = p.Sk;                                   // keys any row of this batch may see
-    if (p.kv_lens) kv_limit = min(kv_limit, max(p.kv_lens[b], 0));
+    kv_limit = p.kv_lens.limit(b, kv_limit);
     int kv_end = kv_limit;                                 // keys this query tile may see
     if (p.causal) kv_end = min(kv_end, q0 + BM);
     const int n_tiles = (kv_end + BN - 1) / BN;
@@ -224,7 +224,7 @@ sdpa_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         ptx::fence_mbar_init();
         if (sbase & 1023u) {
             *abort_flag = 1;
-            atomicCAS(p.status, 0, TC_ERR_ALIGN);
+            ptx::report(p.status, TC_ERR_ALIGN);
         } else if (n_tiles > 0) {
             // The Q tile is requested before the CTA meets: the tensor-memory allocation and the meeting then
             // run under the load's latency instead of in front of it.
@@ -345,7 +345,7 @@ sdpa_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     __syncwarp();
                 }
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_PRODUCER); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, TC_ERR_PRODUCER); }
             if constexpr (Cfg::PROF) {
                 if (prof_on && leader) {
                     p.prof[SEC_LD_TOTAL] = clock64() - t_begin;
@@ -442,7 +442,7 @@ sdpa_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 __syncwarp();
                 tick(5);
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_MMA); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, TC_ERR_MMA); }
             if constexpr (Cfg::PROF) {
                 if (prof_on && leader) {
                     p.prof[SEC_MMA_TOTAL] = clock64() - t_begin;
@@ -676,7 +676,7 @@ sdpa_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 __syncwarp();
             }
         }
-        if (run && !ok) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_SOFTMAX); }
+        if (run && !ok) { *abort_flag = 1; ptx::report(p.status, TC_ERR_SOFTMAX); }
         if constexpr (Cfg::PROF) {
             if (prof_on && warp == 2 && lane == 0) {
                 p.prof[SEC_SM_TOTAL] = t_loop_end - t_begin;

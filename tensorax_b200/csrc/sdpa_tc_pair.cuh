@@ -138,7 +138,7 @@ sdpa_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int kvh = b * p.Hkv + h / (p.Hq / p.Hkv);
 
     int kv_limit = p.Sk;                                         // keys any row of this batch may see
-    if (p.kv_lens) kv_limit = min(kv_limit, max(p.kv_lens[b], 0));
+    kv_limit = p.kv_lens.limit(b, kv_limit);
     // key tiles each query tile walks; tile 1 does not exist when the sequence ends inside tile 0
     const bool live1 = q0 + BM < p.Sq;
     const int kv_end0 = p.causal ? min(kv_limit, q0 + BM) : kv_limit;
@@ -169,7 +169,7 @@ sdpa_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             ptx::fence_mbar_init();
             if (sbase & 1023u) {
                 *abort_flag = 1;
-                atomicCAS(p.status, 0, TC_ERR_ALIGN);
+                ptx::report(p.status, TC_ERR_ALIGN);
             } else if (n_max > 0) {
                 ptx::prefetch_tmap(&tm_q);
                 ptx::prefetch_tmap(&tm_k);
@@ -251,7 +251,7 @@ sdpa_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 }
                 __syncwarp();
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_PRODUCER); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, TC_ERR_PRODUCER); }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
@@ -353,7 +353,7 @@ sdpa_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                     }
                 }
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_MMA); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, TC_ERR_MMA); }
             if constexpr (Cfg::PROF) {
                 if (prof_on && leader) {
                     p.prof[PSEC_MMA_TOTAL] = clock64() - t_begin;
@@ -551,7 +551,7 @@ sdpa_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 __syncwarp();
             }
         }
-        if (run && nt > 0 && !ok) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_SOFTMAX); }
+        if (run && nt > 0 && !ok) { *abort_flag = 1; ptx::report(p.status, TC_ERR_SOFTMAX); }
         if constexpr (Cfg::PROF) {
             if (prof_lane) {
                 long long *dst = p.prof + (t ? 32 : 0);

@@ -58,7 +58,7 @@ struct X3Cfg {
 
 struct X3Params {
     float *out;               // [B,Hq,Sq,D] fp32
-    const int32_t *kv_lens;   // optional [B]
+    KvLens kv_lens;           // optional [B]
     const int *out_of_range;  // device word the split pass sets: nonzero = this kernel does nothing
     int *status;              // device word: 0 = ok, else first failing wait's code
     int Hq, Hkv, Sq, Sk;
@@ -106,7 +106,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
     const int kvh = b * p.Hkv + h / (p.Hq / p.Hkv);
 
     int kv_limit = p.Sk;                                         // keys any row of this batch may see
-    if (p.kv_lens) kv_limit = min(kv_limit, max(p.kv_lens[b], 0));
+    kv_limit = p.kv_lens.limit(b, kv_limit);
     const int kv_end = p.causal ? min(kv_limit, q0 + BM) : kv_limit;
     const int nt = (kv_end + BN - 1) / BN;
 
@@ -142,7 +142,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
             ptx::fence_mbar_init();
             if (sbase & 1023u) {
                 *abort_flag = 1;
-                atomicCAS(p.status, 0, TC_ERR_ALIGN);
+                ptx::report(p.status, TC_ERR_ALIGN);
             } else if (nt > 0) {
                 ptx::prefetch_tmap(&tm_qh);
                 ptx::prefetch_tmap(&tm_kh);
@@ -188,7 +188,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                 if (leader) load_kv(v_s + s * 2 * Cfg::KV_BYTES, &tm_vh, &tm_vl, v_full + 8 * s, j);
                 __syncwarp();
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_PRODUCER); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, TC_ERR_PRODUCER); }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
@@ -266,7 +266,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                 }
                 if (ok) ok = issue_pv(j);
             }
-            if (!ok && leader) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_MMA); }
+            if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, TC_ERR_MMA); }
         }
     }
     } else if (warp < 8) {
@@ -356,7 +356,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(l_full);
         }
-        if (run && !ok) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_SOFTMAX); }
+        if (run && !ok) { *abort_flag = 1; ptx::report(p.status, TC_ERR_SOFTMAX); }
         if (nt == 0 && *abort_flag == 0 && row < p.Sq) {
             // no visible key at all for this tile: the reference's 0/0
             float *orow = p.out + ((size_t)bh * p.Sq + row) * D;
@@ -437,7 +437,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                 __syncwarp();
             }
         }
-        if (run && !ok) { *abort_flag = 1; atomicCAS(p.status, 0, TC_ERR_SOFTMAX); }
+        if (run && !ok) { *abort_flag = 1; ptx::report(p.status, TC_ERR_SOFTMAX); }
     }
 
     // ---------------------------------------------------------------- teardown
