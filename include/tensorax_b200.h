@@ -38,7 +38,7 @@ enum {
     TX_ERR_KERNEL = 4,     /* a kernel gave up on a bounded wait (2 s) and reported it; tx_last_error() names the
                               stage: 1 misaligned shared memory, 2/3/4 forward producer / MMA / softmax warp,
                               12/13/14 linear-kernel producer / MMA / split warps, 22/23/24 backward
-                              producer / MMA / row warps */
+                              producer / MMA / row warps, 32/34 decoding-kernel producer / row warps */
     TX_ERR_UNSUPPORTED = 5
 };
 
@@ -181,7 +181,9 @@ TX_API int tx_sdpa_forward(const tx_sdpa_desc *desc);
  * between return at once and write NaN. */
 TX_API int tx_sdpa_finish(void *stream);
 /* 1 if tx_sdpa_forward would run `desc` on a tcgen05 kernel (fp16, or fp32 as hi/lo fp16 pairs), 0 if on CUDA cores.
- * (For fp32 the answer is about the shape: a value outside the pairs' range still sends the call to CUDA cores.) */
+ * (For fp32 the answer is about the shape: a value outside the pairs' range still sends the call to CUDA cores.)
+ * Calls with few query rows per K/V head -- decoding steps, up to 16 rows in fp16 and 32 in fp32 -- run on a kernel of
+ * their own that reads the cache once and is bound by memory, not arithmetic: 0. */
 TX_API int tx_sdpa_uses_tensor_cores(const tx_sdpa_desc *desc);
 /* How many kernels of this library have been launched by this process so far. */
 TX_API int64_t tx_kernel_launch_count(void);

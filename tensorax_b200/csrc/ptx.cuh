@@ -140,6 +140,14 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *m, 
         : "memory");
 }
 
+// Untiled bulk copy of contiguous memory (both addresses and the size multiples of 16 bytes).
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
 // v when i < lim, else -inf: one compare and one select.  (Written as `if (!visible) v = -inf` over a register
 // array the compiler emitted a divergent branch per element: 27 cycles each on a causal diagonal tile.)
 __device__ __forceinline__ uint32_t keep_if_below(uint32_t v, int i, int lim)

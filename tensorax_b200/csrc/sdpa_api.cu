@@ -37,6 +37,7 @@
 #include "sdpa_tc_pair.cuh"
 #include "sdpa_tc_x3.cuh"
 #include "sdpa_bwd.cuh"
+#include "sdpa_decode.cuh"
 
 namespace {
 
@@ -212,7 +213,8 @@ int make_map(CUtensorMap *m, const void *base, int64_t slabs, int64_t rows, int6
 }
 
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per kernel and device: one bit per device beside each kernel.
-template <auto Kernel>
+// LARGE_CLUSTERS: the kernel may be launched in clusters of more than eight CTAs.
+template <auto Kernel, bool LARGE_CLUSTERS = false>
 int allow_smem(int bytes)
 {
     static std::atomic<uint64_t> done{0};
@@ -221,6 +223,7 @@ int allow_smem(int bytes)
     if (int rc = current_device(&dev)) return rc;
     if (done.load(std::memory_order_acquire) >> dev & 1u) return TX_OK;
     TX_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    if (LARGE_CLUSTERS) TX_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     done.fetch_or(uint64_t{1} << dev, std::memory_order_release);
     return TX_OK;
 }
@@ -514,6 +517,81 @@ int launch_tc(const tx_sdpa_desc *d, cudaStream_t st, int *status, long long *pr
     return fail(TX_ERR_UNSUPPORTED, "SDPA: no tensor-core tile shape for d = %lld", (long long)d->d_k);
 }
 
+// Few query rows per K/V head (a decoding step): the kernel that reads the cache once and cuts the keys over a cluster.
+// fp16 up to 16 rows a head (CTAs of four rows each, side by side, read the same keys through L2; beyond that the
+// tensor-core kernel's 128-row tile is the better use of a CTA) and from one whole tile of keys on; fp32 up to 32 rows, because the
+// tensor-core form first writes and reads back hi / lo copies of the whole cache.
+bool decode_eligible(const tx_sdpa_desc *d)
+{
+    if (d->flags & (TX_SDPA_FORCE_SIMT | TX_SDPA_P_IN_SMEM)) return false;
+    if (d->d_k != d->d_v || (d->d_k != 64 && d->d_k != 128 && d->d_k != 256)) return false;
+    auto al = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    if (!al(d->q) || !al(d->k) || !al(d->v)) return false;
+    const int64_t rows = d->q_heads / d->kv_heads * d->seq_q;
+    return d->dtype == TX_DTYPE_F16 ? (rows <= 16 && d->seq_k >= 128) : rows <= 32;
+}
+
+template <class Cfg>
+int launch_decode_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
+{
+    txb::DecodeParams p;
+    p.q = d->q; p.k = d->k; p.v = d->v; p.mask = d->mask;
+    p.kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
+    p.out = d->out; p.lse = d->lse; p.status = status;
+    p.out_f16 = (d->flags & TX_SDPA_OUT_F16) ? 1 : 0;
+    p.Hkv = (int)d->kv_heads; p.Sq = (int)d->seq_q; p.Sk = (int)d->seq_k;
+    p.rows = (int)(d->q_heads / d->kv_heads * d->seq_q);
+    p.row_parts = (p.rows + Cfg::R - 1) / Cfg::R;
+    p.causal = d->causal ? 1 : 0;
+    p.scale = 1.0f / std::sqrt((float)d->d_k);
+    int sms = 0;
+    if (int rc = sm_count(&sms)) return rc;
+    // CTAs per head: as many as one wave holds, as long as each still has a stage of keys; sixteen (a cluster size that
+    // costs 1.4 us more to start and merge) only where each then has four stages
+    const int64_t items = d->batch * d->kv_heads * p.row_parts;
+    if (items * Cfg::MAX_SPLITS > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA: more than 2^31 work items");
+    int splits = 1;
+    const int most = d->seq_k >= 4 * Cfg::MAX_SPLITS * Cfg::KEYS ? Cfg::MAX_SPLITS : 8;
+    while (splits < most && items * splits * 2 <= Cfg::CTAS_PER_SM * sms && splits * Cfg::KEYS < d->seq_k) splits *= 2;
+    if (int rc = allow_smem<txb::sdpa_decode_kernel<Cfg>, true>((int)Cfg::SMEM)) return rc;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)splits; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(items * splits));
+    cfg.blockDim = dim3(Cfg::THREADS);
+    cfg.dynamicSmemBytes = Cfg::SMEM;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    TX_CUDA(cudaLaunchKernelEx(&cfg, txb::sdpa_decode_kernel<Cfg>, p));
+    g_launches++;
+    return TX_OK;
+}
+
+template <typename T, int D>
+int launch_decode_d(const tx_sdpa_desc *d, cudaStream_t st, int *status)
+{
+    const int64_t rows = d->q_heads / d->kv_heads * d->seq_q;
+    if (rows == 1) return launch_decode_t<txb::DecodeCfg<T, D, 1>>(d, st, status);
+    if (rows == 2) return launch_decode_t<txb::DecodeCfg<T, D, 2>>(d, st, status);
+    return launch_decode_t<txb::DecodeCfg<T, D, 4>>(d, st, status);
+}
+
+template <typename T>
+int launch_decode(const tx_sdpa_desc *d, cudaStream_t st, int *status)
+{
+    if (d->d_k == 64) return launch_decode_d<T, 64>(d, st, status);
+    if (d->d_k == 128) return launch_decode_d<T, 128>(d, st, status);
+    return launch_decode_d<T, 256>(d, st, status);
+}
+
+// fp16 without a dense mask, at the shapes tc_eligible names
+int launch_f16(const tx_sdpa_desc *d, cudaStream_t st, int *status)
+{
+    return decode_eligible(d) ? launch_decode<__half>(d, st, status) : launch_tc(d, st, status);
+}
+
 template <int D, class DqCfg, class DkvCfg>
 int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __half *dout_h, const float *delta)
 {
@@ -706,6 +784,11 @@ int launch_x3(const tx_sdpa_desc *d, cudaStream_t st, int *status)
 int forward_launch(const tx_sdpa_desc *d)
 {
     cudaStream_t st = static_cast<cudaStream_t>(d->stream);
+    if (decode_eligible(d)) {
+        int *status = nullptr;
+        if (int rc = status_word(&status)) return rc;
+        return d->dtype == TX_DTYPE_F16 ? launch_decode<__half>(d, st, status) : launch_decode<float>(d, st, status);
+    }
     if (d->dtype == TX_DTYPE_F32 && (d->flags & TX_SDPA_F32_VIA_F16)) {
         tx_sdpa_desc probe = *d;
         probe.dtype = TX_DTYPE_F16;                 // would the fp16 form of this call run on the tensor cores?
@@ -1400,7 +1483,7 @@ int tx_sdpa_finish(void *stream) { return finish(static_cast<cudaStream_t>(strea
 
 int tx_sdpa_uses_tensor_cores(const tx_sdpa_desc *desc)
 {
-    if (validate(desc) != TX_OK) return 0;
+    if (validate(desc) != TX_OK || decode_eligible(desc)) return 0;
     if (desc->dtype == TX_DTYPE_F32 && (desc->flags & TX_SDPA_F32_VIA_F16)) {
         tx_sdpa_desc probe = *desc;
         probe.dtype = TX_DTYPE_F16;
@@ -1560,7 +1643,7 @@ int tx_sdpa_fp16_static_scratch(const void *Q_h, const void *K_h, const void *V_
         TX_CUDA(cudaMemcpyAsync(scratch + 256, kv_lens_host, (size_t)batch * 4, cudaMemcpyHostToDevice, st));
         desc.kv_lens = reinterpret_cast<const int32_t *>(scratch + 256);
     }
-    if (int rc = launch_tc(&desc, st, status)) return rc;
+    if (int rc = launch_f16(&desc, st, status)) return rc;
     int code = 0;
     TX_CUDA(cudaMemcpyAsync(&code, status, sizeof code, cudaMemcpyDeviceToHost, st));
     TX_CUDA(cudaStreamSynchronize(st));
