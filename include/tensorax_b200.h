@@ -94,12 +94,13 @@ TX_API int tx_host_free_pinned(void *ptr);
  *      Q [B,H,Sq,d_k], K [B,H,Sk,d_k], V [B,H,Sk,d_v], optional dense additive
  *      mask [B,H,Sq,Sk] (NULL = none), out [B,H,Sq,d_v], all fp32 on the device.
  *      Like the reference they return after the result is complete.
- *      Two kernels stand behind the five names.  Calls without a dense mask and with d_k = d_v in {64, 128} run on
- *      the tensor cores: every fp32 operand is carried as two fp16 numbers (hi + lo, 22 significand bits), every
- *      product is three tcgen05 MMAs, tiles are summed in fp32 registers, the softmax is fp32 (within 2e-6 of the
- *      reference's sdpa_cpu on unit-variance inputs, the figure of the exact kernel; 3e-5 at scores of +-100, where
- *      the exact kernel itself is at 1e-5).  A device-side range check sends a call with |x| >= 2^15 or a
- *      non-finite input to the exact CUDA-core kernel, which also takes every other shape and every dense mask. */
+ *      Three kernels stand behind the five names.  Calls with d_k and d_v up to 128 (multiples of 4), with or without a
+ *      dense mask, run on the tensor cores: every fp32 operand is carried as two fp16 numbers (hi + lo, 22 significand
+ *      bits), every product is three tcgen05 MMAs, tiles are summed in fp32 registers, the softmax is fp32 (within 2e-6 of
+ *      the reference's sdpa_cpu on unit-variance inputs, the figure of the exact kernel; 3e-5 at scores of +-100, where the
+ *      exact kernel itself is at 1e-5).  A device-side range check sends a call with |x| >= 2^15 or a non-finite Q, K or V
+ *      to the exact CUDA-core kernel, which also takes every other shape.  Calls with few query rows per K/V head take
+ *      the decoding kernel (exact fp32 products). */
 TX_API int tx_sdpa_naive_cuda(const float *Q, const float *K, const float *V, const float *mask,
                               float *out, int64_t batch_size, int64_t num_heads,
                               int64_t seq_len_q, int64_t seq_len_k, int64_t d_k, int64_t d_v);
@@ -181,7 +182,8 @@ TX_API int tx_sdpa_forward(const tx_sdpa_desc *desc);
  * between return at once and write NaN. */
 TX_API int tx_sdpa_finish(void *stream);
 /* 1 if tx_sdpa_forward would run `desc` on a tcgen05 kernel (fp16, or fp32 as hi/lo fp16 pairs), 0 if on CUDA cores.
- * (For fp32 the answer is about the shape: a value outside the pairs' range still sends the call to CUDA cores.)
+ * (For fp32 the answer is about the shape: a value outside the pairs' range still sends the call to CUDA cores; and it is 1
+ * for the unmasked head dims 64 and 128 only, although masked calls and the head dims between run on the same kernel.)
  * Calls with few query rows per K/V head -- decoding steps, up to 16 rows in fp16 and 32 in fp32 -- run on a kernel of
  * their own that reads the cache once and is bound by memory, not arithmetic: 0. */
 TX_API int tx_sdpa_uses_tensor_cores(const tx_sdpa_desc *desc);

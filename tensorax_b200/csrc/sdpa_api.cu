@@ -32,10 +32,10 @@
 
 #include "linear_simt.cuh"
 #include "linear_tc.cuh"
-#include "sdpa_simt.cuh"
 #include "sdpa_tc.cuh"
 #include "sdpa_tc_pair.cuh"
 #include "sdpa_tc_x3.cuh"
+#include "sdpa_simt.cuh"
 #include "sdpa_bwd.cuh"
 #include "sdpa_decode.cuh"
 
@@ -336,6 +336,14 @@ int launch_simt_t(const txb::SimtParams &p, cudaStream_t st)
 {
     dim3 grid((unsigned)((p.dv + 32 * DVC - 1) / (32 * DVC)),
               (unsigned)((p.Sq + txb::SIMT_BR - 1) / txb::SIMT_BR), (unsigned)(p.B * p.Hq));
+    if (p.only_if) {
+        // a stand-in that nearly always has nothing to do: one wave of CTAs that walk the items if they must (a CTA
+        // each took 6.7 us to find that out at 2048 items)
+        int sms = 0;
+        if (int rc = sm_count(&sms)) return rc;
+        grid.y = std::min<unsigned>(grid.y, (unsigned)sms);
+        grid.z = std::min<unsigned>(grid.z, std::max(1u, (unsigned)sms / grid.y));
+    }
     txb::sdpa_simt_kernel<T, DVC, PROF><<<grid, txb::SIMT_THREADS, 0, st>>>(p);
     g_launches++;
     TX_CUDA(cudaGetLastError());
@@ -689,9 +697,10 @@ int forward_f32_via_f16(const tx_sdpa_desc *d, cudaStream_t st)
 // fp32 in, fp32 out on the fp16 tensor cores (three products per GEMM, sdpa_tc_x3.cuh) for the calls that fit it.
 bool x3_eligible(const tx_sdpa_desc *d)
 {
-    if (d->dtype != TX_DTYPE_F32 || d->mask || d->lse) return false;
+    if (d->dtype != TX_DTYPE_F32 || d->lse) return false;
     if (d->flags & (TX_SDPA_FORCE_SIMT | TX_SDPA_OUT_F16 | TX_SDPA_P_IN_SMEM)) return false;
-    if (d->d_k != d->d_v || (d->d_k != 64 && d->d_k != 128)) return false;
+    // rows of whole 16-byte pieces (the split pass reads them, bulk tensor stores write the result)
+    if (d->d_k > 128 || d->d_v > 128 || d->d_k % 4 || d->d_v % 4) return false;
     auto al = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     if (!al(d->q) || !al(d->k) || !al(d->v) || !al(d->out)) return false;
     // the exact kernel stands behind it and must be launchable for the same call
@@ -716,45 +725,54 @@ void fill_simt_params(txb::SimtParams *p, const tx_sdpa_desc *d)
 template <class Cfg>
 int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
 {
-    const int64_t nq = d->batch * d->q_heads * d->seq_q * d->d_k, nk = d->batch * d->kv_heads * d->seq_k * d->d_k;
-    // workspace: hi and lo fp16 copies of Q, K, V and the range flag, stream-ordered pool memory
-    const size_t bq = align_up((size_t)nq * 2, 256), bk = align_up((size_t)nk * 2, 256);
-    const size_t o_qh = 0, o_ql = bq, o_kh = 2 * bq, o_kl = o_kh + bk, o_vh = o_kl + bk, o_vl = o_vh + bk, o_flag = o_vl + bk;
+    const int64_t rows_q = d->batch * d->q_heads * d->seq_q, rows_k = d->batch * d->kv_heads * d->seq_k;
+    const int64_t dk8 = (d->d_k + 7) / 8 * 8, dv8 = (d->d_v + 7) / 8 * 8;       // row length of the fp16 copies
+    // workspace: hi and lo fp16 copies of Q, K, V and the range words, stream-ordered pool memory
+    const size_t bq = align_up((size_t)(rows_q * dk8) * 2, 256), bk = align_up((size_t)(rows_k * dk8) * 2, 256),
+                 bv = align_up((size_t)(rows_k * dv8) * 2, 256);
+    const size_t o_qh = 0, o_ql = bq, o_kh = 2 * bq, o_kl = o_kh + bk, o_vh = o_kl + bk, o_vl = o_vh + bv, o_flag = o_vl + bv;
     char *ws = nullptr;
     if (int rc = pool_alloc(&ws, o_flag + 256, st)) return rc;
     int rc = TX_OK;
     auto body = [&]() -> int {
-        int *flag = reinterpret_cast<int *>(ws + o_flag);
-        TX_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
+        int *range = reinterpret_cast<int *>(ws + o_flag);
+        TX_CUDA(cudaMemsetAsync(range, 0, 2 * sizeof(int), st));
         txb::SplitParams sp;
-        sp.seg[0] = {static_cast<const float *>(d->q), reinterpret_cast<__half *>(ws + o_qh), reinterpret_cast<__half *>(ws + o_ql), nq};
-        sp.seg[1] = {static_cast<const float *>(d->k), reinterpret_cast<__half *>(ws + o_kh), reinterpret_cast<__half *>(ws + o_kl), nk};
-        sp.seg[2] = {static_cast<const float *>(d->v), reinterpret_cast<__half *>(ws + o_vh), reinterpret_cast<__half *>(ws + o_vl), nk};
-        sp.flag = flag;
+        auto seg = [&](const void *x, size_t hi, size_t lo, int64_t rows, int64_t n, int64_t n8) {
+            return txb::SplitSeg{static_cast<const float *>(x), reinterpret_cast<__half *>(ws + hi), reinterpret_cast<__half *>(ws + lo),
+                                 rows * n8 / 4, (int)(n / 4), (int)(n8 / 4)};
+        };
+        sp.seg[0] = seg(d->q, o_qh, o_ql, rows_q, d->d_k, dk8);
+        sp.seg[1] = seg(d->k, o_kh, o_kl, rows_k, d->d_k, dk8);
+        sp.seg[2] = seg(d->v, o_vh, o_vl, rows_k, d->d_v, dv8);
+        sp.range = range;
         int sms = 0;
         if (int r = sm_count(&sms)) return r;
-        const int64_t want = (std::max(nq, nk) / 4 + 255) / 256;
+        const int64_t want = (std::max({sp.seg[0].n4, sp.seg[1].n4, sp.seg[2].n4}) + 255) / 256;
         txb::split_f32_hi_lo_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(want, 16 * sms)), 256, 0, st>>>(sp);
         g_launches++;
         TX_CUDA(cudaGetLastError());
 
         CUtensorMap qh, ql, kh, kl, vh, vl, to;
         const int64_t sq = d->batch * d->q_heads, sk = d->batch * d->kv_heads;
-        if (int r = make_map(&qh, ws + o_qh, sq, d->seq_q, d->d_k, Cfg::BM)) return r;
-        if (int r = make_map(&ql, ws + o_ql, sq, d->seq_q, d->d_k, Cfg::BM)) return r;
-        if (int r = make_map(&kh, ws + o_kh, sk, d->seq_k, d->d_k, Cfg::BN)) return r;
-        if (int r = make_map(&kl, ws + o_kl, sk, d->seq_k, d->d_k, Cfg::BN)) return r;
-        if (int r = make_map(&vh, ws + o_vh, sk, d->seq_k, d->d_v, Cfg::BN)) return r;
-        if (int r = make_map(&vl, ws + o_vl, sk, d->seq_k, d->d_v, Cfg::BN)) return r;
+        if (int r = make_map(&qh, ws + o_qh, sq, d->seq_q, dk8, Cfg::BM)) return r;
+        if (int r = make_map(&ql, ws + o_ql, sq, d->seq_q, dk8, Cfg::BM)) return r;
+        if (int r = make_map(&kh, ws + o_kh, sk, d->seq_k, dk8, Cfg::BN)) return r;
+        if (int r = make_map(&kl, ws + o_kl, sk, d->seq_k, dk8, Cfg::BN)) return r;
+        if (int r = make_map(&vh, ws + o_vh, sk, d->seq_k, dv8, Cfg::BN)) return r;
+        if (int r = make_map(&vl, ws + o_vl, sk, d->seq_k, dv8, Cfg::BN)) return r;
         if (int r = make_map(&to, d->out, sq, d->seq_q, d->d_v, 32, 4)) return r;
         txb::X3Params p;
         p.out = static_cast<float *>(d->out);
+        p.mask = d->mask;
         p.kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
-        p.out_of_range = flag;
+        p.range = range;
         p.status = status;
         p.Hq = (int)d->q_heads; p.Hkv = (int)d->kv_heads; p.Sq = (int)d->seq_q; p.Sk = (int)d->seq_k;
+        p.dk = (int)d->d_k; p.dv = (int)d->d_v;
         p.causal = d->causal ? 1 : 0;
-        p.scale_log2 = (1.0f / std::sqrt((float)d->d_k)) * 1.4426950408889634f;
+        p.scale = 1.0f / std::sqrt((float)d->d_k);
+        p.scale_log2 = p.scale * 1.4426950408889634f;
         const int64_t n_tiles = (d->seq_q + Cfg::BM - 1) / Cfg::BM;
         int64_t group = 1;
         if (int r = causal_group(d, n_tiles, &group)) return r;
@@ -767,7 +785,7 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
         // the exact kernel behind it: works only when the split pass found a value the fp16 pairs cannot carry
         txb::SimtParams sp2;
         fill_simt_params(&sp2, d);
-        sp2.only_if = flag;
+        sp2.only_if = range;
         return launch_simt<float>(sp2, st);
     };
     rc = body();
@@ -777,8 +795,9 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
 
 int launch_x3(const tx_sdpa_desc *d, cudaStream_t st, int *status)
 {
-    if (d->d_k == 64) return launch_x3_t<txb::X3Cfg<64, 4>>(d, st, status);
-    return launch_x3_t<txb::X3Cfg<128, 2>>(d, st, status);
+    const bool narrow = d->d_k <= 64 && d->d_v <= 64;
+    if (d->mask) return narrow ? launch_x3_t<txb::X3Cfg<64, 2, true>>(d, st, status) : launch_x3_t<txb::X3Cfg<128, 2, true>>(d, st, status);
+    return narrow ? launch_x3_t<txb::X3Cfg<64, 4>>(d, st, status) : launch_x3_t<txb::X3Cfg<128, 2>>(d, st, status);
 }
 
 int forward_launch(const tx_sdpa_desc *d)
@@ -1489,7 +1508,9 @@ int tx_sdpa_uses_tensor_cores(const tx_sdpa_desc *desc)
         probe.dtype = TX_DTYPE_F16;
         return tc_eligible(&probe) ? 1 : 0;
     }
-    return (tc_eligible(desc) || x3_eligible(desc)) ? 1 : 0;
+    if (tc_eligible(desc)) return 1;
+    const bool plain = !desc->mask && desc->d_k == desc->d_v && (desc->d_k == 64 || desc->d_k == 128);
+    return (plain && x3_eligible(desc)) ? 1 : 0;
 }
 
 int64_t tx_kernel_launch_count(void) { return g_launches.load(); }

@@ -27,6 +27,7 @@
 #include <cstdint>
 
 #include "kv_lens.cuh"
+#include "sdpa_tc_x3.cuh"
 
 namespace txb {
 
@@ -40,7 +41,7 @@ struct SimtParams {
     int out_f16;
     float scale;
     long long *prof;         // optional [32]: clock64 stamps of CTA (0,0,0), thread 0 (PROF instantiation only)
-    const int *only_if = nullptr;   // optional device word: the launch does nothing while it is 0 (this kernel as the
+    const int *only_if = nullptr;   // optional: the launch does nothing unless x3_declines(only_if) (this kernel as the
                                     // stand-in behind a faster one that found it could not take the call)
 };
 
@@ -75,7 +76,7 @@ sdpa_simt_kernel(const SimtParams p)
                 p.prof[i] = clock64();
         }
     };
-    if (p.only_if && *reinterpret_cast<const volatile int *>(p.only_if) == 0) return;
+    if (p.only_if && !x3_declines(p.only_if)) return;
     stamp(SIMT_T_START);
     __shared__ float q_s[SIMT_BR][SIMT_DKC + 1];
     __shared__ float k_s[SIMT_BC][SIMT_DKC + 1];
@@ -86,11 +87,12 @@ sdpa_simt_kernel(const SimtParams p)
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    const int64_t bh = blockIdx.z;                 // b*Hq + h
+    // one (batch, head) and row block per CTA, more only where the launch was given fewer CTAs than items
+    for (int64_t bh = blockIdx.z; bh < p.B * p.Hq; bh += gridDim.z)        // b*Hq + h
+    for (int64_t q0 = (int64_t)blockIdx.y * SIMT_BR; q0 < p.Sq; q0 += (int64_t)gridDim.y * SIMT_BR) {
     const int64_t b = bh / p.Hq;
     const int64_t h = bh % p.Hq;
     const int64_t kvh = b * p.Hkv + h / (p.Hq / p.Hkv);
-    const int64_t q0 = (int64_t)blockIdx.y * SIMT_BR;
     const int64_t dv0 = (int64_t)blockIdx.x * (32 * DVC);
 
     const T *Q = static_cast<const T *>(p.q) + bh * p.Sq * p.dk;
@@ -229,6 +231,8 @@ sdpa_simt_kernel(const SimtParams p)
         }
     }
     stamp(SIMT_T_STORED);
+    __syncthreads();        // the next item reuses the shared arrays
+    }
 }
 
 }  // namespace txb

@@ -3,14 +3,15 @@
 //     S  = Qhi Klo^T + Qlo Khi^T + Qhi Khi^T          O += Phi Vlo + Plo Vhi + Phi Vhi
 // accumulated in fp32 in tensor memory (the lo*lo term is below fp32's own rounding).  It stands where the
 // reference's fp32 kernels do (tensorax csrc/cuda/kernels/attn.cu:296-656 sdpa_kernel_mma and the naive / tiled /
-// flash forms before it) for the calls that fit it: no dense mask, d_k = d_v in {64, 128}, |x| < 2^15 everywhere.
+// flash forms before it) for head dims up to 128 (multiples of 4; d_k and d_v may differ), with or without a dense
+// additive mask, for |x| < 2^15 everywhere.
 // The split pass that writes the hi / lo copies also checks the range and raises a device flag when a value does
 // not fit; this kernel then returns at once and the exact CUDA-core kernel, launched behind it, does the work.
 //
 // One CTA per SM and 128-row query tile, 64 keys per tile:
 //   warp 0        TMA producer: Q hi / lo once, then K hi / lo and V hi / lo of every key tile through an NS-deep ring
 //   warp 1        issues the MMAs: QK^T of tile j+1 as soon as the softmax warps have S_j in registers, then PV of tile j
-//   warps 2-3     idle
+//   warps 2-3     idle, or bring the dense mask's [128 rows][64 keys] tile to shared memory (cp.async: any row length)
 //   warps 4-7     softmax, thread = row = tensor-memory lane: fp32 online softmax with the exact running max
 //                 (full-precision `ex2.approx`, no polynomial), P split into hi / lo in registers and stored to
 //                 tensor memory as two fp16 operands; the row's rescale factor of the tile goes to shared memory
@@ -19,17 +20,27 @@
 //                 tensor core's own fp32 accumulation truncates, and carried over hundreds of key tiles that bias
 //                 grows with the sequence length; twelve steps of it stay below fp32's rounding of the result.
 //                 They also write the result (staged bulk tensor stores).
+// The operands are the split pass's fp16 copies, their rows padded to a multiple of 8; the last 64-column panel is
+// filled with zeros by the TMA unit, QK^T runs ceil(d_k / 16) steps and PV's N is d_v rounded up to 16, so a head dim
+// between the two template sizes costs what it needs (fp32 B2 H8 S1000 d80: 608 -> 62 us a call against the CUDA-core kernel).
+// Dense mask: scores stay in the natural-log domain (x = s * scale + mask, p = 2^((x - m) log2 e)) with the running max
+// starting at -FLT_MAX, so that rows masked by the lowest floats average V and rows masked by -inf are 0/0, as in the
+// reference (fp32 B4 H8 S512 d64: 275 -> 56 us a call).
 // Tensor memory: S 64 | Phi 32 | Plo 32 | PV_0 D | PV_1 D columns.
 // Every mbarrier wait is bounded, as in the fp16 kernels.
 #pragma once
+#include <cfloat>
+
 #include "ptx.cuh"
 #include "sdpa_tc.cuh"
 
 namespace txb {
 
-template <int D_, int NS_>
+template <int D_, int NS_, bool MASK_ = false>
 struct X3Cfg {
-    static constexpr int D = D_, NS = NS_;
+    static constexpr int D = D_, NS = NS_;                 // D: 64 or 128, at least d_k and d_v
+    static constexpr bool MASK = MASK_;
+    static constexpr int NM = D_ == 64 ? 2 : 1;            // stages of the mask tile
     static constexpr int BM = 128, BN = 64;
     static constexpr int THREADS = 384;
     // registers: producer / MMA warpgroup, softmax warpgroup, accumulator warpgroup (128 * (56 + 192 + 248) <= 384 * 168)
@@ -41,29 +52,43 @@ struct X3Cfg {
     static constexpr uint32_t OFF_QH = 0, OFF_QL = Q_BYTES;
     static constexpr uint32_t OFF_K = 2 * Q_BYTES;         // per stage: K hi | K lo
     static constexpr uint32_t OFF_V = OFF_K + NS * 2 * KV_BYTES;
-    static constexpr uint32_t OFF_BAR = OFF_V + NS * 2 * KV_BYTES;
+    static constexpr uint32_t MASK_BYTES = BM * BN * 4;
+    static constexpr uint32_t OFF_MASK = OFF_V + NS * 2 * KV_BYTES;
+    static constexpr uint32_t OFF_BAR = OFF_MASK + (MASK ? NM * MASK_BYTES : 0);
     // q_full s_full s_free p_full l_full pv_done[2] pv_free[2] alpha_full[4] k_full[NS] k_empty[NS] v_full[NS] v_empty[NS]
-    static constexpr int N_BARS = 13 + 4 * NS;
+    // mask_full[NM] mask_empty[NM]
+    static constexpr int N_BARS = 13 + 4 * NS + (MASK ? 2 * NM : 0);
     static constexpr uint32_t OFF_ALPHA = OFF_BAR + ((N_BARS * 8 + 15) / 16) * 16;   // [4][BM] rescale factors, then [BM] row sums
     static constexpr uint32_t OFF_TMEM = OFF_ALPHA + 5 * BM * 4;
     static constexpr uint32_t OFF_ABORT = OFF_TMEM + 4;
     static constexpr uint32_t SMEM_BYTES = ((OFF_ABORT + 4 + 127) / 128) * 128;
     static constexpr uint32_t COL_S = 0, COL_PH = BN, COL_PL = BN + BN / 2, COL_PV0 = 2 * BN, COL_PV1 = 2 * BN + D;
     static constexpr uint32_t TMEM_COLS = 512;
-    static_assert(D == 64 || D == 128, "head dim");
+    static_assert(D == 64 || D == 128, "operand width");
     static_assert(2 * BN + 2 * D <= TMEM_COLS, "tensor memory");
     static_assert(SMEM_BYTES <= 232448, "more than the 227 KB a CTA may have");
     static_assert(Q_BYTES / 4 >= 4096, "a softmax warp stages its results in its quarter of the Q buffers");
 };
 
+// range[0]: some |x| >= 2^15 or not finite.  range[1]: the bits of max |v|: a pair is exact to 2^-25 absolutely, which is
+// fp32-grade against a V of ordinary size only (errors of Q and K act on the scores absolutely, so small ones do no harm).
+__device__ __forceinline__ bool x3_declines(const int *range)
+{
+    const volatile int *w = range;
+    return w[0] != 0 || (w[1] != 0 && __int_as_float(w[1]) < 0.0625f);
+}
+
 struct X3Params {
-    float *out;               // [B,Hq,Sq,D] fp32
+    float *out;               // [B,Hq,Sq,dv] fp32
+    const float *mask;        // dense additive [B,Hq,Sq,Sk] (MASK instantiations)
     KvLens kv_lens;           // optional [B]
-    const int *out_of_range;  // device word the split pass sets: nonzero = this kernel does nothing
+    const int *range;         // the split pass's two words (see x3_declines)
     int *status;              // device word: 0 = ok, else first failing wait's code
     int Hq, Hkv, Sq, Sk;
+    int dk, dv;
     int causal;
-    float scale_log2;         // (1/sqrt(d_k)) * log2(e)
+    float scale;              // 1/sqrt(d_k)
+    float scale_log2;         // scale * log2(e)
     int group, n_tiles_q, BH; // work-item order, as in sdpa_tc_pair_kernel (query tiles in place of pairs)
 };
 
@@ -75,7 +100,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                   const __grid_constant__ CUtensorMap tm_o, const X3Params p)
 {
     constexpr int D = Cfg::D, BN = Cfg::BN, NS = Cfg::NS, BM = Cfg::BM;
-    if (*reinterpret_cast<const volatile int *>(p.out_of_range) != 0) return;   // the exact kernel takes this call
+    if (x3_declines(p.range)) return;                            // the exact kernel takes this call
 
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = ptx::smem_u32(smem);
@@ -90,6 +115,8 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
     // its barrier never a phase ahead, while its reader still needs it.
     const uint32_t alpha_full = bar0 + 72;
     const uint32_t k_full = bar0 + 104, k_empty = k_full + 8 * NS, v_full = k_empty + 8 * NS, v_empty = v_full + 8 * NS;
+    const uint32_t mask_full = v_empty + 8 * NS, mask_empty = mask_full + 8 * Cfg::NM;
+    const int kp_k = (p.dk + 63) / 64, kp_v = (p.dv + 63) / 64;  // 64-column panels that hold something
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(smem + Cfg::OFF_TMEM);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + Cfg::OFF_ABORT);
 
@@ -110,10 +137,11 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
     const int kv_end = p.causal ? min(kv_limit, q0 + BM) : kv_limit;
     const int nt = (kv_end + BN - 1) / BN;
 
-    auto load_kv = [&](uint32_t dst, const CUtensorMap *hi, const CUtensorMap *lo, uint32_t bar, int j) {
-        ptx::mbar_arrive_expect_tx(bar, 2 * Cfg::KV_BYTES);
+    auto load_kv = [&](uint32_t dst, const CUtensorMap *hi, const CUtensorMap *lo, uint32_t bar, int j, int panels) {
+        ptx::mbar_arrive_expect_tx(bar, 2 * Cfg::KV_PANEL * (uint32_t)panels);
 #pragma unroll
         for (int pn = 0; pn < Cfg::KP; ++pn) {
+            if (pn >= panels) break;
             ptx::tma_load_3d(dst + pn * Cfg::KV_PANEL, hi, bar, pn * 64, j * BN, kvh);
             ptx::tma_load_3d(dst + Cfg::KV_BYTES + pn * Cfg::KV_PANEL, lo, bar, pn * 64, j * BN, kvh);
         }
@@ -139,6 +167,11 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                 ptx::mbar_init(v_full + 8 * s, 1);
                 ptx::mbar_init(v_empty + 8 * s, 1);
             }
+            if constexpr (Cfg::MASK)
+                for (int t = 0; t < Cfg::NM; ++t) {
+                    ptx::mbar_init(mask_full + 8 * t, 64);       // every loading thread's copies
+                    ptx::mbar_init(mask_empty + 8 * t, 4);
+                }
             ptx::fence_mbar_init();
             if (sbase & 1023u) {
                 *abort_flag = 1;
@@ -146,14 +179,15 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
             } else if (nt > 0) {
                 ptx::prefetch_tmap(&tm_qh);
                 ptx::prefetch_tmap(&tm_kh);
-                ptx::mbar_arrive_expect_tx(q_full, 2 * Cfg::Q_BYTES);
+                ptx::mbar_arrive_expect_tx(q_full, 2 * BM * 128 * (uint32_t)kp_k);
 #pragma unroll
                 for (int pn = 0; pn < Cfg::KP; ++pn) {
+                    if (pn >= kp_k) break;
                     ptx::tma_load_3d(qh_s + pn * (BM * 128), &tm_qh, q_full, pn * 64, q0, bh);
                     ptx::tma_load_3d(ql_s + pn * (BM * 128), &tm_ql, q_full, pn * 64, q0, bh);
                 }
-                load_kv(k_s, &tm_kh, &tm_kl, k_full, 0);
-                load_kv(v_s, &tm_vh, &tm_vl, v_full, 0);
+                load_kv(k_s, &tm_kh, &tm_kl, k_full, 0, kp_k);
+                load_kv(v_s, &tm_vh, &tm_vl, v_full, 0, kp_v);
             }
             if (*reinterpret_cast<volatile int *>(p.status) != 0) *abort_flag = 1;   // an earlier CTA gave up
         }
@@ -181,11 +215,11 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                 const uint32_t ph = (uint32_t)(j / NS) & 1u;
                 ok = ptx::mbar_wait(k_empty + 8 * s, ph ^ 1u, abort_flag);
                 if (!ok) break;
-                if (leader) load_kv(k_s + s * 2 * Cfg::KV_BYTES, &tm_kh, &tm_kl, k_full + 8 * s, j);
+                if (leader) load_kv(k_s + s * 2 * Cfg::KV_BYTES, &tm_kh, &tm_kl, k_full + 8 * s, j, kp_k);
                 __syncwarp();
                 ok = ptx::mbar_wait(v_empty + 8 * s, ph ^ 1u, abort_flag);
                 if (!ok) break;
-                if (leader) load_kv(v_s + s * 2 * Cfg::KV_BYTES, &tm_vh, &tm_vl, v_full + 8 * s, j);
+                if (leader) load_kv(v_s + s * 2 * Cfg::KV_BYTES, &tm_vh, &tm_vl, v_full + 8 * s, j, kp_v);
                 __syncwarp();
             }
             if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, TC_ERR_PRODUCER); }
@@ -196,7 +230,8 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
         if (run) {
             const bool leader = ptx::elect_one();
             constexpr uint32_t idesc_qk = ptx::idesc_f16(BM, BN, false);
-            constexpr uint32_t idesc_pv = ptx::idesc_f16(BM, D, true);
+            const uint32_t idesc_pv = ptx::idesc_f16(BM, (p.dv + 15) / 16 * 16, true);
+            const int steps = (p.dk + 15) / 16;
             constexpr uint32_t desc_hi = ptx::smem_desc_sw128_hi(1024);
             const uint32_t qh_lo = ptx::smem_desc_sw128_lo(qh_s, 16), ql_lo = ptx::smem_desc_sw128_lo(ql_s, 16);
             const uint32_t k_lo = ptx::smem_desc_sw128_lo(k_s, 16);
@@ -217,6 +252,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                         const uint32_t kb0 = c == 0 ? kl : kh;
 #pragma unroll
                         for (int kk = 0; kk < D / 16; ++kk) {
+                            if (kk >= steps) break;
                             const uint32_t qa = ((kk >> 2) * (BM * 128) + (kk & 3) * 32) >> 4;
                             const uint32_t kb = ((kk >> 2) * Cfg::KV_PANEL + (kk & 3) * 32) >> 4;
                             ptx::mma_ss(t_s, ptx::make_desc(qa0 + qa, desc_hi), ptx::make_desc(kb0 + kb, desc_hi),
@@ -268,6 +304,38 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
             }
             if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, TC_ERR_MMA); }
         }
+    } else if constexpr (Cfg::MASK) {
+        // ------------------------------------------------------------ mask loader (warps 2, 3)
+        // 16-byte copies where the mask's rows are 16-byte aligned, 4-byte ones otherwise; a 256-byte tile row keeps its
+        // 16-byte chunks at chunk ^ (row & 7), which is what lets 8 softmax threads read 8 rows without bank conflicts.
+        if (run) {
+            const int t = (warp - 2) * 32 + lane;                // 0..63
+            const float *base = p.mask + ((size_t)bh * p.Sq + q0) * p.Sk;
+            const bool wide = (p.Sk & 3) == 0 && (reinterpret_cast<uintptr_t>(p.mask) & 15u) == 0;
+            const int rows = min(BM, p.Sq - q0);
+            bool ok = true;
+            for (int j = 0; j < nt && ok; ++j) {
+                const int s = j % Cfg::NM;
+                if (j >= Cfg::NM) ok = ptx::mbar_wait(mask_empty + 8 * s, ((uint32_t)(j / Cfg::NM) & 1u) ^ 1u, abort_flag);
+                if (!ok) break;
+                const uint32_t dst = sbase + Cfg::OFF_MASK + (uint32_t)s * Cfg::MASK_BYTES;
+                const int kv0 = j * BN;
+                if (wide) {
+                    const int c = t & 15;                        // chunk of the row: 16 threads a row, 4 rows a step
+                    const bool in = kv0 + c * 4 < p.Sk;
+                    for (int row = t >> 4; row < rows; row += 4)
+                        if (in) ptx::cp_async16(dst + (uint32_t)row * 256 + ((uint32_t)(c ^ (row & 7)) << 4), base + (size_t)row * p.Sk + kv0 + c * 4);
+                } else {
+                    const bool in = kv0 + t < p.Sk;
+                    for (int row = 0; row < rows; ++row)
+                        if (in) ptx::cp_async4(dst + (uint32_t)row * 256 + ((uint32_t)((t >> 2) ^ (row & 7)) << 4) + (t & 3) * 4,
+                                               base + (size_t)row * p.Sk + kv0 + t);
+                }
+                ptx::cp_async_arrive(mask_full + 8 * s);
+            }
+            if (!ok && lane == 0) { *abort_flag = 1; ptx::report(p.status, TC_ERR_PRODUCER); }
+            ptx::cp_async_wait_all();
+        }
     }
     } else if (warp < 8) {
         ptx::setmaxnreg_inc<Cfg::REGS_SOFTMAX>();
@@ -278,8 +346,9 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         const uint32_t t_s = tmem + lane_base + Cfg::COL_S;
         const uint32_t t_ph = tmem + lane_base + Cfg::COL_PH, t_pl = tmem + lane_base + Cfg::COL_PL;
-        const float scale = p.scale_log2;
-        float m_run = -1.0e30f;    // finite stand-in for "no key seen yet"
+        constexpr float kLog2e = 1.4426950408889634f;
+        const float scale = Cfg::MASK ? kLog2e : p.scale_log2;
+        float m_run = Cfg::MASK ? -FLT_MAX : -1.0e30f;           // finite stand-in for "no key seen yet"
         float l = 0.f;
         bool ok = run;
         auto arrive_warp = [&](uint32_t bar) {
@@ -297,6 +366,23 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
             ptx::tmem_wait_ld();
             ptx::reg_fence_cols<BN>(sv);
             arrive_warp(s_free);                         // S belongs to the MMA warp again
+            if constexpr (Cfg::MASK) {
+                const int sm_ = j % Cfg::NM;
+                ok = ptx::mbar_wait(mask_full + 8 * sm_, (uint32_t)(j / Cfg::NM) & 1u, abort_flag);
+                if (!ok) break;
+                const uint32_t mrow = sbase + Cfg::OFF_MASK + (uint32_t)sm_ * Cfg::MASK_BYTES + (uint32_t)r * 256;
+#pragma unroll
+                for (int i = 0; i < BN; i += 4) {
+                    uint32_t a, b2, c, d;
+                    ptx::ld_shared_v4(mrow + ((uint32_t)((i >> 2) ^ (r & 7)) << 4), a, b2, c, d);
+                    sv[i] = __float_as_uint(fmaf(__uint_as_float(sv[i]), p.scale, __uint_as_float(a)));
+                    sv[i + 1] = __float_as_uint(fmaf(__uint_as_float(sv[i + 1]), p.scale, __uint_as_float(b2)));
+                    sv[i + 2] = __float_as_uint(fmaf(__uint_as_float(sv[i + 2]), p.scale, __uint_as_float(c)));
+                    sv[i + 3] = __float_as_uint(fmaf(__uint_as_float(sv[i + 3]), p.scale, __uint_as_float(d)));
+                }
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(mask_empty + 8 * sm_);
+            }
             const bool need_mask = (kv0 + BN > kv_limit) || (p.causal && (kv0 + BN - 1 > q0));
             if (need_mask) {
                 // visible keys of this row are a prefix of the tile: columns [0, lim)
@@ -313,8 +399,8 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                 mx3 = ptx::max3(mx3, __uint_as_float(sv[i + 6]), __uint_as_float(sv[i + 7]));
             }
             const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-            const float m_next = fmaxf(m_run, mx * scale);          // exact running max: every p <= 1
-            const float alpha = ptx::ex2_approx(m_run - m_next);
+            const float m_next = fmaxf(m_run, Cfg::MASK ? mx : mx * scale);   // exact running max: every p <= 1
+            const float alpha = ptx::ex2_approx(Cfg::MASK ? (m_run - m_next) * kLog2e : m_run - m_next);
             m_run = m_next;
             alpha_s[(j & 3) * BM + r] = alpha;                      // for the accumulator thread of this row
             __syncwarp();
@@ -325,8 +411,11 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
             uint32_t pkh[BN / 2], pkl[BN / 2];
 #pragma unroll
             for (int i = 0; i < BN; i += 4) {
-                const float2 xa = __ffma2_rn(make_float2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), scale2, negm2);
-                const float2 xb = __ffma2_rn(make_float2(__uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3])), scale2, negm2);
+                const float2 sa = make_float2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
+                const float2 sb = make_float2(__uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3]));
+                // masked: the difference first, then the scaling (both terms may be as large as floats get)
+                const float2 xa = Cfg::MASK ? __fmul2_rn(__fadd2_rn(sa, negm2), scale2) : __ffma2_rn(sa, scale2, negm2);
+                const float2 xb = Cfg::MASK ? __fmul2_rn(__fadd2_rn(sb, negm2), scale2) : __ffma2_rn(sb, scale2, negm2);
                 const float2 ea = make_float2(ptx::ex2_approx(xa.x), ptx::ex2_approx(xa.y));
                 const float2 eb = make_float2(ptx::ex2_approx(xb.x), ptx::ex2_approx(xb.y));
                 sum_a = __fadd2_rn(sum_a, ea);
@@ -359,8 +448,8 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
         if (run && !ok) { *abort_flag = 1; ptx::report(p.status, TC_ERR_SOFTMAX); }
         if (nt == 0 && *abort_flag == 0 && row < p.Sq) {
             // no visible key at all for this tile: the reference's 0/0
-            float *orow = p.out + ((size_t)bh * p.Sq + row) * D;
-            for (int i = 0; i < D; ++i) orow[i] = __int_as_float(0x7fc00000);
+            float *orow = p.out + ((size_t)bh * p.Sq + row) * p.dv;
+            for (int i = 0; i < p.dv; ++i) orow[i] = __int_as_float(0x7fc00000);
         }
     } else {
         ptx::setmaxnreg_inc<Cfg::REGS_ACC>();
@@ -383,6 +472,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
             const uint32_t t_pv = tmem + lane_base + (a ? Cfg::COL_PV1 : Cfg::COL_PV0);
 #pragma unroll
             for (int c = 0; c < D / 32; ++c) {
+                if (c * 32 >= p.dv) break;
                 uint32_t t[32];
                 ptx::tmem_ld32(t_pv + c * 32, t);
                 ptx::tmem_wait_ld();
@@ -413,7 +503,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                 auto send = [&](uint32_t buf, int col) {
                     ptx::fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0 && row0 < p.Sq) {
+                    if (lane == 0 && row0 < p.Sq && col < p.dv) {
                         ptx::tma_store_3d(&tm_o, buf, col, row0, bh);
                         ptx::tma_store_commit();
                     }
@@ -448,8 +538,8 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
         if (warp >= 4 && warp < 8) {
             const int row_a = q0 + (warp & 3) * 32 + lane;
             if (row_a < p.Sq) {
-                float *orow = p.out + ((size_t)bh * p.Sq + row_a) * D;
-                for (int i = 0; i < D; ++i) orow[i] = __int_as_float(0x7fc00000);
+                float *orow = p.out + ((size_t)bh * p.Sq + row_a) * p.dv;
+                for (int i = 0; i < p.dv; ++i) orow[i] = __int_as_float(0x7fc00000);
             }
         }
         for (int i = 0; i < 64; ++i) __nanosleep(2000);   // let copies in flight land
@@ -461,29 +551,37 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
     }
 }
 
-// The split pass: hi = rn_fp16(x), lo = rn_fp16(x - hi) for up to three tensors in one launch, and the range
-// check that decides between the tensor-core kernel above and the exact one (any |x| >= 2^15, or a value that is
-// not finite, raises *flag).
+// The split pass: hi = rn_fp16(x), lo = rn_fp16(x - hi) for up to three tensors in one launch, rows padded with zeros
+// to a multiple of 8, and the range check that decides between the tensor-core kernel above and the exact one (any
+// |x| >= 2^15, a value that is not finite, or only small values of V: x3_declines).
 struct SplitSeg {
     const float *x;
     __half *hi, *lo;
-    long long n;              // elements, a multiple of 4
+    long long n4;             // quads of the padded copy
+    int q4, p4;               // quads of a row: source, padded copy
 };
 struct SplitParams {
-    SplitSeg seg[3];
-    int *flag;
+    SplitSeg seg[3];          // Q, K, V
+    int *range;
 };
 
 __global__ void __launch_bounds__(256) split_f32_hi_lo_kernel(const SplitParams sp)
 {
     bool bad = false;
+    float vmax = 0.f;
     const long long stride = (long long)gridDim.x * blockDim.x;
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
         const SplitSeg s = sp.seg[t];
-        const long long n4 = s.n >> 2;
-        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
-            const float4 v = reinterpret_cast<const float4 *>(s.x)[i];
+        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < s.n4; i += stride) {
+            float4 v;
+            if (s.q4 == s.p4) {
+                v = reinterpret_cast<const float4 *>(s.x)[i];
+            } else {
+                const long long row = i / s.p4;
+                const int c = (int)(i - row * s.p4);
+                v = c < s.q4 ? reinterpret_cast<const float4 *>(s.x)[row * s.q4 + c] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
             const __half2 h01 = __floats2half2_rn(v.x, v.y), h23 = __floats2half2_rn(v.z, v.w);
             const float2 b01 = __half22float2(h01), b23 = __half22float2(h23);
             const __half2 l01 = __floats2half2_rn(v.x - b01.x, v.y - b01.y), l23 = __floats2half2_rn(v.z - b23.x, v.w - b23.y);
@@ -496,9 +594,21 @@ __global__ void __launch_bounds__(256) split_f32_hi_lo_kernel(const SplitParams 
             reinterpret_cast<uint2 *>(s.lo)[i] = ll;
             // !(|x| < 2^15) is also true for NaN
             bad |= !(fabsf(v.x) < 32768.f) || !(fabsf(v.y) < 32768.f) || !(fabsf(v.z) < 32768.f) || !(fabsf(v.w) < 32768.f);
+            if (t == 2) vmax = fmaxf(vmax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
         }
     }
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(sp.flag, 1);
+    // one atomic per CTA and word; none for a maximum that is large enough already
+    const int wmax = __reduce_max_sync(0xffffffffu, __float_as_int(vmax));
+    __shared__ int cta_max, cta_bad;
+    if (threadIdx.x == 0) { cta_max = 0; cta_bad = 0; }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) atomicMax(&cta_max, wmax);
+    if (bad) cta_bad = 1;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (cta_bad) atomicOr(sp.range, 1);
+        if (cta_max > *reinterpret_cast<volatile int *>(sp.range + 1)) atomicMax(sp.range + 1, cta_max);
+    }
 }
 
 }  // namespace txb
