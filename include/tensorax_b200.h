@@ -38,7 +38,8 @@ enum {
     TX_ERR_KERNEL = 4,     /* a kernel gave up on a bounded wait (2 s) and reported it; tx_last_error() names the
                               stage: 1 misaligned shared memory, 2/3/4 forward producer / MMA / softmax warp,
                               12/13/14 linear-kernel producer / MMA / split warps, 22/23/24 backward
-                              producer / MMA / row warps, 32/34 decoding-kernel producer / row warps */
+                              producer / MMA / row warps, 32/34 decoding-kernel producer / row warps,
+                              42/43/44 layer-GEMM producer / MMA / summing warps */
     TX_ERR_UNSUPPORTED = 5
 };
 
@@ -152,6 +153,26 @@ TX_API int tx_linear_f32_cuda(const float *x, const float *w, const float *bias,
                               int64_t batch, int64_t seq, int64_t in_features, int64_t out_features,
                               int32_t heads_in, int32_t heads_out);
 TX_API int tx_linear_set_cuda_cores_only(int on);
+
+/* ---- multi-head attention layer: the whole of MultiHeadAttention.forward (tensorax/nn/attention/layers.py:105-128) in
+ *      fp32 -- x W^T + b for queries, keys and values, attention per head, output projection -- as one stream-ordered
+ *      sequence without synchronisation.  Projections run on the fp16 tensor cores with operands as row-scaled hi + lo
+ *      pairs and fp32 sums (fp32-grade accuracy at any magnitude); embed must be a multiple of 8, the head dim of 4, pointers
+ *      16-byte aligned (else TX_ERR_UNSUPPORTED).  Does not synchronise; tx_sdpa_finish reports failures. */
+enum { TX_MHA_F16_ATTENTION = 32 };  /* flag: heads rounded to fp16 for the attention step (as cast_f32_to_f16 of them) */
+typedef struct tx_mha_desc {
+    const float *xq, *xk, *xv;              /* [batch, seq_q, embed], [batch, seq_k, embed] x 2; may be the same tensor */
+    const float *wq, *wk, *wv, *wo;         /* [embed, embed] each: [out_features, in_features] */
+    const float *bq, *bk, *bv, *bo;         /* [embed] each, or NULL */
+    const float *mask;                      /* optional dense additive [batch, heads, seq_q, seq_k] */
+    const int32_t *kv_lens;                 /* optional [batch] (device, or host with TX_SDPA_KV_LENS_HOST) */
+    float *out;                             /* [batch, seq_q, embed] */
+    int64_t batch, seq_q, seq_k, embed, heads;
+    int32_t causal;
+    int32_t flags;                          /* TX_SDPA_KV_LENS_HOST, TX_MHA_F16_ATTENTION */
+    void *stream;
+} tx_mha_desc;
+TX_API int tx_mha_forward_f32(const tx_mha_desc *desc);
 
 /* ---- general form (no reference counterpart: the reference has no fp16+mask,
  *      no implicit causal / key-length mask and no grouped K/V heads; its dense

@@ -198,6 +198,44 @@ def linear(x: TensorImpl, weight: TensorImpl, bias: Optional[TensorImpl] = None,
     return out
 
 
+def multi_head_attention(query, key, value, weights, biases, num_heads, mask=None, causal=False, kv_lens=None,
+                         fp16_attention=False) -> Optional[TensorImpl]:
+    """MultiHeadAttention.forward (tensorax/nn/attention/layers.py:105-128) as one call of the library: `weights` and
+    `biases` of the query, key, value and output projections (a bias may be None).  None where the library has no
+    such form for the shapes; anything that is wrong is left for the step-by-step form to report."""
+    tensors = [query, key, value, *weights]
+    if any(t.device != "cuda" or t.dtype != "float32" for t in tensors + [b for b in biases if b is not None]):
+        return None
+    E = weights[0]._shape[0]
+    if any(w._shape != [E, E] for w in weights) or any(b is not None and b._shape != [E] for b in biases):
+        return None
+    if any(len(t._shape) != 3 or t._shape[2] != E or t._shape[0] != query._shape[0] for t in (query, key, value)):
+        return None
+    B, Sq, _ = query._shape
+    Sk = key._shape[1]
+    if value._shape[1] != Sk or E % 8 or (E // num_heads) % 4:
+        return None
+    if mask is not None and (mask.device != "cuda" or mask.dtype != "float32" or mask._shape != [B, num_heads, Sq, Sk]):
+        return None
+    lens, flags = None, _lib.TX_MHA_F16_ATTENTION if fp16_attention else 0
+    if kv_lens is not None:
+        lens = _host_lens(kv_lens, B, "SDPA")
+        flags |= _lib.TX_SDPA_KV_LENS_HOST
+    out = TensorImpl([B, Sq, E], "float32", "cuda")
+    ptr = [t.data_ptr for t in tensors]
+    bias = [b.data_ptr if b is not None else None for b in biases]
+    desc = _lib.MhaDesc(*ptr, *bias, mask.data_ptr if mask is not None else None,
+                        ctypes.addressof(lens) if lens is not None else None, out.data_ptr, B, Sq, Sk, E, num_heads,
+                        int(bool(causal)), flags, None)
+    lib = _lib.load()
+    rc = lib.tx_mha_forward_f32(ctypes.byref(desc))
+    if rc == _lib.TX_ERR_UNSUPPORTED:
+        return None
+    _lib.check(rc)
+    _lib.check(lib.tx_sdpa_finish(None))
+    return out
+
+
 # ------------------------------------------------------------------ SDPA dispatchers
 def _validate(query, key, value, mask, who="SDPA"):
     """Validation order and messages of csrc/tensor_ops.cpp:855-898."""

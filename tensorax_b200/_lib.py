@@ -21,6 +21,8 @@ TX_SDPA_P_IN_SMEM = 2
 TX_SDPA_OUT_F16 = 4
 TX_SDPA_F32_VIA_F16 = 8
 TX_SDPA_KV_LENS_HOST = 16
+TX_MHA_F16_ATTENTION = 32
+TX_ERR_UNSUPPORTED = 5
 
 # every symbol include/tensorax_b200.h declares
 EXPORTED_SYMBOLS = (
@@ -37,6 +39,7 @@ EXPORTED_SYMBOLS = (
     "tx_sdpa_naive_profile_sections_cuda", "tx_sdpa_tiled_profile_sections_cuda", "tx_sdpa_flash_profile_sections_cuda",
     "tx_sdpa_mma_profile_sections_cuda", "tx_sdpa_optimized_flash_profile_sections_cuda",
     "tx_selftest_wait_timeout", "tx_sdpa_forward_host_copies_only", "tx_sdpa_set_group_l2_bytes",
+    "tx_mha_forward_f32",
 )
 
 
@@ -59,6 +62,18 @@ class SdpaBwdDesc(ctypes.Structure):
         ("lse", c_void_p), ("kv_lens", c_void_p), ("dq", c_void_p), ("dk", c_void_p), ("dv", c_void_p),
         ("batch", c_int64), ("q_heads", c_int64), ("kv_heads", c_int64),
         ("seq_q", c_int64), ("seq_k", c_int64), ("d", c_int64),
+        ("causal", c_int32), ("flags", c_int32), ("stream", c_void_p),
+    ]
+
+
+class MhaDesc(ctypes.Structure):
+    """Mirror of ``tx_mha_desc``."""
+    _fields_ = [
+        ("xq", c_void_p), ("xk", c_void_p), ("xv", c_void_p),
+        ("wq", c_void_p), ("wk", c_void_p), ("wv", c_void_p), ("wo", c_void_p),
+        ("bq", c_void_p), ("bk", c_void_p), ("bv", c_void_p), ("bo", c_void_p),
+        ("mask", c_void_p), ("kv_lens", c_void_p), ("out", c_void_p),
+        ("batch", c_int64), ("seq_q", c_int64), ("seq_k", c_int64), ("embed", c_int64), ("heads", c_int64),
         ("causal", c_int32), ("flags", c_int32), ("stream", c_void_p),
     ]
 
@@ -116,6 +131,7 @@ def load():
     lib.tx_sdpa_uses_tensor_cores.argtypes = [ctypes.POINTER(SdpaDesc)]
     lib.tx_sdpa_finish.argtypes = [c_void_p]
     lib.tx_sdpa_fp16_static_scratch.argtypes = [c_void_p] * 4 + [c_int64] * 6 + [c_int32, c_void_p, c_void_p]
+    lib.tx_mha_forward_f32.argtypes = [ctypes.POINTER(MhaDesc)]
     lib.tx_kernel_launch_count.restype = c_int64
     _lib = lib
     return lib

@@ -30,6 +30,7 @@
 #define TX_NVTX_RANGE(name) ((void)0)
 #endif
 
+#include "gemm_x3.cuh"
 #include "linear_simt.cuh"
 #include "linear_tc.cuh"
 #include "sdpa_tc.cuh"
@@ -849,6 +850,138 @@ int finish(cudaStream_t st)
     return TX_OK;
 }
 
+// ------------------------------------------------------------------ multi-head attention layer
+template <class Cfg>
+int launch_gemm_x3_t(const txb::GemmX3Params &p0, const __half *const *xh, const __half *const *xl, const __half *wh, const __half *wl,
+                     int64_t w_rows, cudaStream_t st)
+{
+    txb::GemmX3Params p = p0;
+    txb::GemmX3Maps maps;
+    p.n_tiles = 0;
+    for (int i = 0; i < p.n_probs; ++i) {
+        txb::GemmX3Problem &pr = p.prob[i];
+        pr.tiles_n = (p.N + Cfg::BN - 1) / Cfg::BN;
+        pr.first_tile = p.n_tiles;
+        p.n_tiles += (pr.M + Cfg::BM - 1) / Cfg::BM * pr.tiles_n;
+        if (int rc = make_map(&maps.xh[i], xh[i], 1, pr.M, p.K, Cfg::BM)) return rc;
+        if (int rc = make_map(&maps.xl[i], xl[i], 1, pr.M, p.K, Cfg::BM)) return rc;
+    }
+    if (int rc = make_map(&maps.wh, wh, 1, w_rows, p.K, Cfg::BN)) return rc;
+    if (int rc = make_map(&maps.wl, wl, 1, w_rows, p.K, Cfg::BN)) return rc;
+    int sms = 0;
+    if (int rc = sm_count(&sms)) return rc;
+    if (int rc = allow_smem<txb::gemm_x3_kernel<Cfg>>((int)Cfg::SMEM_BYTES)) return rc;
+    txb::gemm_x3_kernel<Cfg><<<(unsigned)std::min(p.n_tiles, sms), Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(maps, p);
+    g_launches++;
+    TX_CUDA(cudaGetLastError());
+    return TX_OK;
+}
+
+// Tile width by the number of rounds the persistent CTAs need: a 128 x 128 tile takes about 0.6 of a 128 x 256 one and
+// 128 x 64 about 0.4 (the narrower the tile, the more of its time goes to bringing x).
+int launch_gemm_x3(const txb::GemmX3Params &p, const __half *const *xh, const __half *const *xl, const __half *wh, const __half *wl,
+                   int64_t w_rows, cudaStream_t st)
+{
+    int sms = 0;
+    if (int rc = sm_count(&sms)) return rc;
+    auto time = [&](int bn, double tile) {
+        int64_t tiles = 0;
+        for (int i = 0; i < p.n_probs; ++i) tiles += (int64_t)((p.prob[i].M + 127) / 128) * ((p.N + bn - 1) / bn);
+        return (double)((tiles + sms - 1) / sms) * tile;
+    };
+    const double t256 = time(256, 1.0), t128 = time(128, 0.6), t64 = time(64, 0.4);
+    if (t256 <= t128 && t256 <= t64) return launch_gemm_x3_t<txb::GemmX3Cfg<256>>(p, xh, xl, wh, wl, w_rows, st);
+    if (t128 <= t64) return launch_gemm_x3_t<txb::GemmX3Cfg<128>>(p, xh, xl, wh, wl, w_rows, st);
+    return launch_gemm_x3_t<txb::GemmX3Cfg<64>>(p, xh, xl, wh, wl, w_rows, st);
+}
+
+// The whole layer on one stream: operands split, three projections in one launch (head-split, fp32 or fp16), attention,
+// its result split (heads merged on the way), output projection.  One workspace from the pool.
+int mha_launch(const tx_mha_desc *d)
+{
+    cudaStream_t st = static_cast<cudaStream_t>(d->stream);
+    int *status = nullptr;
+    if (int rc = status_word(&status)) return rc;
+    const int64_t E = d->embed, Mq = d->batch * d->seq_q, Mk = d->batch * d->seq_k;
+    const bool f16 = (d->flags & TX_MHA_F16_ATTENTION) != 0;
+    const int64_t M[3] = {Mq, Mk, Mk};
+    const float *x[3] = {d->xq, d->xk, d->xv}, *w[4] = {d->wq, d->wk, d->wv, d->wo}, *bias[3] = {d->bq, d->bk, d->bv};
+    const int64_t seq[3] = {d->seq_q, d->seq_k, d->seq_k};
+
+    size_t total = 0;
+    auto take = [&](size_t bytes) { const size_t at = total; total += align_up(bytes, 256); return at; };
+    int from[3];                                                  // inputs passed more than once are split once
+    size_t o_xh[3], o_xl[3], o_xi[3];
+    for (int i = 0; i < 3; ++i) {
+        from[i] = i;
+        for (int j = 0; j < i; ++j)
+            if (x[j] == x[i] && M[j] == M[i]) { from[i] = j; break; }
+        if (from[i] != i) { o_xh[i] = o_xh[from[i]]; o_xl[i] = o_xl[from[i]]; o_xi[i] = o_xi[from[i]]; continue; }
+        o_xh[i] = take((size_t)(M[i] * E) * 2); o_xl[i] = take((size_t)(M[i] * E) * 2); o_xi[i] = take((size_t)M[i] * 4);
+    }
+    const size_t o_wh = take((size_t)(4 * E * E) * 2), o_wl = take((size_t)(4 * E * E) * 2), o_wi = take((size_t)(4 * E) * 4);
+    const size_t es = f16 ? 2 : 4;
+    const size_t o_p[3] = {take((size_t)(Mq * E) * es), take((size_t)(Mk * E) * es), take((size_t)(Mk * E) * es)};
+    const size_t o_a = take((size_t)(Mq * E) * 4);
+    // the attention result's halves go where the inputs' were (none is needed any more and Q's are as large)
+    const size_t o_ah = o_xh[0], o_al = o_xl[0], o_ai = o_xi[0];
+
+    char *ws = nullptr;
+    if (int rc = pool_alloc(&ws, total, st)) return rc;
+    auto half_at = [&](size_t at) { return reinterpret_cast<__half *>(ws + at); };
+    auto float_at = [&](size_t at) { return reinterpret_cast<float *>(ws + at); };
+    auto body = [&]() -> int {
+        txb::SplitRowsParams sp;
+        sp.n_segs = 0; sp.rows = 0; sp.K = (int)E;
+        auto add = [&](const float *src, size_t hi, size_t lo, size_t inv, int64_t rows, int64_t first_row, int heads, int64_t S) {
+            txb::SplitRowsSeg &s = sp.seg[sp.n_segs++];
+            s.x = src; s.hi = half_at(hi) + first_row * E; s.lo = half_at(lo) + first_row * E; s.inv = float_at(inv) + first_row;
+            s.rows = (int)rows; s.heads = heads; s.S = (int)S; s.first = sp.rows;
+            sp.rows += (int)rows;
+        };
+        auto split = [&]() -> int {
+            txb::split_rows_kernel<<<(unsigned)((sp.rows + 7) / 8), 256, 0, st>>>(sp);
+            g_launches++;
+            TX_CUDA(cudaGetLastError());
+            return TX_OK;
+        };
+        for (int i = 0; i < 3; ++i)
+            if (from[i] == i) add(x[i], o_xh[i], o_xl[i], o_xi[i], M[i], 0, 0, 1);
+        for (int i = 0; i < 4; ++i) add(w[i], o_wh, o_wl, o_wi, E, i * E, 0, 1);
+        if (int rc = split()) return rc;
+
+        txb::GemmX3Params g;
+        g.N = g.K = (int)E; g.status = status; g.out_f16 = f16 ? 1 : 0; g.n_probs = 3;
+        const __half *xh[3], *xl[3];
+        for (int i = 0; i < 3; ++i) {
+            xh[i] = half_at(o_xh[i]); xl[i] = half_at(o_xl[i]);
+            g.prob[i] = {float_at(o_xi[i]), float_at(o_wi) + i * E, bias[i], ws + o_p[i], (int)M[i], (int)seq[i], (int)d->heads, (int)(i * E), 0, 0};
+        }
+        if (int rc = launch_gemm_x3(g, xh, xl, half_at(o_wh), half_at(o_wl), 3 * E, st)) return rc;
+
+        tx_sdpa_desc a;
+        std::memset(&a, 0, sizeof a);
+        a.q = ws + o_p[0]; a.k = ws + o_p[1]; a.v = ws + o_p[2];
+        a.mask = d->mask; a.kv_lens = d->kv_lens; a.out = ws + o_a;
+        a.batch = d->batch; a.q_heads = a.kv_heads = d->heads;
+        a.seq_q = d->seq_q; a.seq_k = d->seq_k; a.d_k = a.d_v = E / d->heads;
+        a.dtype = f16 ? TX_DTYPE_F16 : TX_DTYPE_F32;
+        a.causal = d->causal; a.flags = d->flags & TX_SDPA_KV_LENS_HOST; a.stream = d->stream;
+        if (int rc = forward(&a)) return rc;
+
+        sp.n_segs = 0; sp.rows = 0;
+        add(float_at(o_a), o_ah, o_al, o_ai, Mq, 0, (int)d->heads, d->seq_q);
+        if (int rc = split()) return rc;
+        g.n_probs = 1; g.out_f16 = 0;
+        g.prob[0] = {float_at(o_ai), float_at(o_wi) + 3 * E, d->bo, d->out, (int)Mq, (int)d->seq_q, 0, 0, 0, 0};
+        xh[0] = half_at(o_ah); xl[0] = half_at(o_al);
+        return launch_gemm_x3(g, xh, xl, half_at(o_wh) + 3 * E * E, half_at(o_wl) + 3 * E * E, E, st);
+    };
+    const int rc = body();
+    pool_free(ws, st);
+    return rc;
+}
+
 int sync_f32(const float *Q, const float *K, const float *V, const float *mask, float *out,
              int64_t B, int64_t H, int64_t Sq, int64_t Sk, int64_t dk, int64_t dv)
 {
@@ -1385,6 +1518,23 @@ int tx_linear_f32_cuda(const float *x, const float *w, const float *bias, float 
     g_launches++;
     TX_CUDA(cudaGetLastError());
     return TX_OK;
+}
+
+int tx_mha_forward_f32(const tx_mha_desc *d)
+{
+    TX_NVTX_RANGE("mha.forward");
+    if (!d || !d->xq || !d->xk || !d->xv || !d->wq || !d->wk || !d->wv || !d->wo || !d->out)
+        return fail(TX_ERR_INVALID, "MHA: inputs, weights and output must not be null");
+    if (d->batch <= 0 || d->seq_q <= 0 || d->seq_k <= 0 || d->embed <= 0 || d->heads <= 0 || d->embed % d->heads)
+        return fail(TX_ERR_INVALID, "MHA: every dimension must be positive and embed a multiple of heads");
+    const void *ptrs[] = {d->xq, d->xk, d->xv, d->wq, d->wk, d->wv, d->wo, d->bq, d->bk, d->bv, d->bo, d->out};
+    bool aligned = true;
+    for (const void *q : ptrs) aligned = aligned && (reinterpret_cast<uintptr_t>(q) & 15u) == 0;
+    const int64_t M = d->batch * std::max(d->seq_q, d->seq_k);
+    if (!aligned || d->embed % 8 || d->embed / d->heads % 4 || 4 * d->embed > 0x7fffffff || 3 * M > 0x7fffffff - 4 * d->embed)
+        return fail(TX_ERR_UNSUPPORTED, "MHA: built for 16-byte aligned tensors, embed a multiple of 8 and head dims of 4");
+    if (int rc = ensure_device()) return rc;
+    return mha_launch(d);
 }
 
 int tx_sdpa_forward(const tx_sdpa_desc *desc)

@@ -1,0 +1,72 @@
+"""tx_mha_forward_f32 -- the layer as one call, projections on fp16 pairs (csrc/gemm_x3.cuh) -- at the edges of its tiles:
+partial k-stages, partial row and column tiles, rows longer than the split pass keeps in registers, more than one
+accumulator chunk, separate and shared inputs."""
+import numpy as np
+import pytest
+
+import oracle
+import tensorax_b200 as ts
+from conftest import assert_close_fp16, assert_close_fp32, seeded
+from tensorax_b200 import _C
+from tensorax_b200.nn.attention import MultiHeadAttention
+
+pytestmark = pytest.mark.gpu
+
+NAMES = ("q", "k", "v", "out")
+
+
+def layer(E, H, bias, **kw):
+    mha = MultiHeadAttention(E, H, bias=bias, **kw).cuda()
+    for i, n in enumerate(NAMES):
+        mha._parameters[n + "_weight"] = ts.Tensor(seeded(50 + i, E, E) / np.sqrt(E), device="cuda")
+        if bias:
+            mha._parameters[n + "_bias"] = ts.Tensor(0.1 * seeded(60 + i, E), device="cuda")
+    return mha, {n: p.numpy() for n, p in mha._parameters.items() if p is not None}
+
+
+@pytest.mark.parametrize("B,Sq,Sk,E,H,bias", [
+    (1, 1, 1, 8, 1, True), (2, 5, 7, 40, 2, True), (1, 129, 129, 72, 3, False), (3, 43, 43, 200, 5, True),
+    (2, 130, 65, 256, 4, True), (1, 260, 260, 320, 5, False), (1, 70, 70, 1088, 17, True), (2, 64, 300, 512, 8, True),
+])
+def test_layer_against_the_composition_of_cpu_ops(B, Sq, Sk, E, H, bias):
+    mha, params = layer(E, H, bias)
+    x, y = seeded(1, B, Sq, E), seeded(2, B, Sk, E)
+    xt, yt = ts.Tensor(x, device="cuda"), ts.Tensor(y, device="cuda")
+    names = [mha._parameters[n + "_weight"]._c_tensor for n in NAMES]
+    biases = [mha._parameters[n + "_bias"]._c_tensor if bias else None for n in NAMES]
+    assert _C.multi_head_attention(xt._c_tensor, yt._c_tensor, yt._c_tensor, names, biases, H) is not None
+    got = mha(xt, yt, yt).numpy()
+    assert_close_fp32(got, oracle.mha_forward_f32(x, y, y, params, H, None), atol=2e-5)   # four chained fp32 stages
+    assert np.array_equal(got, mha(xt, yt, yt).numpy())
+    if Sq == Sk:
+        same = mha(xt, xt, xt, causal=True, kv_lens=[max(1, Sk - 3)] * B).numpy()
+        i, j = np.arange(Sq)[:, None], np.arange(Sk)[None, :]
+        m = np.where((j <= i) & (j < max(1, Sk - 3)), 0.0, -np.inf).astype(np.float32)
+        m = np.ascontiguousarray(np.broadcast_to(m, (B, H, Sq, Sk)))
+        ref = oracle.mha_forward_f32(x, x, x, params, H, m)
+        assert_close_fp32(same, ref, atol=2e-5)
+        assert_close_fp32(mha(xt, xt, xt, ts.Tensor(m, device="cuda")).numpy(), ref, atol=2e-5)
+
+
+@pytest.mark.parametrize("E,H", [(128, 2), (256, 2)])
+def test_fp16_attention_step(E, H):
+    mha, params = layer(E, H, True, attention_dtype="float16")
+    x = seeded(3, 2, 150, E)
+    got = mha(ts.Tensor(x, device="cuda"), ts.Tensor(x, device="cuda"), ts.Tensor(x, device="cuda")).numpy()
+    assert_close_fp16(got, oracle.mha_forward_f32(x, x, x, params, H, None))
+
+
+def test_rows_of_any_magnitude_keep_their_relative_precision():
+    """Row scaling by powers of two: rows of 1e-20, 1 and 1e20 side by side, each as exact as the others.  (Without biases and
+    with one key, the layer is (x Wv^T) Wo^T; float64 reference; bound: 22-bit operands and fp32 sums over E = 256,
+    twice: 2 * 256 * 2^-23 worst, 1e-6 in norm.)"""
+    E, H = 256, 4
+    mha, params = layer(E, H, False)
+    x = seeded(4, 3, 1, E) * np.array([1e-20, 1.0, 1e20]).reshape(3, 1, 1)
+    x = x.astype(np.float32)
+    q = ts.Tensor(seeded(5, 3, 1, E), device="cuda")
+    xt = ts.Tensor(x, device="cuda")
+    got = mha(q, q, xt).numpy()
+    ref = x.astype(np.float64) @ params["v_weight"].astype(np.float64).T @ params["out_weight"].astype(np.float64).T
+    for b in range(3):
+        assert np.linalg.norm(got[b] - ref[b]) <= 1e-6 * np.linalg.norm(ref[b])
