@@ -11,12 +11,15 @@
 //                       to [2^13, 2^14), then hi = rn16(x), lo = rn16(x - hi).  With the scale a pair is exact to 2^-39
 //                       of the row's maximum and to 22 bits down to 2^-17 of it, whatever the row's magnitude.
 //   gemm_x3_kernel      persistent, one CTA per SM, 128 x BN tiles.  The tensor core's fp32 accumulation truncates, so a
-//                       tensor-memory accumulator takes one stage (K = 64) only, the small products first, so that
-//                       four of its twelve MMAs add at full magnitude; two accumulators ping-pong and two warpgroups
-//                       fold them into fp32 register sums, rounded to nearest (an eighth of a stage's MMA time at BN = 256).
+//                       tensor-memory accumulator takes two stages (K = 128) only, a stage's small products first, so
+//                       that few of its 24 MMAs add at full magnitude; two accumulators ping-pong and two warpgroups
+//                       fold them into fp32 register sums, rounded to nearest.
 //                       warp 0 TMA producer, warp 1 MMA issuer, warps 4-7 / 8-11 sums and results of the left / right
 //                       half of a tile's columns (thread = row); results are turned through shared memory so that a
 //                       warp stores whole 128-byte pieces of rows, head-split, fp32 or fp16.
+// Bound: L2 -> SM traffic (a 128 x 256 tile brings 96 KB per 64 k, 128 FLOP per byte) next to the tensor pipe.  Measured, B4
+// S1024 E1024 (three projections, then the output's): 94 us together = 1.1 PFLOP/s of fp16 MMAs; folding after every stage
+// 103 us, after four 93; CTA pairs on 256 x 256 tiles (cta_group::2, 64 KB per 64 k and SM) 95 us, 128 x 128 tiles 99 us.
 // Every mbarrier wait is bounded.
 #pragma once
 #include "ptx.cuh"
@@ -113,7 +116,7 @@ struct GemmX3Maps {
 
 template <int BN_>
 struct GemmX3Cfg {
-    static constexpr int BM = 128, BN = BN_, BK = 64, CHUNK = 1;          // CHUNK: stages per accumulator
+    static constexpr int BM = 128, BN = BN_, BK = 64, CHUNK = 2;          // CHUNK: stages per accumulator
     static constexpr int THREADS = 384, REGS_LIGHT = 56, REGS_SUMS = 224; // 128 * 56 + 256 * 224 = 64512 = 384 * 168
     static constexpr uint32_t X_BYTES = BM * BK * 2, W_BYTES = BN * BK * 2;
     static constexpr uint32_t STAGE = 2 * X_BYTES + 2 * W_BYTES;          // x hi | x lo | W hi | W lo

@@ -877,8 +877,8 @@ int launch_gemm_x3_t(const txb::GemmX3Params &p0, const __half *const *xh, const
     return TX_OK;
 }
 
-// Tile width by the number of rounds the persistent CTAs need: a 128 x 128 tile takes about 0.6 of a 128 x 256 one and
-// 128 x 64 about 0.4 (the narrower the tile, the more of its time goes to bringing x).
+// Tile width by the number of rounds the persistent CTAs need: a 128 x 128 tile takes about 0.53 of a 128 x 256 one and
+// 128 x 64 about 0.37 (the narrower the tile, the more of its time goes to bringing x).
 int launch_gemm_x3(const txb::GemmX3Params &p, const __half *const *xh, const __half *const *xl, const __half *wh, const __half *wl,
                    int64_t w_rows, cudaStream_t st)
 {
@@ -889,7 +889,7 @@ int launch_gemm_x3(const txb::GemmX3Params &p, const __half *const *xh, const __
         for (int i = 0; i < p.n_probs; ++i) tiles += (int64_t)((p.prob[i].M + 127) / 128) * ((p.N + bn - 1) / bn);
         return (double)((tiles + sms - 1) / sms) * tile;
     };
-    const double t256 = time(256, 1.0), t128 = time(128, 0.6), t64 = time(64, 0.4);
+    const double t256 = time(256, 1.0), t128 = time(128, 0.53), t64 = time(64, 0.37);
     if (t256 <= t128 && t256 <= t64) return launch_gemm_x3_t<txb::GemmX3Cfg<256>>(p, xh, xl, wh, wl, w_rows, st);
     if (t128 <= t64) return launch_gemm_x3_t<txb::GemmX3Cfg<128>>(p, xh, xl, wh, wl, w_rows, st);
     return launch_gemm_x3_t<txb::GemmX3Cfg<64>>(p, xh, xl, wh, wl, w_rows, st);
