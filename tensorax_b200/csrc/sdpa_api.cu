@@ -528,8 +528,11 @@ int launch_tc(const tx_sdpa_desc *d, cudaStream_t st, int *status, long long *pr
 
 // Few query rows per K/V head (a decoding step): the kernel that reads the cache once and cuts the keys over a cluster.
 // fp16 up to 16 rows a head (CTAs of four rows each, side by side, read the same keys through L2; beyond that the
-// tensor-core kernel's 128-row tile is the better use of a CTA) and from one whole tile of keys on; fp32 up to 32 rows, because the
-// tensor-core form first writes and reads back hi / lo copies of the whole cache.
+// tensor-core kernel's 128-row tile is the better use of a CTA) and from one whole tile of keys on; fp32 up to 32 rows,
+// because the tensor-core form first writes and reads back hi / lo copies of the whole cache.
+// Small fp32 calls go there too: one launch without a workspace against three and a memset.  Up to 2^23 products (B1 H2
+// S128 d64 44 -> 31 us a call, B1 H8 S128 d64 38 -> 28, B4 H8 S64 d64 37 -> 33; at 2^24 products and 1024 row groups it
+// was 37 against 43) or up to two query rows per SM in all (B1 H4 Sq64 Sk2048 d128 84 -> 42: four CTAs' work otherwise).
 bool decode_eligible(const tx_sdpa_desc *d)
 {
     if (d->flags & (TX_SDPA_FORCE_SIMT | TX_SDPA_P_IN_SMEM)) return false;
@@ -537,7 +540,9 @@ bool decode_eligible(const tx_sdpa_desc *d)
     auto al = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     if (!al(d->q) || !al(d->k) || !al(d->v)) return false;
     const int64_t rows = d->q_heads / d->kv_heads * d->seq_q;
-    return d->dtype == TX_DTYPE_F16 ? (rows <= 16 && d->seq_k >= 128) : rows <= 32;
+    if (d->dtype == TX_DTYPE_F16) return rows <= 16 && d->seq_k >= 128;
+    const double all_rows = (double)(d->batch * d->kv_heads * rows);
+    return rows <= 32 || all_rows <= 296 || all_rows * (double)d->seq_k * (double)d->d_k <= 8388608.0;
 }
 
 template <class Cfg>
@@ -1652,7 +1657,7 @@ int tx_sdpa_finish(void *stream) { return finish(static_cast<cudaStream_t>(strea
 
 int tx_sdpa_uses_tensor_cores(const tx_sdpa_desc *desc)
 {
-    if (validate(desc) != TX_OK || decode_eligible(desc)) return 0;
+    if (validate(desc) != TX_OK) return 0;
     if (desc->dtype == TX_DTYPE_F32 && (desc->flags & TX_SDPA_F32_VIA_F16)) {
         tx_sdpa_desc probe = *desc;
         probe.dtype = TX_DTYPE_F16;
