@@ -606,6 +606,43 @@ int launch_f16(const tx_sdpa_desc *d, cudaStream_t st, int *status)
     return decode_eligible(d) ? launch_decode<__half>(d, st, status) : launch_tc(d, st, status);
 }
 
+// CTAs per work item of a backward kernel: `items` items, the longest of `longest` tiles and `mean` on average, on
+// `slots` CTA places.  Time in tiles, a CTA's start and end counting as three: the longest CTA, or all of them spread
+// over the places, in whole waves where the items are equal.  An item is cut (in two, four or eight, a cluster) where that
+// shortens the launch by a tenth or more; a CTA keeps two tiles at least.
+int bwd_split(double items, double longest, double mean, double slots)
+{
+    auto cost = [&](int z) {
+        const double fixed = z > 1 ? 4.0 : 3.0, one = std::ceil(longest / z) + fixed, waves = items * z / slots;
+        return std::max(one, mean < longest ? waves * (mean / z + fixed) : std::ceil(waves) * one);
+    };
+    int best = 1;
+    for (int z = 2; z <= 8 && longest >= 2.0 * z; z *= 2)
+        if (cost(z) < 0.9 * cost(best)) best = z;
+    return best;
+}
+
+// One of the backward kernels on `ctas` CTAs, in clusters of `split`
+template <class K>
+int launch_bwd_kernel(K kernel, int64_t ctas, int split, int threads, size_t smem, cudaStream_t st, const CUtensorMap &tq,
+                      const CUtensorMap &tdo, const CUtensorMap &tk, const CUtensorMap &tv, const txb::BwdParams &p)
+{
+    if (ctas > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA backward: more than 2^31 work items");
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)split; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = split > 1 ? 1 : 0;
+    TX_CUDA(cudaLaunchKernelEx(&cfg, kernel, tq, tdo, tk, tv, p));
+    g_launches++;
+    return TX_OK;
+}
+
 template <int D, class DqCfg, class DkvCfg>
 int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __half *dout_h, const float *delta)
 {
@@ -619,6 +656,9 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
     p.scale_log2 = p.scale * 1.4426950408889634f;
     p.group_q = p.group_k = 1;
     p.items_q = p.items_k = p.slabs_q = p.slabs_k = 1;
+    p.split_q = p.split_k = 1;
+    int sms = 0;
+    if (int rc = sm_count(&sms)) return rc;
     {
         CUtensorMap tq, tdo, tk, tv;
         if (int rc = make_map(&tq, d->q, d->batch * d->q_heads, d->seq_q, D, DqCfg::BM)) return rc;
@@ -634,11 +674,11 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
         if (int rc = launch_group(d->causal != 0, slabs, items, 4.0 * (double)d->seq_k * (double)D / (double)ratio, ratio, &group, 32))
             return rc;
         p.group_q = (int)group; p.items_q = (int)items; p.slabs_q = (int)slabs;
-        if (items * slabs > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA backward: more than 2^31 work items");
-        dim3 grid((unsigned)(items * slabs));
-        txb::sdpa_bwd_dq_kernel<DqCfg><<<grid, DqCfg::THREADS, DqCfg::SMEM_BYTES, st>>>(tq, tdo, tk, tv, p);
-        g_launches++;
-        TX_CUDA(cudaGetLastError());
+        const double tiles = (double)((d->seq_k + DqCfg::BN - 1) / DqCfg::BN);
+        p.split_q = bwd_split((double)(items * slabs), tiles, d->causal ? 0.5 * (tiles + 1) : tiles, (double)DqCfg::CTAS_PER_SM * sms);
+        if (int rc = launch_bwd_kernel(txb::sdpa_bwd_dq_kernel<DqCfg>, items * slabs * p.split_q, p.split_q, DqCfg::THREADS,
+                                       DqCfg::SMEM_BYTES, st, tq, tdo, tk, tv, p))
+            return rc;
     }
     {
         CUtensorMap tq, tdo, tk, tv;
@@ -655,11 +695,12 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
         if (int rc = launch_group(d->causal != 0, slabs, items * DkvCfg::ZS, 4.0 * (double)ratio * (double)d->seq_q * (double)D, 1, &group, 32))
             return rc;
         p.group_k = (int)group; p.items_k = (int)items; p.slabs_k = (int)slabs;
-        if (items * slabs * DkvCfg::ZS > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA backward: more than 2^31 work items");
-        dim3 grid((unsigned)(items * slabs * DkvCfg::ZS));
-        txb::sdpa_bwd_dkv_kernel<DkvCfg><<<grid, DkvCfg::THREADS, DkvCfg::SMEM_BYTES, st>>>(tq, tdo, tk, tv, p);
-        g_launches++;
-        TX_CUDA(cudaGetLastError());
+        const double tiles = (double)((d->seq_q + DkvCfg::BQ - 1) / DkvCfg::BQ * ratio);
+        p.split_k = bwd_split((double)(items * slabs * DkvCfg::ZS), tiles, d->causal ? 0.5 * (tiles + ratio) : tiles,
+                              (double)DkvCfg::CTAS_PER_SM * sms);
+        if (int rc = launch_bwd_kernel(txb::sdpa_bwd_dkv_kernel<DkvCfg>, items * slabs * DkvCfg::ZS * p.split_k, p.split_k,
+                                       DkvCfg::THREADS, DkvCfg::SMEM_BYTES, st, tq, tdo, tk, tv, p))
+            return rc;
     }
     return TX_OK;
 }

@@ -23,6 +23,8 @@
 // sets the CTA's abort flag and a code in the device status word.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "ptx.cuh"
 #include "sdpa_tc.cuh"
 
@@ -45,7 +47,68 @@ struct BwdParams {
     // *_k: the dK/dV kernel (slab = (batch, K/V head), item = key tile; its ZS column parts stay side by side).
     int group_q, items_q, slabs_q;
     int group_k, items_k, slabs_k;
+    // CTAs (a thread-block cluster, neighbours in the 1-D grid) that share one work item: CTA z of `split_*` takes the
+    // item's tiles z, z + split, z + 2 split ... and the cluster adds the partial gradients in rank order.
+    int split_q, split_k;
 };
+
+// ------------------------------------------------------------------ result
+// Gradient tiles leave tensor memory through shared memory, so that global memory is written in whole lines (one row a
+// thread straight from tensor memory, 32 rows an instruction, cost 5 900 cycles a CTA in the dQ kernel and 9 800 in the
+// dK/dV kernel at d = 128, of 31 000 and 58 000 in all), and so that the CTAs of a cluster can add theirs up.
+// A staged tile is [128 rows][W floats]; 16-byte chunk c of row r sits at chunk c ^ (r % 8) (both sides conflict-free).
+template <int W>
+__device__ __forceinline__ uint32_t grad_chunk(int r, int c) { return (uint32_t)(r * (W / 4) + (c ^ (r & 7))) * 16u; }
+
+// 32 accumulator columns of the thread's row (TMEM lane) to the staged tile; zeros where the CTA had no tile to walk
+template <int W>
+__device__ __forceinline__ void stage_grad32(uint32_t tile, uint32_t taddr, int r, int col, bool any)
+{
+    uint32_t o[32];
+    if (any) {
+        ptx::tmem_ld32(taddr, o);
+        ptx::tmem_wait_ld();
+        ptx::reg_fence32(o);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < 32; i += 4)
+        ptx::st_shared_v4(tile + grad_chunk<W>(r, (col + i) / 4), o[i], o[i + 1], o[i + 2], o[i + 3]);
+}
+
+// This CTA's share of the tile's rows: summed over the cluster's CTAs in rank order, written to dst[row * ld + column].
+// `fill` stands in for the sum where no CTA of the item had anything to walk.
+template <int W, int THREADS>
+__device__ __forceinline__ void store_grad(const uint8_t *tile, float *dst, int64_t ld, int rows_ok, int rank, int split,
+                                           bool filled, float fill, int tid)
+{
+    namespace cg = cooperative_groups;
+    constexpr int C = W / 4;
+    const int rows = 128 / split, r0 = rank * rows;
+    for (int i = tid; i < rows * C; i += THREADS) {
+        const int r = r0 + i / C, c = i % C;
+        if (r >= rows_ok) break;
+        float4 v = make_float4(fill, fill, fill, fill);
+        if (!filled) {
+            const uint32_t off = grad_chunk<W>(r, c);
+            if (split == 1) {
+                v = *reinterpret_cast<const float4 *>(tile + off);
+            } else {
+                v = make_float4(0.f, 0.f, 0.f, 0.f);
+                cg::cluster_group cluster = cg::this_cluster();
+                for (int z = 0; z < split; z += 2) {               // two remote loads under way at a time
+                    const float4 a = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(tile, z) + off);
+                    const float4 b = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(tile, z + 1) + off);
+                    v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+                    v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+                }
+            }
+        }
+        *reinterpret_cast<float4 *>(dst + (int64_t)r * ld + c * 4) = v;
+    }
+}
 
 // ------------------------------------------------------------------ preprocess
 // dO fp32 -> fp16 (MMA operand) and delta = rowsum(dO o O); one warp per row.
@@ -106,6 +169,7 @@ struct BwdDqCfg {
     static constexpr int CTAS_PER_SM = (SMEM_BYTES <= 115712 && TMEM_COLS <= 256) ? 2 : 1;
     static_assert(D % 64 == 0 && CW % 32 == 0 && (D / 32) % WGS == 0 && COLS_USED <= 512 && SMEM_BYTES <= 232448,
                   "tile shape");
+    static_assert(BM * D * 4 <= OFF_BAR, "the staged dQ tile lies over the operand tiles");
 };
 
 template <class Cfg>
@@ -129,8 +193,10 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // work item: group-major, then longest first over all slabs of the group (late causal query tiles walk most keys)
+    const int split = p.split_q, rank = (int)blockIdx.x % split;
+    const int item = (int)blockIdx.x / split;
     const int span = p.group_q * p.items_q;
-    const int grp = (int)blockIdx.x / span, rem = (int)blockIdx.x % span;
+    const int grp = item / span, rem = item % span;
     const int in_grp = min(p.group_q, p.slabs_q - grp * p.group_q);
     const int q_tile = p.items_q - 1 - rem / in_grp;
     const int q0 = q_tile * BM;
@@ -141,8 +207,25 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     kv_limit = p.kv_lens.limit(b, kv_limit);
     int kv_end = kv_limit;
     if (p.causal) kv_end = min(kv_end, q0 + BM);
-    const int n_tiles = (kv_end + BN - 1) / BN;
+    const int n_all = (kv_end + BN - 1) / BN;
+    const int n_tiles = n_all > rank ? (n_all - rank + split - 1) / split : 0;      // tiles rank, rank + split, ...
 
+    auto load_k = [&](int j) {
+        const int s = j % NS;
+        ptx::mbar_arrive_expect_tx(k_full + 8 * s, Cfg::KV_BYTES);
+#pragma unroll
+        for (int pn = 0; pn < Cfg::KP; ++pn)
+            ptx::tma_load_3d(k_s + s * Cfg::KV_BYTES + pn * Cfg::KV_PANEL, &tm_k, k_full + 8 * s, pn * 64,
+                             (rank + j * split) * BN, kvh);
+    };
+    auto load_v = [&](int j) {
+        const int s = j % NSV;
+        ptx::mbar_arrive_expect_tx(v_full + 8 * s, Cfg::KV_BYTES);
+#pragma unroll
+        for (int pn = 0; pn < Cfg::KP; ++pn)
+            ptx::tma_load_3d(v_s + s * Cfg::KV_BYTES + pn * Cfg::KV_PANEL, &tm_v, v_full + 8 * s, pn * 64,
+                             (rank + j * split) * BN, kvh);
+    };
     if (tid == 0) {
         *abort_flag = 0;
         ptx::mbar_init(qdo_full, 1);
@@ -160,7 +243,21 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             ptx::mbar_init(v_empty + 8 * s, 1);
         }
         ptx::fence_mbar_init();
-        if (sbase & 1023u) { *abort_flag = 1; ptx::report(p.status, TC_ERR_ALIGN); }
+        if (sbase & 1023u) {
+            *abort_flag = 1;
+            ptx::report(p.status, TC_ERR_ALIGN);
+        } else if (n_tiles > 0) {
+            // the first loads run under the tensor-memory allocation and the meeting
+            ptx::mbar_arrive_expect_tx(qdo_full, 2 * Cfg::Q_BYTES);
+#pragma unroll
+            for (int pn = 0; pn < Cfg::KP; ++pn)
+                ptx::tma_load_3d(q_s + pn * (BM * 128), &tm_q, qdo_full, pn * 64, q0, bh);
+            load_k(0);
+#pragma unroll
+            for (int pn = 0; pn < Cfg::KP; ++pn)
+                ptx::tma_load_3d(do_s + pn * (BM * 128), &tm_do, qdo_full, pn * 64, q0, bh);
+            load_v(0);
+        }
         if (*reinterpret_cast<volatile int *>(p.status) != 0) *abort_flag = 1;
     }
     if (warp == 1) {
@@ -176,44 +273,16 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (warp == 0) {
         if (run) {
             const bool leader = ptx::elect_one();
-            if (leader) {
-                ptx::prefetch_tmap(&tm_q);
-                ptx::prefetch_tmap(&tm_do);
-                ptx::prefetch_tmap(&tm_k);
-                ptx::prefetch_tmap(&tm_v);
-                ptx::mbar_arrive_expect_tx(qdo_full, 2 * Cfg::Q_BYTES);
-#pragma unroll
-                for (int pn = 0; pn < Cfg::KP; ++pn) {
-                    ptx::tma_load_3d(q_s + pn * (BM * 128), &tm_q, qdo_full, pn * 64, q0, bh);
-                    ptx::tma_load_3d(do_s + pn * (BM * 128), &tm_do, qdo_full, pn * 64, q0, bh);
-                }
-            }
-            __syncwarp();
             bool ok = true;
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                const int s = j % NS;
-                const uint32_t ph = (uint32_t)(j / NS) & 1u;
-                ok = ptx::mbar_wait(k_empty + 8 * s, ph ^ 1u, abort_flag);
+            // tile 0 went out before the meeting: no wait is taken on its behalf (its stages may be released already)
+            for (int j = 1; j < n_tiles && ok; ++j) {
+                ok = ptx::mbar_wait(k_empty + 8 * (j % NS), ((uint32_t)(j / NS) & 1u) ^ 1u, abort_flag);
                 if (!ok) break;
-                if (leader) {
-                    ptx::mbar_arrive_expect_tx(k_full + 8 * s, Cfg::KV_BYTES);
-#pragma unroll
-                    for (int pn = 0; pn < Cfg::KP; ++pn)
-                        ptx::tma_load_3d(k_s + s * Cfg::KV_BYTES + pn * Cfg::KV_PANEL, &tm_k, k_full + 8 * s,
-                                         pn * 64, j * BN, kvh);
-                }
+                if (leader) load_k(j);
                 __syncwarp();
-                const int sv_ = j % NSV;
-                const uint32_t phv = (uint32_t)(j / NSV) & 1u;
-                ok = ptx::mbar_wait(v_empty + 8 * sv_, phv ^ 1u, abort_flag);
+                ok = ptx::mbar_wait(v_empty + 8 * (j % NSV), ((uint32_t)(j / NSV) & 1u) ^ 1u, abort_flag);
                 if (!ok) break;
-                if (leader) {
-                    ptx::mbar_arrive_expect_tx(v_full + 8 * sv_, Cfg::KV_BYTES);
-#pragma unroll
-                    for (int pn = 0; pn < Cfg::KP; ++pn)
-                        ptx::tma_load_3d(v_s + sv_ * Cfg::KV_BYTES + pn * Cfg::KV_PANEL, &tm_v, v_full + 8 * sv_,
-                                         pn * 64, j * BN, kvh);
-                }
+                if (leader) load_v(j);
                 __syncwarp();
             }
             if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, BWD_ERR_PRODUCER); }
@@ -315,7 +384,7 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (lane == 0) ptx::mbar_arrive(bar);
         };
         for (int j = 0; j < n_tiles && ok; ++j) {
-            const int kv0 = j * BN + c0;
+            const int kv0 = (rank + j * split) * BN + c0;
             ok = ptx::mbar_wait(s_full, (uint32_t)j & 1u, abort_flag);
             if (!ok) break;
             ptx::tc_fence_after_sync();
@@ -358,44 +427,33 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
         if (run && ok) {
             ok = ptx::mbar_wait(dq_done, (uint32_t)(n_tiles - 1) & 1u, abort_flag);
-            if (ok) {
-                ptx::tc_fence_after_sync();
-                float *grow = p.dq + ((size_t)bh * p.Sq + row) * D;
-#pragma unroll
-                for (int cc = 0; cc < D / 32 / Cfg::WGS; ++cc) {
-                    const int c = cc * Cfg::WGS + wg;          // the warpgroups share the row's chunks
-                    uint32_t o[32];
-                    ptx::tmem_ld32(t_dq + c * 32, o);
-                    ptx::tmem_wait_ld();
-                    ptx::reg_fence32(o);
-                    if (row_ok) {
-#pragma unroll
-                        for (int i = 0; i < 32; i += 4)
-                            *reinterpret_cast<float4 *>(grow + c * 32 + i) =
-                                make_float4(__uint_as_float(o[i]), __uint_as_float(o[i + 1]), __uint_as_float(o[i + 2]),
-                                            __uint_as_float(o[i + 3]));
-                    }
-                }
-            }
+            ptx::tc_fence_after_sync();
         }
         if (run && !ok) { *abort_flag = 1; ptx::report(p.status, BWD_ERR_ROWS); }
-        if (!run && *abort_flag == 0 && row_ok) {
-            // no visible key: the forward row is 0/0, and so is its gradient
-            float *grow = p.dq + ((size_t)bh * p.Sq + row) * D;
-            for (int i = 0; i < D; ++i) grow[i] = __int_as_float(0x7fc00000);
+        // every load and MMA of this CTA is done: the operand tiles make room for the result
+        if (ok || (split > 1 && n_tiles == 0)) {
+#pragma unroll
+            for (int cc = 0; cc < D / 32 / Cfg::WGS; ++cc) {
+                const int c = (cc * Cfg::WGS + wg) * 32;       // the warpgroups share the row's chunks
+                stage_grad32<D>(sbase, t_dq + c, r, c, ok);
+            }
         }
     }
 
     ptx::tc_fence_before_sync();
-    __syncthreads();
-    if (*abort_flag) {
+    if (split > 1) cooperative_groups::this_cluster().sync();
+    else __syncthreads();
+    // a row without any visible key: the forward row is 0/0, and so is its gradient
+    if (*abort_flag == 0)
+        store_grad<D, Cfg::THREADS>(smem, p.dq + ((size_t)bh * p.Sq + q0) * D, D, p.Sq - q0, rank, split, n_all == 0,
+                                    __int_as_float(0x7fc00000), tid);
+    else
         for (int i = 0; i < 64; ++i) __nanosleep(2000);
-        __syncthreads();
-    }
     if (warp == 1) {
         ptx::tc_fence_after_sync();
         ptx::tmem_dealloc(tmem, Cfg::TMEM_COLS);
     }
+    if (split > 1) cooperative_groups::this_cluster().sync();       // nobody leaves while its shared memory is read
 }
 
 // ------------------------------------------------------------------ dK, dV
@@ -434,6 +492,7 @@ struct BwdDkvCfg {
     static constexpr int CTAS_PER_SM = (SMEM_BYTES <= 115712 && TMEM_COLS <= 256) ? 2 : 1;
     static_assert(D % 64 == 0 && DA % 64 == 0 && CW % 32 == 0 && (DA / 32) % WGS == 0 && 2 * BQ <= 128 * WGS &&
                       COLS_USED <= 512 && SMEM_BYTES <= 232448 && (!PS_SMEM || BQ == 64), "tile shape");
+    static_assert(2 * BMK * DA * 4 <= OFF_STAT, "the staged dK and dV tiles lie over the operand tiles");
     static_assert(NS >= 2 && NSD >= 2, "Q and dO stages are held from their first read to their second");
 };
 
@@ -460,12 +519,13 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // work item: column part fastest, then group-major and longest first over the group's slabs (with a causal
     // mask the FIRST key tiles are seen by most queries)
-    const int item = (int)blockIdx.x / Cfg::ZS;
+    const int split = p.split_k, rank = (int)blockIdx.x % split, part = (int)blockIdx.x / split;
+    const int item = part / Cfg::ZS;
     const int span = p.group_k * p.items_k;
     const int grp = item / span, rem = item % span;
     const int in_grp = min(p.group_k, p.slabs_k - grp * p.group_k);
     const int key0 = (rem / in_grp) * BMK;
-    const int col0 = ((int)blockIdx.x % Cfg::ZS) * DA;          // first dK / dV column of this CTA
+    const int col0 = (part % Cfg::ZS) * DA;          // first dK / dV column of this CTA
     const int kvh = grp * p.group_k + rem % in_grp;             // b * Hkv + kv head
     const int b = kvh / p.Hkv;
     const int group = p.Hq / p.Hkv;
@@ -476,7 +536,31 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     // causal: query rows below the tile's first key see none of its keys
     const int i_start = p.causal ? min(key0 / BQ, nq) : 0;
     const int per_head = (key0 < kv_limit) ? nq - i_start : 0;  // a tile beyond the valid keys gets zero gradients
-    const int n_it = per_head * group;
+    const int n_all = per_head * group;
+    const int n_it = n_all > rank ? (n_all - rank + split - 1) / split : 0;         // tiles rank, rank + split, ...
+    auto tile_of = [&](int t, int &head, int &row0) {           // query head and first query row of this CTA's tile t
+        const int g = rank + t * split, hd = g / per_head;
+        head = bh0 + hd;
+        row0 = (i_start + g - hd * per_head) * BQ;
+    };
+    auto load_q = [&](int t) {
+        const int s = t % NS;
+        int bhq, qr0;
+        tile_of(t, bhq, qr0);
+        ptx::mbar_arrive_expect_tx(q_full + 8 * s, Cfg::Q_BYTES);
+#pragma unroll
+        for (int pn = 0; pn < Cfg::KP; ++pn)
+            ptx::tma_load_3d(q_s + s * Cfg::Q_BYTES + pn * Cfg::Q_PANEL, &tm_q, q_full + 8 * s, pn * 64, qr0, bhq);
+    };
+    auto load_do = [&](int t) {
+        const int s = t % NSD;
+        int bhq, qr0;
+        tile_of(t, bhq, qr0);
+        ptx::mbar_arrive_expect_tx(do_full + 8 * s, Cfg::Q_BYTES);
+#pragma unroll
+        for (int pn = 0; pn < Cfg::KP; ++pn)
+            ptx::tma_load_3d(do_s + s * Cfg::Q_BYTES + pn * Cfg::Q_PANEL, &tm_do, do_full + 8 * s, pn * 64, qr0, bhq);
+    };
 
     if (tid == 0) {
         *abort_flag = 0;
@@ -495,7 +579,21 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             ptx::mbar_init(do_empty + 8 * s, 1);
         }
         ptx::fence_mbar_init();
-        if (sbase & 1023u) { *abort_flag = 1; ptx::report(p.status, TC_ERR_ALIGN); }
+        if (sbase & 1023u) {
+            *abort_flag = 1;
+            ptx::report(p.status, TC_ERR_ALIGN);
+        } else if (n_it > 0) {
+            // the first loads run under the tensor-memory allocation and the meeting
+            ptx::mbar_arrive_expect_tx(kv_full, 2 * Cfg::KV_BYTES);
+#pragma unroll
+            for (int pn = 0; pn < Cfg::KP; ++pn)
+                ptx::tma_load_3d(k_s + pn * (BMK * 128), &tm_k, kv_full, pn * 64, key0, kvh);
+            load_q(0);
+#pragma unroll
+            for (int pn = 0; pn < Cfg::KP; ++pn)
+                ptx::tma_load_3d(v_s + pn * (BMK * 128), &tm_v, kv_full, pn * 64, key0, kvh);
+            load_do(0);
+        }
         if (*reinterpret_cast<volatile int *>(p.status) != 0) *abort_flag = 1;
     }
     if (warp == 1) {
@@ -511,45 +609,16 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     if (warp == 0) {
         if (run) {
             const bool leader = ptx::elect_one();
-            if (leader) {
-                ptx::prefetch_tmap(&tm_q);
-                ptx::prefetch_tmap(&tm_do);
-                ptx::prefetch_tmap(&tm_k);
-                ptx::prefetch_tmap(&tm_v);
-                ptx::mbar_arrive_expect_tx(kv_full, 2 * Cfg::KV_BYTES);
-#pragma unroll
-                for (int pn = 0; pn < Cfg::KP; ++pn) {
-                    ptx::tma_load_3d(k_s + pn * (BMK * 128), &tm_k, kv_full, pn * 64, key0, kvh);
-                    ptx::tma_load_3d(v_s + pn * (BMK * 128), &tm_v, kv_full, pn * 64, key0, kvh);
-                }
-            }
-            __syncwarp();
             bool ok = true;
-            for (int t = 0; t < n_it && ok; ++t) {
-                const int bhq = bh0 + t / per_head;
-                const int qr0 = (i_start + t % per_head) * BQ;
-                const int s = t % NS;
-                const uint32_t ph = (uint32_t)(t / NS) & 1u;
-                ok = ptx::mbar_wait(q_empty + 8 * s, ph ^ 1u, abort_flag);
+            // tile 0 went out before the meeting: no wait is taken on its behalf (its stages may be released already)
+            for (int t = 1; t < n_it && ok; ++t) {
+                ok = ptx::mbar_wait(q_empty + 8 * (t % NS), ((uint32_t)(t / NS) & 1u) ^ 1u, abort_flag);
                 if (!ok) break;
-                if (leader) {
-                    ptx::mbar_arrive_expect_tx(q_full + 8 * s, Cfg::Q_BYTES);
-#pragma unroll
-                    for (int pn = 0; pn < Cfg::KP; ++pn)
-                        ptx::tma_load_3d(q_s + s * Cfg::Q_BYTES + pn * Cfg::Q_PANEL, &tm_q, q_full + 8 * s, pn * 64, qr0, bhq);
-                }
+                if (leader) load_q(t);
                 __syncwarp();
-                const int sd = t % NSD;
-                const uint32_t phd = (uint32_t)(t / NSD) & 1u;
-                ok = ptx::mbar_wait(do_empty + 8 * sd, phd ^ 1u, abort_flag);
+                ok = ptx::mbar_wait(do_empty + 8 * (t % NSD), ((uint32_t)(t / NSD) & 1u) ^ 1u, abort_flag);
                 if (!ok) break;
-                if (leader) {
-                    ptx::mbar_arrive_expect_tx(do_full + 8 * sd, Cfg::Q_BYTES);
-#pragma unroll
-                    for (int pn = 0; pn < Cfg::KP; ++pn)
-                        ptx::tma_load_3d(do_s + sd * Cfg::Q_BYTES + pn * Cfg::Q_PANEL, &tm_do, do_full + 8 * sd, pn * 64, qr0,
-                                         bhq);
-                }
+                if (leader) load_do(t);
                 __syncwarp();
             }
             if (!ok && leader) { *abort_flag = 1; ptx::report(p.status, BWD_ERR_PRODUCER); }
@@ -668,21 +737,28 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(bar);
         };
+        // The row statistics of a tile's queries: requested one tile ahead (a thread holds one of them; asking for them
+        // where they are needed cost 870 of 2 310 cycles a tile at d = 128), through shared memory to all row warps.
+        auto fetch_stat = [&](int t) -> float {
+            if (t >= n_it || st >= 2 * BQ) return 0.f;
+            int bhq, qr0;
+            tile_of(t, bhq, qr0);
+            const int qrow = qr0 + (st < BQ ? st : st - BQ);
+            const size_t at = (size_t)bhq * p.Sq + qrow;
+            if (st < BQ) return qrow < p.Sq ? -p.lse[at] : -INFINITY;            // -lse; -inf: P = 0
+            return qrow < p.Sq ? -p.scale * p.delta[at] : 0.f;                   // -D*scale
+        };
+        float next_stat = fetch_stat(0);
         for (int t = 0; t < n_it; ++t) {
             // All row warps take every iteration's named barrier, also after a failed wait, so
             // that none of them is left behind at it.
-            const int bhq = bh0 + t / per_head;
-            const int qr0 = (i_start + t % per_head) * BQ;
+            int bhq, qr0;
+            tile_of(t, bhq, qr0);
             float *st_lse = stat + (t & 1) * 2 * BQ, *st_delta = st_lse + BQ;
-            if (st < BQ) {
-                const int qrow = qr0 + st;
-                st_lse[st] = qrow < p.Sq ? -p.lse[(size_t)bhq * p.Sq + qrow] : -INFINITY;   // -lse; -inf: P = 0
-            } else if (st < 2 * BQ) {
-                const int qrow = qr0 + st - BQ;
-                st_delta[st - BQ] = qrow < p.Sq ? -p.scale * p.delta[(size_t)bhq * p.Sq + qrow] : 0.f;   // -D*scale
-            }
+            if (st < 2 * BQ) st_lse[st] = next_stat;
             if constexpr (Cfg::WGS == 1) asm volatile("bar.sync 1, 128;" ::: "memory");
             else asm volatile("bar.sync 1, 256;" ::: "memory");
+            next_stat = fetch_stat(t + 1);
             if (!ok) continue;
             ok = ptx::mbar_wait(s_full, (uint32_t)t & 1u, abort_flag);
             if (!ok) continue;
@@ -742,60 +818,40 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             }
             arrive_warp(pds_full);
         }
-        const size_t gbase = ((size_t)kvh * p.Sk + key) * D + col0;
         if (run && ok) {
             ok = ptx::mbar_wait(pds_done, (uint32_t)(n_it - 1) & 1u, abort_flag);
-            if (ok) {
-                ptx::tc_fence_after_sync();
-#pragma unroll
-                for (int cc = 0; cc < DA / 32 / Cfg::WGS; ++cc) {
-                    const int c = cc * Cfg::WGS + wg;          // the warpgroups share the row's chunks
-                    uint32_t o[32];
-                    ptx::tmem_ld32(t_dk + c * 32, o);
-                    ptx::tmem_wait_ld();
-                    ptx::reg_fence32(o);
-                    if (key < p.Sk) {
-#pragma unroll
-                        for (int i = 0; i < 32; i += 4)
-                            *reinterpret_cast<float4 *>(p.dk + gbase + c * 32 + i) =
-                                make_float4(__uint_as_float(o[i]), __uint_as_float(o[i + 1]), __uint_as_float(o[i + 2]),
-                                            __uint_as_float(o[i + 3]));
-                    }
-                    ptx::tmem_ld32(t_dv + c * 32, o);
-                    ptx::tmem_wait_ld();
-                    ptx::reg_fence32(o);
-                    if (key < p.Sk) {
-#pragma unroll
-                        for (int i = 0; i < 32; i += 4)
-                            *reinterpret_cast<float4 *>(p.dv + gbase + c * 32 + i) =
-                                make_float4(__uint_as_float(o[i]), __uint_as_float(o[i + 1]), __uint_as_float(o[i + 2]),
-                                            __uint_as_float(o[i + 3]));
-                    }
-                }
-            }
+            ptx::tc_fence_after_sync();
         }
         if (run && !ok) { *abort_flag = 1; ptx::report(p.status, BWD_ERR_ROWS); }
-        if (!run && *abort_flag == 0 && key < p.Sk) {
-            // no query sees these keys: zero gradients -- unless the batch element has no valid key at
-            // all, where the forward rows are 0/0 and the reference's rule propagates NaN to every gradient
-            const float fill = kv_limit == 0 ? __int_as_float(0x7fc00000) : 0.f;
-            for (int i = 0; i < DA; i += 4) {
-                *reinterpret_cast<float4 *>(p.dk + gbase + i) = make_float4(fill, fill, fill, fill);
-                *reinterpret_cast<float4 *>(p.dv + gbase + i) = make_float4(fill, fill, fill, fill);
+        // every load and MMA of this CTA is done: the operand tiles make room for the result
+        if (ok || (split > 1 && n_it == 0)) {
+#pragma unroll
+            for (int cc = 0; cc < DA / 32 / Cfg::WGS; ++cc) {
+                const int c = (cc * Cfg::WGS + wg) * 32;       // the warpgroups share the row's chunks
+                stage_grad32<DA>(sbase, t_dk + c, r, c, ok);
+                stage_grad32<DA>(sbase + BMK * DA * 4, t_dv + c, r, c, ok);
             }
         }
     }
 
     ptx::tc_fence_before_sync();
-    __syncthreads();
-    if (*abort_flag) {
+    if (split > 1) cooperative_groups::this_cluster().sync();
+    else __syncthreads();
+    if (*abort_flag == 0) {
+        // keys no query sees: zero gradients -- unless the batch element has no valid key at
+        // all, where the forward rows are 0/0 and the reference's rule propagates NaN to every gradient
+        const float fill = kv_limit == 0 ? __int_as_float(0x7fc00000) : 0.f;
+        const size_t gbase = ((size_t)kvh * p.Sk + key0) * D + col0;
+        store_grad<DA, Cfg::THREADS>(smem, p.dk + gbase, D, p.Sk - key0, rank, split, n_all == 0, fill, tid);
+        store_grad<DA, Cfg::THREADS>(smem + BMK * DA * 4, p.dv + gbase, D, p.Sk - key0, rank, split, n_all == 0, fill, tid);
+    } else {
         for (int i = 0; i < 64; ++i) __nanosleep(2000);
-        __syncthreads();
     }
     if (warp == 1) {
         ptx::tc_fence_after_sync();
         ptx::tmem_dealloc(tmem, Cfg::TMEM_COLS);
     }
+    if (split > 1) cooperative_groups::this_cluster().sync();       // nobody leaves while its shared memory is read
 }
 
 }  // namespace txb
