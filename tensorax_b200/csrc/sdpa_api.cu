@@ -606,19 +606,22 @@ int launch_f16(const tx_sdpa_desc *d, cudaStream_t st, int *status)
     return decode_eligible(d) ? launch_decode<__half>(d, st, status) : launch_tc(d, st, status);
 }
 
-// CTAs per work item of a backward kernel: `items` items, the longest of `longest` tiles and `mean` on average, on
-// `slots` CTA places.  Time in tiles, a CTA's start and end counting as three: the longest CTA, or all of them spread
-// over the places, in whole waves where the items are equal.  An item is cut (in two, four or eight, a cluster) where that
-// shortens the launch by a tenth or more; a CTA keeps two tiles at least.
-int bwd_split(double items, double longest, double mean, double slots)
+// CTAs per work item of a backward kernel: `items` items, the longest of `longest` tiles and `mean` on average, on `sms`
+// multiprocessors of `per_sm` CTAs (two on one get through half as much again as one does).  Time in tiles, a CTA's start
+// and end counting as three, five with the sum over the cluster: the longest CTA, or all of them spread over the places, in
+// whole waves where the items are equal.  An item is cut (in two, four or eight, a cluster) where that shortens the launch
+// by a fifth or more; a CTA keeps two tiles at least.  B2 Hq12 Hkv4 S921 d64 causal: the dK/dV kernel 79 us uncut, 28 us
+// in four, 36 us in eight; the dQ kernel 19 us uncut, 22 us in two.
+int bwd_split(double items, double longest, double mean, int sms, int per_sm)
 {
+    const double places = per_sm == 2 ? 1.5 * sms : (double)sms;
     auto cost = [&](int z) {
-        const double fixed = z > 1 ? 4.0 : 3.0, one = std::ceil(longest / z) + fixed, waves = items * z / slots;
+        const double fixed = z > 1 ? 5.0 : 3.0, one = std::ceil(longest / z) + fixed, waves = items * z / places;
         return std::max(one, mean < longest ? waves * (mean / z + fixed) : std::ceil(waves) * one);
     };
     int best = 1;
     for (int z = 2; z <= 8 && longest >= 2.0 * z; z *= 2)
-        if (cost(z) < 0.9 * cost(best)) best = z;
+        if (cost(z) < 0.8 * cost(best)) best = z;
     return best;
 }
 
@@ -675,7 +678,7 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
             return rc;
         p.group_q = (int)group; p.items_q = (int)items; p.slabs_q = (int)slabs;
         const double tiles = (double)((d->seq_k + DqCfg::BN - 1) / DqCfg::BN);
-        p.split_q = bwd_split((double)(items * slabs), tiles, d->causal ? 0.5 * (tiles + 1) : tiles, (double)DqCfg::CTAS_PER_SM * sms);
+        p.split_q = bwd_split((double)(items * slabs), tiles, d->causal ? 0.5 * (tiles + 1) : tiles, sms, DqCfg::CTAS_PER_SM);
         if (int rc = launch_bwd_kernel(txb::sdpa_bwd_dq_kernel<DqCfg>, items * slabs * p.split_q, p.split_q, DqCfg::THREADS,
                                        DqCfg::SMEM_BYTES, st, tq, tdo, tk, tv, p))
             return rc;
@@ -697,7 +700,7 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
         p.group_k = (int)group; p.items_k = (int)items; p.slabs_k = (int)slabs;
         const double tiles = (double)((d->seq_q + DkvCfg::BQ - 1) / DkvCfg::BQ * ratio);
         p.split_k = bwd_split((double)(items * slabs * DkvCfg::ZS), tiles, d->causal ? 0.5 * (tiles + ratio) : tiles,
-                              (double)DkvCfg::CTAS_PER_SM * sms);
+                              sms, DkvCfg::CTAS_PER_SM);
         if (int rc = launch_bwd_kernel(txb::sdpa_bwd_dkv_kernel<DkvCfg>, items * slabs * DkvCfg::ZS * p.split_k, p.split_k,
                                        DkvCfg::THREADS, DkvCfg::SMEM_BYTES, st, tq, tdo, tk, tv, p))
             return rc;

@@ -86,25 +86,34 @@ __device__ __forceinline__ void store_grad(const uint8_t *tile, float *dst, int6
 {
     namespace cg = cooperative_groups;
     constexpr int C = W / 4;
+    if (split == 1 && !filled) {
+        // unrolled: several rows under way at once
+        constexpr int N = 128 * C;
+#pragma unroll 8
+        for (int n = 0; n < (N + THREADS - 1) / THREADS; ++n) {
+            const int i = n * THREADS + tid, r = i / C, c = i % C;
+            if (i < N && r < rows_ok)
+                *reinterpret_cast<float4 *>(dst + (int64_t)r * ld + c * 4) =
+                    *reinterpret_cast<const float4 *>(tile + grad_chunk<W>(r, c));
+        }
+        return;
+    }
     const int rows = 128 / split, r0 = rank * rows;
     for (int i = tid; i < rows * C; i += THREADS) {
         const int r = r0 + i / C, c = i % C;
         if (r >= rows_ok) break;
         float4 v = make_float4(fill, fill, fill, fill);
         if (!filled) {
-            const uint32_t off = grad_chunk<W>(r, c);
-            if (split == 1) {
-                v = *reinterpret_cast<const float4 *>(tile + off);
-            } else {
-                v = make_float4(0.f, 0.f, 0.f, 0.f);
-                cg::cluster_group cluster = cg::this_cluster();
-                for (int z = 0; z < split; z += 2) {               // two remote loads under way at a time
-                    const float4 a = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(tile, z) + off);
-                    const float4 b = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(tile, z + 1) + off);
-                    v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
-                    v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
-                }
-            }
+            cg::cluster_group cluster = cg::this_cluster();
+            const uint8_t *at = tile + grad_chunk<W>(r, c);
+            float4 part[8];                                        // all remote loads first: they take as long as one
+#pragma unroll
+            for (int z = 0; z < 8; ++z)
+                if (z < split) part[z] = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(at, z));
+            v = part[0];
+#pragma unroll
+            for (int z = 1; z < 8; ++z)
+                if (z < split) { v.x += part[z].x; v.y += part[z].y; v.z += part[z].z; v.w += part[z].w; }
         }
         *reinterpret_cast<float4 *>(dst + (int64_t)r * ld + c * 4) = v;
     }
@@ -739,26 +748,30 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         };
         // The row statistics of a tile's queries: requested one tile ahead (a thread holds one of them; asking for them
         // where they are needed cost 870 of 2 310 cycles a tile at d = 128), through shared memory to all row warps.
-        auto fetch_stat = [&](int t) -> float {
-            if (t >= n_it || st >= 2 * BQ) return 0.f;
-            int bhq, qr0;
-            tile_of(t, bhq, qr0);
-            const int qrow = qr0 + (st < BQ ? st : st - BQ);
-            const size_t at = (size_t)bhq * p.Sq + qrow;
-            if (st < BQ) return qrow < p.Sq ? -p.lse[at] : -INFINITY;            // -lse; -inf: P = 0
-            return qrow < p.Sq ? -p.scale * p.delta[at] : 0.f;                   // -D*scale
+        // The value stays as it was loaded until it is stored: arithmetic on it here would wait for it here.
+        const float *stat_src = st < BQ ? p.lse : p.delta;
+        const float stat_mul = st < BQ ? -1.f : -p.scale;                        // -lse, -D*scale
+        int head_n = 0, i_n = rank;                                              // tile t + 1: head of the group, query tile
+        auto settle = [&]() { while (i_n >= per_head && per_head > 0) { i_n -= per_head; ++head_n; } };
+        auto fetch_stat = [&]() -> float {
+            float v = st < BQ ? INFINITY : 0.f;                                  // no such query: -lse = -inf, P = 0
+            const int qrow = (i_start + i_n) * BQ + (st < BQ ? st : st - BQ);
+            if (head_n < group && st < 2 * BQ && qrow < p.Sq) v = stat_src[(size_t)(bh0 + head_n) * p.Sq + qrow];
+            return v;
         };
-        float next_stat = fetch_stat(0);
+        settle();
+        float next_stat = fetch_stat();
         for (int t = 0; t < n_it; ++t) {
             // All row warps take every iteration's named barrier, also after a failed wait, so
             // that none of them is left behind at it.
-            int bhq, qr0;
-            tile_of(t, bhq, qr0);
+            const int qr0 = (i_start + i_n) * BQ;
             float *st_lse = stat + (t & 1) * 2 * BQ, *st_delta = st_lse + BQ;
-            if (st < 2 * BQ) st_lse[st] = next_stat;
+            if (st < 2 * BQ) st_lse[st] = stat_mul * next_stat;
             if constexpr (Cfg::WGS == 1) asm volatile("bar.sync 1, 128;" ::: "memory");
             else asm volatile("bar.sync 1, 256;" ::: "memory");
-            next_stat = fetch_stat(t + 1);
+            i_n += split;
+            settle();
+            next_stat = fetch_stat();
             if (!ok) continue;
             ok = ptx::mbar_wait(s_full, (uint32_t)t & 1u, abort_flag);
             if (!ok) continue;
