@@ -46,6 +46,8 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const SplitRowsParams p
 {
     const int lane = threadIdx.x & 31;
     const int g = (int)blockIdx.x * 8 + (threadIdx.x >> 5);
+    ptx::grid_trigger();
+    ptx::grid_wait();
     if (g >= p.rows) return;
     int t = 0;
 #pragma unroll
@@ -173,6 +175,8 @@ gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ 
     ptx::tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
     const bool run = *abort_flag == 0;
+    ptx::grid_trigger();
+    ptx::grid_wait();                                                     // the split pass; the start above ran under its end
 
     if (warp < 4) {
     ptx::setmaxnreg_dec<Cfg::REGS_LIGHT>();

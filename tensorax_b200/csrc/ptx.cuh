@@ -477,6 +477,15 @@ __device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.
 template <int N>
 __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
+// ---------------------------------------------------------------- launches that overlap the one before
+// A kernel launched with programmatic stream serialization starts while its predecessor's last CTAs still run.  Before it
+// touches anything an earlier launch of the stream writes or reads, it waits here for the predecessor's end; since every
+// kernel of such a chain does so before it ends, a launch that has ended has all earlier ones behind it.  Without the launch
+// attribute both are no-ops.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next launch may start once every CTA of this one has come by here (or has ended).
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- math
 __device__ __forceinline__ float ex2_approx(float x)
 {

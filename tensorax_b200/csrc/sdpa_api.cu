@@ -332,6 +332,28 @@ int with_device_lens(const Desc *d, Call call)
     return rc;
 }
 
+// A launch that may start under the end of the one before it in the stream (ptx::grid_wait inside the kernel orders what
+// has to be ordered), in clusters of `cluster` CTAs.  A plain launch starts 1 to 2 us after its predecessor has ended.
+template <class... Params, class... Args>
+int launch_behind(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, int cluster, const Args &...args)
+{
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    TX_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+    g_launches++;
+    return TX_OK;
+}
+
 template <typename T, int DVC, bool PROF>
 int launch_simt_t(const txb::SimtParams &p, cudaStream_t st)
 {
@@ -344,6 +366,7 @@ int launch_simt_t(const txb::SimtParams &p, cudaStream_t st)
         if (int rc = sm_count(&sms)) return rc;
         grid.y = std::min<unsigned>(grid.y, (unsigned)sms);
         grid.z = std::min<unsigned>(grid.z, std::max(1u, (unsigned)sms / grid.y));
+        return launch_behind(txb::sdpa_simt_kernel<T, DVC, PROF>, grid, txb::SIMT_THREADS, 0, st, 1, p);
     }
     txb::sdpa_simt_kernel<T, DVC, PROF><<<grid, txb::SIMT_THREADS, 0, st>>>(p);
     g_launches++;
@@ -625,27 +648,6 @@ int bwd_split(double items, double longest, double mean, int sms, int per_sm)
     return best;
 }
 
-// One of the backward kernels on `ctas` CTAs, in clusters of `split`
-template <class K>
-int launch_bwd_kernel(K kernel, int64_t ctas, int split, int threads, size_t smem, cudaStream_t st, const CUtensorMap &tq,
-                      const CUtensorMap &tdo, const CUtensorMap &tk, const CUtensorMap &tv, const txb::BwdParams &p)
-{
-    if (ctas > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA backward: more than 2^31 work items");
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)split; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = split > 1 ? 1 : 0;
-    TX_CUDA(cudaLaunchKernelEx(&cfg, kernel, tq, tdo, tk, tv, p));
-    g_launches++;
-    return TX_OK;
-}
-
 template <int D, class DqCfg, class DkvCfg>
 int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __half *dout_h, const float *delta)
 {
@@ -679,8 +681,9 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
         p.group_q = (int)group; p.items_q = (int)items; p.slabs_q = (int)slabs;
         const double tiles = (double)((d->seq_k + DqCfg::BN - 1) / DqCfg::BN);
         p.split_q = bwd_split((double)(items * slabs), tiles, d->causal ? 0.5 * (tiles + 1) : tiles, sms, DqCfg::CTAS_PER_SM);
-        if (int rc = launch_bwd_kernel(txb::sdpa_bwd_dq_kernel<DqCfg>, items * slabs * p.split_q, p.split_q, DqCfg::THREADS,
-                                       DqCfg::SMEM_BYTES, st, tq, tdo, tk, tv, p))
+        if (items * slabs * p.split_q > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA backward: more than 2^31 work items");
+        if (int rc = launch_behind(txb::sdpa_bwd_dq_kernel<DqCfg>, dim3((unsigned)(items * slabs * p.split_q)), DqCfg::THREADS,
+                                   DqCfg::SMEM_BYTES, st, p.split_q, tq, tdo, tk, tv, p))
             return rc;
     }
     {
@@ -701,8 +704,10 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
         const double tiles = (double)((d->seq_q + DkvCfg::BQ - 1) / DkvCfg::BQ * ratio);
         p.split_k = bwd_split((double)(items * slabs * DkvCfg::ZS), tiles, d->causal ? 0.5 * (tiles + ratio) : tiles,
                               sms, DkvCfg::CTAS_PER_SM);
-        if (int rc = launch_bwd_kernel(txb::sdpa_bwd_dkv_kernel<DkvCfg>, items * slabs * DkvCfg::ZS * p.split_k, p.split_k,
-                                       DkvCfg::THREADS, DkvCfg::SMEM_BYTES, st, tq, tdo, tk, tv, p))
+        const int64_t ctas = items * slabs * DkvCfg::ZS * p.split_k;
+        if (ctas > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA backward: more than 2^31 work items");
+        if (int rc = launch_behind(txb::sdpa_bwd_dkv_kernel<DkvCfg>, dim3((unsigned)ctas), DkvCfg::THREADS, DkvCfg::SMEM_BYTES, st,
+                                   p.split_k, tq, tdo, tk, tv, p))
             return rc;
     }
     return TX_OK;
@@ -829,9 +834,9 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
         p.group = (int)group; p.n_tiles_q = (int)n_tiles; p.BH = (int)sq;
         if (n_tiles * sq > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA: more than 2^31 work items");
         if (int r = allow_smem<txb::sdpa_tc_x3_kernel<Cfg>>((int)Cfg::SMEM_BYTES)) return r;
-        txb::sdpa_tc_x3_kernel<Cfg><<<(unsigned)(n_tiles * sq), Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(qh, ql, kh, kl, vh, vl, to, p);
-        g_launches++;
-        TX_CUDA(cudaGetLastError());
+        if (int r = launch_behind(txb::sdpa_tc_x3_kernel<Cfg>, dim3((unsigned)(n_tiles * sq)), Cfg::THREADS, Cfg::SMEM_BYTES, st, 1,
+                                  qh, ql, kh, kl, vh, vl, to, p))
+            return r;
         // the exact kernel behind it: works only when the split pass found a value the fp16 pairs cannot carry
         txb::SimtParams sp2;
         fill_simt_params(&sp2, d);
@@ -920,10 +925,7 @@ int launch_gemm_x3_t(const txb::GemmX3Params &p0, const __half *const *xh, const
     int sms = 0;
     if (int rc = sm_count(&sms)) return rc;
     if (int rc = allow_smem<txb::gemm_x3_kernel<Cfg>>((int)Cfg::SMEM_BYTES)) return rc;
-    txb::gemm_x3_kernel<Cfg><<<(unsigned)std::min(p.n_tiles, sms), Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(maps, p);
-    g_launches++;
-    TX_CUDA(cudaGetLastError());
-    return TX_OK;
+    return launch_behind(txb::gemm_x3_kernel<Cfg>, dim3((unsigned)std::min(p.n_tiles, sms)), Cfg::THREADS, Cfg::SMEM_BYTES, st, 1, maps, p);
 }
 
 // Tile width by the number of rounds the persistent CTAs need: a 128 x 128 tile takes about 0.53 of a 128 x 256 one and
@@ -988,16 +990,13 @@ int mha_launch(const tx_mha_desc *d)
             s.rows = (int)rows; s.heads = heads; s.S = (int)S; s.first = sp.rows;
             sp.rows += (int)rows;
         };
-        auto split = [&]() -> int {
-            txb::split_rows_kernel<<<(unsigned)((sp.rows + 7) / 8), 256, 0, st>>>(sp);
-            g_launches++;
-            TX_CUDA(cudaGetLastError());
-            return TX_OK;
-        };
+        auto split_grid = [&]() { return dim3((unsigned)((sp.rows + 7) / 8)); };
         for (int i = 0; i < 3; ++i)
             if (from[i] == i) add(x[i], o_xh[i], o_xl[i], o_xi[i], M[i], 0, 0, 1);
         for (int i = 0; i < 4; ++i) add(w[i], o_wh, o_wl, o_wi, E, i * E, 0, 1);
-        if (int rc = split()) return rc;
+        txb::split_rows_kernel<<<split_grid(), 256, 0, st>>>(sp);          // behind whatever the caller enqueued: a plain launch
+        g_launches++;
+        TX_CUDA(cudaGetLastError());
 
         txb::GemmX3Params g;
         g.N = g.K = (int)E; g.status = status; g.out_f16 = f16 ? 1 : 0; g.n_probs = 3;
@@ -1020,7 +1019,7 @@ int mha_launch(const tx_mha_desc *d)
 
         sp.n_segs = 0; sp.rows = 0;
         add(float_at(o_a), o_ah, o_al, o_ai, Mq, 0, (int)d->heads, d->seq_q);
-        if (int rc = split()) return rc;
+        if (int rc = launch_behind(txb::split_rows_kernel, split_grid(), 256, 0, st, 1, sp)) return rc;
         g.n_probs = 1; g.out_f16 = 0;
         g.prob[0] = {float_at(o_ai), float_at(o_wi) + 3 * E, d->bo, d->out, (int)Mq, (int)d->seq_q, 0, 0, 0, 0};
         xh[0] = half_at(o_ah); xl[0] = half_at(o_al);

@@ -125,6 +125,7 @@ template <typename OT>
 __global__ void sdpa_bwd_prep_kernel(const float *__restrict__ dout, const OT *__restrict__ out,
                                      __half *__restrict__ dout_h, float *__restrict__ delta, int64_t rows, int d)
 {
+    ptx::grid_trigger();
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
@@ -256,6 +257,7 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             *abort_flag = 1;
             ptx::report(p.status, TC_ERR_ALIGN);
         } else if (n_tiles > 0) {
+            ptx::grid_wait();                    // the preprocess: dO in fp16 and the row sums
             // the first loads run under the tensor-memory allocation and the meeting
             ptx::mbar_arrive_expect_tx(qdo_full, 2 * Cfg::Q_BYTES);
 #pragma unroll
@@ -278,6 +280,8 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     ptx::tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
     const bool run = (*abort_flag == 0) && n_tiles > 0;
+    ptx::grid_wait();
+    ptx::grid_trigger();                         // after the wait: the dK/dV kernel relies on the preprocess being done
 
     if (warp == 0) {
         if (run) {
@@ -860,6 +864,9 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     } else {
         for (int i = 0; i < 64; ++i) __nanosleep(2000);
     }
+    // This kernel reads nothing the dQ kernel writes and starts under its last CTAs; it must not end before it, though:
+    // what follows in the stream takes both for done.
+    if (tid == 0) ptx::grid_wait();
     if (warp == 1) {
         ptx::tc_fence_after_sync();
         ptx::tmem_dealloc(tmem, Cfg::TMEM_COLS);

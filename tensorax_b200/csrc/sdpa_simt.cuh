@@ -76,7 +76,11 @@ sdpa_simt_kernel(const SimtParams p)
                 p.prof[i] = clock64();
         }
     };
-    if (p.only_if && !x3_declines(p.only_if)) return;
+    if (p.only_if) {
+        ptx::grid_trigger();
+        ptx::grid_wait();
+        if (!x3_declines(p.only_if)) return;
+    }
     stamp(SIMT_T_START);
     __shared__ float q_s[SIMT_BR][SIMT_DKC + 1];
     __shared__ float k_s[SIMT_BC][SIMT_DKC + 1];

@@ -100,6 +100,8 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                   const __grid_constant__ CUtensorMap tm_o, const X3Params p)
 {
     constexpr int D = Cfg::D, BN = Cfg::BN, NS = Cfg::NS, BM = Cfg::BM;
+    ptx::grid_trigger();
+    ptx::grid_wait();                                            // the split pass
     if (x3_declines(p.range)) return;                            // the exact kernel takes this call
 
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -567,6 +569,7 @@ struct SplitParams {
 
 __global__ void __launch_bounds__(256) split_f32_hi_lo_kernel(const SplitParams sp)
 {
+    ptx::grid_trigger();
     bool bad = false;
     float vmax = 0.f;
     const long long stride = (long long)gridDim.x * blockDim.x;
