@@ -567,37 +567,58 @@ struct SplitParams {
     int *range;
 };
 
+// hi and lo halves of four values
+__device__ __forceinline__ void split_quad(float4 v, uint2 &hh, uint2 &ll)
+{
+    const __half2 h01 = __floats2half2_rn(v.x, v.y), h23 = __floats2half2_rn(v.z, v.w);
+    const float2 b01 = __half22float2(h01), b23 = __half22float2(h23);
+    const __half2 l01 = __floats2half2_rn(v.x - b01.x, v.y - b01.y), l23 = __floats2half2_rn(v.z - b23.x, v.w - b23.y);
+    hh.x = *reinterpret_cast<const uint32_t *>(&h01);
+    hh.y = *reinterpret_cast<const uint32_t *>(&h23);
+    ll.x = *reinterpret_cast<const uint32_t *>(&l01);
+    ll.y = *reinterpret_cast<const uint32_t *>(&l23);
+}
+// !(|x| < 2^15) is also true for NaN
+__device__ __forceinline__ bool quad_too_large(float4 v)
+{
+    return !(fabsf(v.x) < 32768.f) || !(fabsf(v.y) < 32768.f) || !(fabsf(v.z) < 32768.f) || !(fabsf(v.w) < 32768.f);
+}
+__device__ __forceinline__ float quad_max(float4 v) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))); }
+
 __global__ void __launch_bounds__(256) split_f32_hi_lo_kernel(const SplitParams sp)
 {
     ptx::grid_trigger();
     bool bad = false;
     float vmax = 0.f;
     const long long stride = (long long)gridDim.x * blockDim.x;
+    const long long n = max(sp.seg[0].n4, max(sp.seg[1].n4, sp.seg[2].n4));
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        // the three tensors' quads are requested together: a thread has one or two of each, and one tensor after the other
+        // waits for memory three times (B2 H8 S1000 d80: 8.6 -> 7.4 us)
+        float4 x[3];
 #pragma unroll
-    for (int t = 0; t < 3; ++t) {
-        const SplitSeg s = sp.seg[t];
-        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < s.n4; i += stride) {
-            float4 v;
+        for (int t = 0; t < 3; ++t) {
+            const SplitSeg &s = sp.seg[t];
+            x[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i >= s.n4) continue;
             if (s.q4 == s.p4) {
-                v = reinterpret_cast<const float4 *>(s.x)[i];
+                x[t] = reinterpret_cast<const float4 *>(s.x)[i];
             } else {
                 const long long row = i / s.p4;
                 const int c = (int)(i - row * s.p4);
-                v = c < s.q4 ? reinterpret_cast<const float4 *>(s.x)[row * s.q4 + c] : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (c < s.q4) x[t] = reinterpret_cast<const float4 *>(s.x)[row * s.q4 + c];
             }
-            const __half2 h01 = __floats2half2_rn(v.x, v.y), h23 = __floats2half2_rn(v.z, v.w);
-            const float2 b01 = __half22float2(h01), b23 = __half22float2(h23);
-            const __half2 l01 = __floats2half2_rn(v.x - b01.x, v.y - b01.y), l23 = __floats2half2_rn(v.z - b23.x, v.w - b23.y);
+        }
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            const SplitSeg &s = sp.seg[t];
+            if (i >= s.n4) continue;
             uint2 hh, ll;
-            hh.x = *reinterpret_cast<const uint32_t *>(&h01);
-            hh.y = *reinterpret_cast<const uint32_t *>(&h23);
-            ll.x = *reinterpret_cast<const uint32_t *>(&l01);
-            ll.y = *reinterpret_cast<const uint32_t *>(&l23);
+            split_quad(x[t], hh, ll);
             reinterpret_cast<uint2 *>(s.hi)[i] = hh;
             reinterpret_cast<uint2 *>(s.lo)[i] = ll;
-            // !(|x| < 2^15) is also true for NaN
-            bad |= !(fabsf(v.x) < 32768.f) || !(fabsf(v.y) < 32768.f) || !(fabsf(v.z) < 32768.f) || !(fabsf(v.w) < 32768.f);
-            if (t == 2) vmax = fmaxf(vmax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+            bad |= quad_too_large(x[t]);
+            if (t == 2) vmax = fmaxf(vmax, quad_max(x[t]));
         }
     }
     // one atomic per CTA and word; none for a maximum that is large enough already

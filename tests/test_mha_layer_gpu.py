@@ -70,3 +70,16 @@ def test_rows_of_any_magnitude_keep_their_relative_precision():
     ref = x.astype(np.float64) @ params["v_weight"].astype(np.float64).T @ params["out_weight"].astype(np.float64).T
     for b in range(3):
         assert np.linalg.norm(got[b] - ref[b]) <= 1e-6 * np.linalg.norm(ref[b])
+
+
+@pytest.mark.parametrize("E,H", [(512, 8), (384, 3), (240, 5)])
+@pytest.mark.parametrize("scale", [1.0, 1e-4, 1e6])
+def test_halves_written_by_the_projections(E, H, scale):
+    """Attention reads the fp16 halves that the projections write (head dims 64, 128, 48; partial row tiles); values too
+    small or too large for them go to the exact kernel.  Bound: four chained fp32 stages, 2e-5 of the result."""
+    mha, params = layer(E, H, False)
+    x, y = seeded(6, 2, 301, E), (scale * seeded(7, 2, 333, E)).astype(np.float32)
+    k = seeded(8, 2, 333, E)
+    got = mha(*(ts.Tensor(t, device="cuda") for t in (x, k, y))).numpy()
+    ref = oracle.mha_forward_f32(x, k, y, params, H, None)
+    assert np.linalg.norm(got - ref) <= 2e-5 * np.linalg.norm(ref)
