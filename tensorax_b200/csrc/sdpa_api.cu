@@ -15,6 +15,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -1711,14 +1712,18 @@ static int backward_launch(const tx_sdpa_bwd_desc *d)
     if (int rc = pool_alloc(&ws, h_bytes + (size_t)rows * 4, st)) return rc;
     __half *dout_h = reinterpret_cast<__half *>(ws);
     float *delta = reinterpret_cast<float *>(ws + h_bytes);
-    const int warps = 8;
-    const unsigned blocks = (unsigned)((rows + warps - 1) / warps);
-    if (d->flags & TX_SDPA_OUT_F16)
-        txb::sdpa_bwd_prep_kernel<__half><<<blocks, warps * 32, 0, st>>>(d->dout, static_cast<const __half *>(d->out),
-                                                                       dout_h, delta, rows, (int)d->d);
-    else
-        txb::sdpa_bwd_prep_kernel<float><<<blocks, warps * 32, 0, st>>>(d->dout, static_cast<const float *>(d->out),
-                                                                      dout_h, delta, rows, (int)d->d);
+    auto prep = [&](auto out, auto dim) {
+        constexpr int D = decltype(dim)::value, rows_per_cta = 8 * 2 * (D == 64 ? 2 : 1);
+        txb::sdpa_bwd_prep_kernel<std::remove_const_t<std::remove_pointer_t<decltype(out)>>, D>
+            <<<(unsigned)((rows + rows_per_cta - 1) / rows_per_cta), 256, 0, st>>>(d->dout, out, dout_h, delta, rows);
+    };
+    auto prep_of = [&](auto out) {
+        if (d->d == 64) prep(out, std::integral_constant<int, 64>{});
+        else if (d->d == 128) prep(out, std::integral_constant<int, 128>{});
+        else prep(out, std::integral_constant<int, 256>{});
+    };
+    if (d->flags & TX_SDPA_OUT_F16) prep_of(static_cast<const __half *>(d->out));
+    else prep_of(static_cast<const float *>(d->out));
     g_launches++;
     int rc = (cudaGetLastError() == cudaSuccess) ? TX_OK : fail(TX_ERR_CUDA, "SDPA backward: preprocess launch failed");
     if (rc == TX_OK) {

@@ -21,6 +21,11 @@
 // tile's columns).  Head dims 64, 128 and 256 (at 256 the dK/dV kernel runs two CTAs per key tile,
 // each accumulating half of the gradient columns).  Every wait is bounded (ptx::mbar_wait); a wait that runs out
 // sets the CTA's abort flag and a code in the device status word.
+//
+// Bound, d = 128: shared-memory traffic in the dQ kernel (operands of the SS MMAs and the TMA writes: about 1 800 of 2 000
+// cycles per 128 x 128 tile), MMA issue in the dK/dV kernel (about 1 300 cycles per 128 x 64 tile); a CTA's start and end
+// are 15 to 25 % of a causal one.  B4 H16 S2048 d128 causal: 148 -> 141 us and 218 -> 182 us; B2 Hq12 Hkv4 S921 d64 causal:
+// dK/dV 79 -> 27 us, its items cut over clusters (split_k).
 #pragma once
 
 #include <cooperative_groups.h>
@@ -120,36 +125,50 @@ __device__ __forceinline__ void store_grad(const uint8_t *tile, float *dst, int6
 }
 
 // ------------------------------------------------------------------ preprocess
-// dO fp32 -> fp16 (MMA operand) and delta = rowsum(dO o O); one warp per row.
-template <typename OT>
-__global__ void sdpa_bwd_prep_kernel(const float *__restrict__ dout, const OT *__restrict__ out,
-                                     __half *__restrict__ dout_h, float *__restrict__ delta, int64_t rows, int d)
+// dO fp32 -> fp16 (MMA operand) and delta = rowsum(dO o O).  Bound: HBM (10 d + 4 or 8 d + 4 bytes a row).  Sixteen lanes a row
+// at d = 64, 32 otherwise, four values a lane and step; a warp requests two steps of rows at a time.  One row a warp and
+// eight bytes a lane took 30.3 us at B4 H16 S2048 d128, this 23.4 (6.9 TB/s; dO and O partly in L2).
+template <typename OT, int D>
+__global__ void __launch_bounds__(256) sdpa_bwd_prep_kernel(const float *__restrict__ dout, const OT *__restrict__ out,
+                                                            __half *__restrict__ dout_h, float *__restrict__ delta, int64_t rows)
 {
     ptx::grid_trigger();
-    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    const float *g = dout + row * d;
-    const OT *o = out + row * d;
-    __half *gh = dout_h + row * d;
-    float acc = 0.f;
-    for (int c = lane * 2; c < d; c += 64) {
-        const float2 gv = *reinterpret_cast<const float2 *>(g + c);
-        float ox, oy;
-        if constexpr (sizeof(OT) == 2) {
-            const __half2 hv = *reinterpret_cast<const __half2 *>(o + c);
-            ox = __low2float(hv); oy = __high2float(hv);
-        } else {
-            const float2 ov = *reinterpret_cast<const float2 *>(o + c);
-            ox = ov.x; oy = ov.y;
-        }
-        acc = fmaf(gv.x, ox, acc);
-        acc = fmaf(gv.y, oy, acc);
-        *reinterpret_cast<__half2 *>(gh + c) = __floats2half2_rn(gv.x, gv.y);
-    }
+    constexpr int LPR = D / 4 < 32 ? D / 4 : 32, RPW = 32 / LPR, STEPS = 2, PIECES = D / 4 / LPR;   // lanes a row, rows a warp step
+    const int lane = threadIdx.x & 31, gl = lane % LPR;
+    const int64_t row0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (RPW * STEPS) + lane / LPR;
+    float4 g[STEPS][PIECES], o[STEPS][PIECES];
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-    if (lane == 0) delta[row] = acc;
+    for (int t = 0; t < STEPS; ++t)
+#pragma unroll
+        for (int c = 0; c < PIECES; ++c) {
+            const int64_t row = row0 + t * RPW;
+            g[t][c] = o[t][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row >= rows) continue;
+            const int64_t at = row * D + (c * LPR + gl) * 4;
+            g[t][c] = *reinterpret_cast<const float4 *>(dout + at);
+            if constexpr (sizeof(OT) == 2) {
+                const uint2 h = *reinterpret_cast<const uint2 *>(out + at);
+                const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&h.x)), hi = __half22float2(*reinterpret_cast<const __half2 *>(&h.y));
+                o[t][c] = make_float4(lo.x, lo.y, hi.x, hi.y);
+            } else {
+                o[t][c] = *reinterpret_cast<const float4 *>(out + at);
+            }
+        }
+#pragma unroll
+    for (int t = 0; t < STEPS; ++t) {
+        const int64_t row = row0 + t * RPW;
+        float acc = 0.f;
+#pragma unroll
+        for (int c = 0; c < PIECES; ++c) {
+            const float4 a = g[t][c], b = o[t][c];
+            acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
+            if (row < rows)
+                *reinterpret_cast<uint2 *>(dout_h + row * D + (c * LPR + gl) * 4) = make_uint2(ptx::pack_half2(a.x, a.y), ptx::pack_half2(a.z, a.w));
+        }
+#pragma unroll
+        for (int w = LPR / 2; w > 0; w >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, w);
+        if (gl == 0 && row < rows) delta[row] = acc;
+    }
 }
 
 // ------------------------------------------------------------------ dQ

@@ -2,9 +2,9 @@
 //
 // This kernel backs the fp32 entry points (tensorax csrc/tensor_ops.h:170-194:
 // sdpa_naive_cuda / sdpa_tiled_cuda / sdpa_flash_cuda / sdpa_optimized_flash_cuda /
-// sdpa_mma_cuda when a mask or an unaligned shape is given) and every shape or
-// mask form the tcgen05 kernel does not take (dense additive masks, ragged head
-// dims, d_k != d_v).  All products and sums are fp32 FMAs and the exponential is
+// sdpa_mma_cuda) for what the tensor-core and decoding kernels do not take: fp32
+// head dims above 128 or no multiple of 4, unaligned tensors, fp16 with a dense
+// mask, and fp32 values that fp16 pairs cannot carry.  All products and sums are fp32 FMAs and the exponential is
 // expf, so results stay within 1e-5 of the reference CPU path
 // (csrc/cpu/tensor_cpu.cpp:464-529), which the fp16-operand tensor-core variants
 // of the reference cannot do.
