@@ -40,7 +40,10 @@ template <int D_, int NS_, bool MASK_ = false>
 struct X3Cfg {
     static constexpr int D = D_, NS = NS_;                 // D: 64 or 128, at least d_k and d_v
     static constexpr bool MASK = MASK_;
-    static constexpr int NM = D_ == 64 ? 2 : 1;            // stages of the mask tile
+    // Stages of the mask tile, as many as shared memory has room for: the mask comes from memory, 32 KB a tile, and with two
+    // stages and a rolled copy loop the softmax warps waited 1 480 of 3 060 cycles a tile for it (B4 H8 S512 d64: 49.6 -> 49.2 us
+    // a call with four, 48.4 with the loop unrolled as well).
+    static constexpr int NM = D_ == 64 ? 4 : 1;
     static constexpr int BM = 128, BN = 64;
     static constexpr int THREADS = 384;
     // registers: producer / MMA warpgroup, softmax warpgroup, accumulator warpgroup (128 * (56 + 192 + 248) <= 384 * 168)
@@ -325,8 +328,19 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                 if (wide) {
                     const int c = t & 15;                        // chunk of the row: 16 threads a row, 4 rows a step
                     const bool in = kv0 + c * 4 < p.Sk;
-                    for (int row = t >> 4; row < rows; row += 4)
-                        if (in) ptx::cp_async16(dst + (uint32_t)row * 256 + ((uint32_t)(c ^ (row & 7)) << 4), base + (size_t)row * p.Sk + kv0 + c * 4);
+                    const int r0 = t >> 4;
+                    // rows r0, r0 + 4, r0 + 8 ...: the swizzle alternates between two places, all else advances evenly
+                    const uint32_t d0 = dst + (uint32_t)r0 * 256;
+                    const uint32_t sw[2] = {(uint32_t)(c ^ r0) << 4, (uint32_t)(c ^ (r0 + 4)) << 4};
+                    const float *src = base + (size_t)r0 * p.Sk + kv0 + c * 4;
+                    const size_t step = (size_t)4 * p.Sk;
+                    const int n = in ? (rows - r0 + 3) / 4 : 0;
+                    if (n == BM / 4) {
+#pragma unroll
+                        for (int i = 0; i < BM / 4; ++i, src += step) ptx::cp_async16(d0 + (uint32_t)i * 1024 + sw[i & 1], src);
+                    } else {
+                        for (int i = 0; i < n; ++i, src += step) ptx::cp_async16(d0 + (uint32_t)i * 1024 + sw[i & 1], src);
+                    }
                 } else {
                     const bool in = kv0 + t < p.Sk;
                     for (int row = 0; row < rows; ++row)
