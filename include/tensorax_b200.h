@@ -55,7 +55,8 @@ enum {
                                 its kernel (fp32 in/out, fp16 MMA operands, csrc/cuda/kernels/attn.cu:441-603); fp16
                                 tolerances then apply.  Without the flag fp32 inputs always get exact fp32 arithmetic. */
     TX_SDPA_KV_LENS_HOST = 16, /* `kv_lens` is a HOST array, read during the call: up to 32 lengths travel with the launch,
-                                 longer arrays are copied to the device first (forward and backward descriptors) */
+                                 longer arrays with launches of their own in front of it, so that a captured call keeps
+                                 the lengths it was recorded with (forward, backward and layer descriptors) */
     TX_SDPA_P_IN_SMEM = 2    /* tensor-core kernel: stage P in shared memory instead of tensor memory
                                 (ignored for d = 512, where shared memory has no room for it) */
 };

@@ -22,4 +22,16 @@ struct KvLens {
     }
 };
 
+// Longer host arrays are brought to the device by value too, a chunk per launch: a copy would read the caller's array when
+// the stream gets to it -- after the call, where the array is pinned, and again at every replay, where the call was captured.
+struct KvLensChunk {
+    static constexpr int kMax = 960;   // with the rest of the parameters inside 4 KB
+    int32_t n, val[kMax];
+};
+
+__global__ void __launch_bounds__(256) put_kv_lens_kernel(const __grid_constant__ KvLensChunk c, int32_t *__restrict__ dst)
+{
+    for (int i = threadIdx.x; i < c.n; i += blockDim.x) dst[i] = c.val[i];
+}
+
 }  // namespace txb

@@ -313,7 +313,7 @@ txb::KvLens lens_of(const int32_t *lens, int flags, int64_t batch)
 void pool_free(char *p, cudaStream_t st);
 
 // `call(desc)` with the key lengths where the kernels can read them: a host array too long for the parameter block is
-// copied to the device first (the copy has read it when the call returns).
+// written to the device first, by launches that carry it (it has been read when the call returns).
 template <class Desc, class Call>
 int with_device_lens(const Desc *d, Call call)
 {
@@ -321,14 +321,22 @@ int with_device_lens(const Desc *d, Call call)
     cudaStream_t st = static_cast<cudaStream_t>(d->stream);
     char *ws = nullptr;
     if (int rc = pool_alloc(&ws, (size_t)d->batch * 4, st)) return rc;
-    Desc on_device = *d;
-    on_device.kv_lens = reinterpret_cast<const int32_t *>(ws);
-    on_device.flags &= ~TX_SDPA_KV_LENS_HOST;
-    int rc = TX_OK;
-    if (cudaMemcpyAsync(ws, d->kv_lens, (size_t)d->batch * 4, cudaMemcpyHostToDevice, st) != cudaSuccess)
-        rc = fail(TX_ERR_CUDA, "SDPA: copying the key lengths failed");
-    else
-        rc = call(&on_device);
+    int32_t *lens = reinterpret_cast<int32_t *>(ws);
+    auto body = [&]() -> int {
+        for (int64_t at = 0; at < d->batch; at += txb::KvLensChunk::kMax) {
+            txb::KvLensChunk c;
+            c.n = (int32_t)std::min<int64_t>(txb::KvLensChunk::kMax, d->batch - at);
+            std::copy(d->kv_lens + at, d->kv_lens + at + c.n, c.val);
+            txb::put_kv_lens_kernel<<<1, 256, 0, st>>>(c, lens + at);
+            g_launches++;
+            TX_CUDA(cudaGetLastError());
+        }
+        Desc on_device = *d;
+        on_device.kv_lens = lens;
+        on_device.flags &= ~TX_SDPA_KV_LENS_HOST;
+        return call(&on_device);
+    };
+    const int rc = body();
     pool_free(ws, st);
     return rc;
 }
