@@ -485,6 +485,20 @@ __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The next launch may start once every CTA of this one has come by here (or has ended).
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A word that hands what one kernel may see on to another: the store comes after everything visible to its thread, the
+// load before everything its thread (and, behind a barrier, its CTA) reads next.
+__device__ __forceinline__ void store_release(int *p, int v)
+{
+    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ int load_acquire(const int *p)
+{
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+// Orders this thread's earlier memory accesses before its later bulk-tensor copies (global and shared memory).
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
 // ---------------------------------------------------------------- math
 __device__ __forceinline__ float ex2_approx(float x)

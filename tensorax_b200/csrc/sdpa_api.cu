@@ -658,12 +658,12 @@ int bwd_split(double items, double longest, double mean, int sms, int per_sm)
 }
 
 template <int D, class DqCfg, class DkvCfg>
-int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __half *dout_h, const float *delta)
+int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __half *dout_h, const float *delta, int *prepared)
 {
     txb::BwdParams p;
     p.lse = d->lse; p.delta = delta; p.kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
     p.dq = d->dq; p.dk = d->dk; p.dv = d->dv;
-    p.status = status;
+    p.status = status; p.prepared = prepared;
     p.Hq = (int)d->q_heads; p.Hkv = (int)d->kv_heads; p.Sq = (int)d->seq_q; p.Sk = (int)d->seq_k;
     p.causal = d->causal ? 1 : 0;
     p.scale = 1.0f / std::sqrt((float)D);
@@ -1715,15 +1715,16 @@ static int backward_launch(const tx_sdpa_bwd_desc *d)
     if (int rc = status_word(&status)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(d->stream);
     const int64_t rows = d->batch * d->q_heads * d->seq_q;
-    const size_t h_bytes = align_up((size_t)rows * (size_t)d->d * 2, 256);
+    const size_t h_bytes = align_up((size_t)rows * (size_t)d->d * 2, 256), delta_bytes = align_up((size_t)rows * 4, 256);
     char *ws = nullptr;
-    if (int rc = pool_alloc(&ws, h_bytes + (size_t)rows * 4, st)) return rc;
+    if (int rc = pool_alloc(&ws, h_bytes + delta_bytes + sizeof(int), st)) return rc;
     __half *dout_h = reinterpret_cast<__half *>(ws);
     float *delta = reinterpret_cast<float *>(ws + h_bytes);
+    int *prepared = reinterpret_cast<int *>(ws + h_bytes + delta_bytes);
     auto prep = [&](auto out, auto dim) {
         constexpr int D = decltype(dim)::value, rows_per_cta = 8 * 2 * (D == 64 ? 2 : 1);
         txb::sdpa_bwd_prep_kernel<std::remove_const_t<std::remove_pointer_t<decltype(out)>>, D>
-            <<<(unsigned)((rows + rows_per_cta - 1) / rows_per_cta), 256, 0, st>>>(d->dout, out, dout_h, delta, rows);
+            <<<(unsigned)((rows + rows_per_cta - 1) / rows_per_cta), 256, 0, st>>>(d->dout, out, dout_h, delta, rows, prepared);
     };
     auto prep_of = [&](auto out) {
         if (d->d == 64) prep(out, std::integral_constant<int, 64>{});
@@ -1740,15 +1741,15 @@ static int backward_launch(const tx_sdpa_bwd_desc *d)
         // per SM and two row warpgroups, config-2 size).
         // d = 128: one CTA per SM for both, two row warpgroups, 128-key / 64-query tiles (all of tensor memory).
         if (d->d == 64)
-            rc = launch_bwd<64, txb::BwdDqCfg<64, 64, 3, 1, 2>, txb::BwdDkvCfg<64, 64, 3, 1, true, 2>>(d, st, status, dout_h, delta);
+            rc = launch_bwd<64, txb::BwdDqCfg<64, 64, 3, 1, 2>, txb::BwdDkvCfg<64, 64, 3, 1, true, 2>>(d, st, status, dout_h, delta, prepared);
         else if (d->d == 128)
-            rc = launch_bwd<128, txb::BwdDqCfg<128, 128, 3, 2, 2>, txb::BwdDkvCfg<128, 64, 3, 2, false, 3>>(d, st, status, dout_h, delta);
+            rc = launch_bwd<128, txb::BwdDqCfg<128, 128, 3, 2, 2>, txb::BwdDkvCfg<128, 64, 3, 2, false, 3>>(d, st, status, dout_h, delta, prepared);
         else
             // d = 256: dQ alone takes 256 tensor-memory columns (64-key tiles, single V stage: 224 KB of shared
             // memory); two CTAs per key tile each own 128 columns of dK and dV, with 32-query tiles so that two
             // stages each of Q and dO fit beside the resident K and V (a stage stays occupied from its first
             // read to its second, so one stage per ring would deadlock the MMA warp).
-            rc = launch_bwd<256, txb::BwdDqCfg<256, 64, 2, 1, 1>, txb::BwdDkvCfg<256, 32, 2, 1, false, 2, 2>>(d, st, status, dout_h, delta);
+            rc = launch_bwd<256, txb::BwdDqCfg<256, 64, 2, 1, 1>, txb::BwdDkvCfg<256, 32, 2, 1, false, 2, 2>>(d, st, status, dout_h, delta, prepared);
     }
     pool_free(ws, st);        // ordered after the kernels on `st`
     return rc;

@@ -43,6 +43,7 @@ struct BwdParams {
     KvLens kv_lens;           // optional [B]
     float *dq, *dk, *dv;      // [B,Hq,Sq,D], [B,Hkv,Sk,D], [B,Hkv,Sk,D] fp32
     int *status;
+    int *prepared;            // word of the workspace: 1 once the dQ kernel has the preprocess behind it
     int Hq, Hkv, Sq, Sk;
     int causal;
     float scale;              // 1/sqrt(d)
@@ -130,9 +131,11 @@ __device__ __forceinline__ void store_grad(const uint8_t *tile, float *dst, int6
 // eight bytes a lane took 30.3 us at B4 H16 S2048 d128, this 23.4 (6.9 TB/s; dO and O partly in L2).
 template <typename OT, int D>
 __global__ void __launch_bounds__(256) sdpa_bwd_prep_kernel(const float *__restrict__ dout, const OT *__restrict__ out,
-                                                            __half *__restrict__ dout_h, float *__restrict__ delta, int64_t rows)
+                                                            __half *__restrict__ dout_h, float *__restrict__ delta, int64_t rows,
+                                                            int *prepared)
 {
     ptx::grid_trigger();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *prepared = 0;
     constexpr int LPR = D / 4 < 32 ? D / 4 : 32, RPW = 32 / LPR, STEPS = 2, PIECES = D / 4 / LPR;   // lanes a row, rows a warp step
     const int lane = threadIdx.x & 31, gl = lane % LPR;
     const int64_t row0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (RPW * STEPS) + lane / LPR;
@@ -299,8 +302,13 @@ sdpa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     ptx::tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
     const bool run = (*abort_flag == 0) && n_tiles > 0;
+    // The dK/dV kernel starts under this one and reads what the preprocess wrote.  The wait makes that visible to this
+    // kernel, the word hands it on, and no CTA lets the dK/dV kernel start before its own thread 0 is past both.
     ptx::grid_wait();
-    ptx::grid_trigger();                         // after the wait: the dK/dV kernel relies on the preprocess being done
+    if (tid == 0) {
+        if (blockIdx.x == 0) ptx::store_release(p.prepared, 1);
+        ptx::grid_trigger();
+    }
 
     if (warp == 0) {
         if (run) {
@@ -624,6 +632,11 @@ sdpa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
             for (int pn = 0; pn < Cfg::KP; ++pn)
                 ptx::tma_load_3d(v_s + pn * (BMK * 128), &tm_v, kv_full, pn * 64, key0, kvh);
+            // From here on the preprocess' results are read (by the row warps behind the meeting).  The word stands: every
+            // CTA of the dQ kernel let this one start after it was stored.  Were it not seen, waiting for that kernel's end
+            // would do as well.
+            if (ptx::load_acquire(p.prepared) != 1) ptx::grid_wait();
+            ptx::fence_proxy_async();
             load_do(0);
         }
         if (*reinterpret_cast<volatile int *>(p.status) != 0) *abort_flag = 1;
