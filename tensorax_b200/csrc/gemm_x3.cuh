@@ -23,7 +23,6 @@
 // Every mbarrier wait is bounded.
 #pragma once
 #include "ptx.cuh"
-#include "sdpa_tc_x3.cuh"
 
 namespace txb {
 
@@ -104,7 +103,6 @@ struct GemmX3Problem {
     const float *bias;                     // optional [N]
     void *out;                             // [M, N], or [M / S, heads, S, N / heads] when heads > 0
     int M, S, heads;
-    __half *hi, *lo;                       // HALVES: the result's fp16 halves beside it, as the fp32 attention kernel reads them
     int w_row;                             // first row of this problem's W inside the W map
     int first_tile, tiles_n;
 };
@@ -112,18 +110,14 @@ struct GemmX3Params {
     GemmX3Problem prob[3];
     int n_probs, n_tiles, N, K;
     int out_f16;
-    int *range;                            // HALVES: x3_declines' two words; problem 2 is V
     int *status;
 };
 struct GemmX3Maps {
     CUtensorMap xh[3], xl[3], wh, wl;
 };
 
-// HALVES: the results' fp16 halves and the range words are written beside them (an instantiation of its own: carrying the
-// branch cost the output projection, which does not need it, 30 -> 34 us at B4 S1024 E1024)
-template <int BN_, bool HALVES_ = false>
+template <int BN_>
 struct GemmX3Cfg {
-    static constexpr bool HALVES = HALVES_;
     static constexpr int BM = 128, BN = BN_, BK = 64, CHUNK = 2;          // CHUNK: stages per accumulator
     static constexpr int THREADS = 384, REGS_LIGHT = 56, REGS_SUMS = 224; // 128 * 56 + 256 * 224 = 64512 = 384 * 168
     static constexpr uint32_t X_BYTES = BM * BK * 2, W_BYTES = BN * BK * 2;
@@ -259,8 +253,6 @@ gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ 
         const uint32_t turn = sbase + Cfg::OFF_TURN + (uint32_t)(warp - 4) * 4096;
         bool ok = run;
         int c = 0;
-        bool bad = false;
-        float vmax = 0.f;
         for (int tile = blockIdx.x; tile < p.n_tiles && ok; tile += gridDim.x) {
             float sum[HALF];
 #pragma unroll
@@ -287,9 +279,7 @@ gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ 
             if (!ok) break;
             // result: 32 rows x 32 columns at a time through shared memory (16-byte pieces at piece ^ (row & 7)), then
             // eight lanes store 128 bytes of one row
-            const int which = problem_of(tile);
-            const bool is_v = which == 2;
-            const GemmX3Problem &pr = p.prob[which];
+            const GemmX3Problem &pr = p.prob[problem_of(tile)];
             const int local = tile - pr.first_tile;
             const int row0 = local / pr.tiles_n * BM + quarter * 32, col0 = local % pr.tiles_n * BN + half * HALF;
             const float inv = row0 + lane < pr.M ? pr.inv_x[row0 + lane] : 0.f;
@@ -324,26 +314,12 @@ gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ 
                             *reinterpret_cast<uint2 *>(static_cast<__half *>(pr.out) + at) = u;
                         } else {
                             *reinterpret_cast<float4 *>(static_cast<float *>(pr.out) + at) = f;
-                            if constexpr (Cfg::HALVES) {
-                                uint2 hh, ll;
-                                split_quad(f, hh, ll);
-                                *reinterpret_cast<uint2 *>(pr.hi + at) = hh;
-                                *reinterpret_cast<uint2 *>(pr.lo + at) = ll;
-                                bad |= quad_too_large(f);
-                                if (is_v) vmax = fmaxf(vmax, quad_max(f));
-                            }
                         }
                     }
                 }
             }
         }
         if (run && !ok) { *abort_flag = 1; ptx::report(p.status, GX3_ERR_SUMS); }
-        if constexpr (Cfg::HALVES) {
-            const int wmax = __reduce_max_sync(0xffffffffu, __float_as_int(vmax));
-            const bool wbad = __any_sync(0xffffffffu, bad);
-            if (lane == 0 && wbad) atomicOr(p.range, 1);
-            if (lane == 0 && wmax > *reinterpret_cast<volatile int *>(p.range + 1)) atomicMax(p.range + 1, wmax);
-        }
     }
 
     ptx::tc_fence_before_sync();

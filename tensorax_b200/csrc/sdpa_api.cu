@@ -786,15 +786,6 @@ void fill_simt_params(txb::SimtParams *p, const tx_sdpa_desc *d)
     p->prof = nullptr;
 }
 
-// The operands of the fp32 tensor-core kernel where the caller has them already: fp16 halves of Q, K and V and the range words
-struct X3Operands {
-    const __half *qh, *ql, *kh, *kl, *vh, *vl;
-    const int *range;
-};
-
-template <class Cfg>
-int launch_x3_on(const tx_sdpa_desc *d, cudaStream_t st, int *status, const X3Operands &x);
-
 template <class Cfg>
 int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
 {
@@ -826,60 +817,49 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
         g_launches++;
         TX_CUDA(cudaGetLastError());
 
-        auto at = [&](size_t o) { return reinterpret_cast<const __half *>(ws + o); };
-        return launch_x3_on<Cfg>(d, st, status, {at(o_qh), at(o_ql), at(o_kh), at(o_kl), at(o_vh), at(o_vl), range});
+        CUtensorMap qh, ql, kh, kl, vh, vl, to;
+        const int64_t sq = d->batch * d->q_heads, sk = d->batch * d->kv_heads;
+        if (int r = make_map(&qh, ws + o_qh, sq, d->seq_q, dk8, Cfg::BM)) return r;
+        if (int r = make_map(&ql, ws + o_ql, sq, d->seq_q, dk8, Cfg::BM)) return r;
+        if (int r = make_map(&kh, ws + o_kh, sk, d->seq_k, dk8, Cfg::BN)) return r;
+        if (int r = make_map(&kl, ws + o_kl, sk, d->seq_k, dk8, Cfg::BN)) return r;
+        if (int r = make_map(&vh, ws + o_vh, sk, d->seq_k, dv8, Cfg::BN)) return r;
+        if (int r = make_map(&vl, ws + o_vl, sk, d->seq_k, dv8, Cfg::BN)) return r;
+        if (int r = make_map(&to, d->out, sq, d->seq_q, d->d_v, 32, 4)) return r;
+        txb::X3Params p;
+        p.out = static_cast<float *>(d->out);
+        p.mask = d->mask;
+        p.kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
+        p.range = range;
+        p.status = status;
+        p.Hq = (int)d->q_heads; p.Hkv = (int)d->kv_heads; p.Sq = (int)d->seq_q; p.Sk = (int)d->seq_k;
+        p.dk = (int)d->d_k; p.dv = (int)d->d_v;
+        p.causal = d->causal ? 1 : 0;
+        p.scale = 1.0f / std::sqrt((float)d->d_k);
+        p.scale_log2 = p.scale * 1.4426950408889634f;
+        const int64_t n_tiles = (d->seq_q + Cfg::BM - 1) / Cfg::BM;
+        int64_t group = 1;
+        if (int r = causal_group(d, n_tiles, &group)) return r;
+        p.group = (int)group; p.n_tiles_q = (int)n_tiles; p.BH = (int)sq;
+        if (n_tiles * sq > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA: more than 2^31 work items");
+        if (int r = allow_smem<txb::sdpa_tc_x3_kernel<Cfg>>((int)Cfg::SMEM_BYTES)) return r;
+        if (int r = launch_behind(txb::sdpa_tc_x3_kernel<Cfg>, dim3((unsigned)(n_tiles * sq)), Cfg::THREADS, Cfg::SMEM_BYTES, st, 1,
+                                  qh, ql, kh, kl, vh, vl, to, p))
+            return r;
+        // the exact kernel behind it: works only when the split pass found a value the fp16 pairs cannot carry
+        txb::SimtParams sp2;
+        fill_simt_params(&sp2, d);
+        sp2.only_if = range;
+        return launch_simt<float>(sp2, st);
     };
     rc = body();
     pool_free(ws, st);
     return rc;
 }
 
-template <class Cfg>
-int launch_x3_on(const tx_sdpa_desc *d, cudaStream_t st, int *status, const X3Operands &x)
+int launch_x3(const tx_sdpa_desc *d, cudaStream_t st, int *status)
 {
-    const int64_t dk8 = (d->d_k + 7) / 8 * 8, dv8 = (d->d_v + 7) / 8 * 8;
-    CUtensorMap qh, ql, kh, kl, vh, vl, to;
-    const int64_t sq = d->batch * d->q_heads, sk = d->batch * d->kv_heads;
-    if (int r = make_map(&qh, x.qh, sq, d->seq_q, dk8, Cfg::BM)) return r;
-    if (int r = make_map(&ql, x.ql, sq, d->seq_q, dk8, Cfg::BM)) return r;
-    if (int r = make_map(&kh, x.kh, sk, d->seq_k, dk8, Cfg::BN)) return r;
-    if (int r = make_map(&kl, x.kl, sk, d->seq_k, dk8, Cfg::BN)) return r;
-    if (int r = make_map(&vh, x.vh, sk, d->seq_k, dv8, Cfg::BN)) return r;
-    if (int r = make_map(&vl, x.vl, sk, d->seq_k, dv8, Cfg::BN)) return r;
-    if (int r = make_map(&to, d->out, sq, d->seq_q, d->d_v, 32, 4)) return r;
-    txb::X3Params p;
-    p.out = static_cast<float *>(d->out);
-    p.mask = d->mask;
-    p.kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
-    p.range = x.range;
-    p.status = status;
-    p.Hq = (int)d->q_heads; p.Hkv = (int)d->kv_heads; p.Sq = (int)d->seq_q; p.Sk = (int)d->seq_k;
-    p.dk = (int)d->d_k; p.dv = (int)d->d_v;
-    p.causal = d->causal ? 1 : 0;
-    p.scale = 1.0f / std::sqrt((float)d->d_k);
-    p.scale_log2 = p.scale * 1.4426950408889634f;
-    const int64_t n_tiles = (d->seq_q + Cfg::BM - 1) / Cfg::BM;
-    int64_t group = 1;
-    if (int r = causal_group(d, n_tiles, &group)) return r;
-    p.group = (int)group; p.n_tiles_q = (int)n_tiles; p.BH = (int)sq;
-    if (n_tiles * sq > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA: more than 2^31 work items");
-    if (int r = allow_smem<txb::sdpa_tc_x3_kernel<Cfg>>((int)Cfg::SMEM_BYTES)) return r;
-    if (int r = launch_behind(txb::sdpa_tc_x3_kernel<Cfg>, dim3((unsigned)(n_tiles * sq)), Cfg::THREADS, Cfg::SMEM_BYTES, st, 1,
-                              qh, ql, kh, kl, vh, vl, to, p))
-        return r;
-    // the exact kernel behind it: works only when the split pass found a value the fp16 pairs cannot carry
-    txb::SimtParams sp2;
-    fill_simt_params(&sp2, d);
-    sp2.only_if = x.range;
-    return launch_simt<float>(sp2, st);
-}
-
-int launch_x3(const tx_sdpa_desc *d, cudaStream_t st, int *status, const X3Operands *x = nullptr)
-{
-    auto on = [&](auto cfg) {
-        using Cfg = decltype(cfg);
-        return x ? launch_x3_on<Cfg>(d, st, status, *x) : launch_x3_t<Cfg>(d, st, status);
-    };
+    auto on = [&](auto cfg) { return launch_x3_t<decltype(cfg)>(d, st, status); };
     const bool narrow = d->d_k <= 64 && d->d_v <= 64;
     if (d->mask) return narrow ? on(txb::X3Cfg<64, 2, true>{}) : on(txb::X3Cfg<128, 2, true>{});
     return narrow ? on(txb::X3Cfg<64, 4>{}) : on(txb::X3Cfg<128, 2>{});
@@ -971,13 +951,9 @@ int launch_gemm_x3(const txb::GemmX3Params &p, const __half *const *xh, const __
         return (double)((tiles + sms - 1) / sms) * tile;
     };
     const double t256 = time(256, 1.0), t128 = time(128, 0.53), t64 = time(64, 0.37);
-    auto on = [&](auto plain, auto halves) {
-        return p.range ? launch_gemm_x3_t<decltype(halves)>(p, xh, xl, wh, wl, w_rows, st)
-                       : launch_gemm_x3_t<decltype(plain)>(p, xh, xl, wh, wl, w_rows, st);
-    };
-    if (t256 <= t128 && t256 <= t64) return on(txb::GemmX3Cfg<256>{}, txb::GemmX3Cfg<256, true>{});
-    if (t128 <= t64) return on(txb::GemmX3Cfg<128>{}, txb::GemmX3Cfg<128, true>{});
-    return on(txb::GemmX3Cfg<64>{}, txb::GemmX3Cfg<64, true>{});
+    if (t256 <= t128 && t256 <= t64) return launch_gemm_x3_t<txb::GemmX3Cfg<256>>(p, xh, xl, wh, wl, w_rows, st);
+    if (t128 <= t64) return launch_gemm_x3_t<txb::GemmX3Cfg<128>>(p, xh, xl, wh, wl, w_rows, st);
+    return launch_gemm_x3_t<txb::GemmX3Cfg<64>>(p, xh, xl, wh, wl, w_rows, st);
 }
 
 // The whole layer on one stream: operands split, three projections in one launch (head-split, fp32 or fp16), attention,
@@ -1008,23 +984,6 @@ int mha_launch(const tx_mha_desc *d)
     const size_t es = f16 ? 2 : 4;
     const size_t o_p[3] = {take((size_t)(Mq * E) * es), take((size_t)(Mk * E) * es), take((size_t)(Mk * E) * es)};
     const size_t o_a = take((size_t)(Mq * E) * 4);
-    // fp32 attention on the tensor cores: the projections write the fp16 halves it reads beside their fp32 results (which
-    // stay for the exact kernel), in place of a pass over the results (B4 S1024 E1024: 18 us of 224, and a memset's wait)
-    tx_sdpa_desc a;
-    std::memset(&a, 0, sizeof a);
-    a.q = reinterpret_cast<const void *>(o_p[0]); a.k = reinterpret_cast<const void *>(o_p[1]); a.v = reinterpret_cast<const void *>(o_p[2]);
-    a.mask = d->mask; a.kv_lens = d->kv_lens; a.out = reinterpret_cast<void *>(o_a);
-    a.batch = d->batch; a.q_heads = a.kv_heads = d->heads;
-    a.seq_q = d->seq_q; a.seq_k = d->seq_k; a.d_k = a.d_v = E / d->heads;
-    a.dtype = f16 ? TX_DTYPE_F16 : TX_DTYPE_F32;
-    a.causal = d->causal; a.flags = d->flags & TX_SDPA_KV_LENS_HOST; a.stream = d->stream;
-    // (the offsets are as aligned as the pointers will be; the halves' rows are unpadded, so whole 16-byte pieces)
-    const bool halves = !f16 && a.d_k % 8 == 0 && x3_eligible(&a) && !decode_eligible(&a);
-    size_t o_h[3] = {}, o_l[3] = {}, o_range = 0;
-    if (halves) {
-        for (int i = 0; i < 3; ++i) { o_h[i] = take((size_t)(M[i] * E) * 2); o_l[i] = take((size_t)(M[i] * E) * 2); }
-        o_range = take(2 * sizeof(int));
-    }
     // the attention result's halves go where the inputs' were (none is needed any more and Q's are as large)
     const size_t o_ah = o_xh[0], o_al = o_xl[0], o_ai = o_xi[0];
 
@@ -1045,37 +1004,36 @@ int mha_launch(const tx_mha_desc *d)
         for (int i = 0; i < 3; ++i)
             if (from[i] == i) add(x[i], o_xh[i], o_xl[i], o_xi[i], M[i], 0, 0, 1);
         for (int i = 0; i < 4; ++i) add(w[i], o_wh, o_wl, o_wi, E, i * E, 0, 1);
-        int *range = halves ? reinterpret_cast<int *>(ws + o_range) : nullptr;
-        if (halves) TX_CUDA(cudaMemsetAsync(range, 0, 2 * sizeof(int), st));
         txb::split_rows_kernel<<<split_grid(), 256, 0, st>>>(sp);          // behind whatever the caller enqueued: a plain launch
         g_launches++;
         TX_CUDA(cudaGetLastError());
 
         txb::GemmX3Params g;
-        g.N = g.K = (int)E; g.status = status; g.out_f16 = f16 ? 1 : 0; g.n_probs = 3; g.range = range;
+        g.N = g.K = (int)E; g.status = status; g.out_f16 = f16 ? 1 : 0; g.n_probs = 3;
         const __half *xh[3], *xl[3];
         for (int i = 0; i < 3; ++i) {
             xh[i] = half_at(o_xh[i]); xl[i] = half_at(o_xl[i]);
             g.prob[i] = {float_at(o_xi[i]), float_at(o_wi) + i * E, bias[i], ws + o_p[i], (int)M[i], (int)seq[i], (int)d->heads,
-                         halves ? half_at(o_h[i]) : nullptr, halves ? half_at(o_l[i]) : nullptr, (int)(i * E), 0, 0};
+                         (int)(i * E), 0, 0};
         }
         if (int rc = launch_gemm_x3(g, xh, xl, half_at(o_wh), half_at(o_wl), 3 * E, st)) return rc;
 
+        tx_sdpa_desc a;
+        std::memset(&a, 0, sizeof a);
         a.q = ws + o_p[0]; a.k = ws + o_p[1]; a.v = ws + o_p[2]; a.out = ws + o_a;
-        if (halves) {
-            const X3Operands ops = {half_at(o_h[0]), half_at(o_l[0]), half_at(o_h[1]), half_at(o_l[1]), half_at(o_h[2]), half_at(o_l[2]), range};
-            if (int rc = validate(&a)) return rc;
-            if (int rc = with_device_lens(&a, [&](const tx_sdpa_desc *e) { return launch_x3(e, st, status, &ops); })) return rc;
-        } else if (int rc = forward(&a)) {
-            return rc;
-        }
+        a.mask = d->mask; a.kv_lens = d->kv_lens;
+        a.batch = d->batch; a.q_heads = a.kv_heads = d->heads;
+        a.seq_q = d->seq_q; a.seq_k = d->seq_k; a.d_k = a.d_v = E / d->heads;
+        a.dtype = f16 ? TX_DTYPE_F16 : TX_DTYPE_F32;
+        a.causal = d->causal; a.flags = d->flags & TX_SDPA_KV_LENS_HOST; a.stream = d->stream;
+        if (int rc = forward(&a)) return rc;
 
         sp.n_segs = 0; sp.rows = 0;
         add(float_at(o_a), o_ah, o_al, o_ai, Mq, 0, (int)d->heads, d->seq_q);
         if (int rc = launch_behind(txb::split_rows_kernel, split_grid(), 256, 0, st, 1, sp)) return rc;
-        g.n_probs = 1; g.out_f16 = 0; g.range = nullptr;
+        g.n_probs = 1; g.out_f16 = 0;
         g.prob[0] = {float_at(o_ai), float_at(o_wi) + 3 * E, d->bo, d->out, (int)Mq, (int)d->seq_q, 0,
-                     nullptr, nullptr, 0, 0, 0};
+                     0, 0, 0};
         xh[0] = half_at(o_ah); xl[0] = half_at(o_al);
         return launch_gemm_x3(g, xh, xl, half_at(o_wh) + 3 * E * E, half_at(o_wl) + 3 * E * E, E, st);
     };

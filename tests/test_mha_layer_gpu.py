@@ -75,8 +75,8 @@ def test_rows_of_any_magnitude_keep_their_relative_precision():
 @pytest.mark.parametrize("E,H", [(512, 8), (384, 3), (240, 5)])
 @pytest.mark.parametrize("scale", [1.0, 1e-4, 1e6])
 def test_halves_written_by_the_projections(E, H, scale):
-    """Attention reads the fp16 halves that the projections write (head dims 64, 128, 48; partial row tiles); values too
-    small or too large for them go to the exact kernel.  Bound: four chained fp32 stages, 2e-5 of the result."""
+    """From the projections into the attention step (head dims 64, 128, 48; partial row tiles), with values of any size.
+    Bound: four chained fp32 stages, 2e-5 of the result."""
     mha, params = layer(E, H, False)
     x, y = seeded(6, 2, 301, E), (scale * seeded(7, 2, 333, E)).astype(np.float32)
     k = seeded(8, 2, 333, E)
