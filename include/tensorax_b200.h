@@ -100,8 +100,10 @@ TX_API int tx_host_free_pinned(void *ptr);
  *      dense mask, run on the tensor cores: every fp32 operand is carried as two fp16 numbers (hi + lo, 22 significand
  *      bits), every product is three tcgen05 MMAs, tiles are summed in fp32 registers, the softmax is fp32 (within 2e-6 of
  *      the reference's sdpa_cpu on unit-variance inputs, the figure of the exact kernel; 3e-5 at scores of +-100, where the
- *      exact kernel itself is at 1e-5).  A device-side range check sends a call with |x| >= 2^15 or a non-finite Q, K or V
- *      to the exact CUDA-core kernel, which also takes every other shape.  Calls with few query rows per K/V head take
+ *      exact kernel itself is at 1e-5).  Rows of Q and 64-key tiles of K and V are scaled by powers of two first, so magnitudes
+ *      do not matter.  A device-side check sends a call to the exact CUDA-core kernel, which also takes every other shape,
+ *      where scaling does not help: a value that is not finite, max |Q| * max |K| above 2^19, or a tile of V whose keys'
+ *      largest elements are more than 2^13 apart.  Calls with few query rows per K/V head take
  *      the decoding kernel (exact fp32 products). */
 TX_API int tx_sdpa_naive_cuda(const float *Q, const float *K, const float *V, const float *mask,
                               float *out, int64_t batch_size, int64_t num_heads,

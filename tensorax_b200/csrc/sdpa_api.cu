@@ -786,36 +786,49 @@ void fill_simt_params(txb::SimtParams *p, const tx_sdpa_desc *d)
     p->prof = nullptr;
 }
 
+// `zeroed`: three words of device memory that are zero behind a launch of this library that lets its successor start under
+// its end (the layer); without them the call brings its own.
 template <class Cfg>
-int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
+int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status, int *zeroed)
 {
     const int64_t rows_q = d->batch * d->q_heads * d->seq_q, rows_k = d->batch * d->kv_heads * d->seq_k;
     const int64_t dk8 = (d->d_k + 7) / 8 * 8, dv8 = (d->d_v + 7) / 8 * 8;       // row length of the fp16 copies
-    // workspace: hi and lo fp16 copies of Q, K, V and the range words, stream-ordered pool memory
-    const size_t bq = align_up((size_t)(rows_q * dk8) * 2, 256), bk = align_up((size_t)(rows_k * dk8) * 2, 256),
-                 bv = align_up((size_t)(rows_k * dv8) * 2, 256);
-    const size_t o_qh = 0, o_ql = bq, o_kh = 2 * bq, o_kl = o_kh + bk, o_vh = o_kl + bk, o_vl = o_vh + bv, o_flag = o_vl + bv;
+    const int64_t slabs_k = d->batch * d->kv_heads, tiles_k = (d->seq_k + txb::X3_TILE - 1) / txb::X3_TILE;
+    const int64_t tiles_q = (rows_q + txb::X3_TILE - 1) / txb::X3_TILE;
+    if (tiles_q + 2 * slabs_k * tiles_k > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA: more than 2^31 work items");
+    // workspace: hi and lo fp16 copies of Q, K and V, their factors and the range words, stream-ordered pool memory
+    size_t total = 0;
+    auto take = [&](int64_t bytes) { const size_t at = total; total += align_up((size_t)bytes, 256); return at; };
+    const size_t o_qh = take(rows_q * dk8 * 2), o_ql = take(rows_q * dk8 * 2), o_kh = take(rows_k * dk8 * 2), o_kl = take(rows_k * dk8 * 2),
+                 o_vh = take(rows_k * dv8 * 2), o_vl = take(rows_k * dv8 * 2);
+    const size_t o_qf = take(rows_q * 4), o_kf = take(slabs_k * tiles_k * 4), o_vf = take(slabs_k * tiles_k * 4), o_range = take(3 * sizeof(int));
     char *ws = nullptr;
-    if (int rc = pool_alloc(&ws, o_flag + 256, st)) return rc;
+    if (int rc = pool_alloc(&ws, total, st)) return rc;
+    auto float_at = [&](size_t at) { return reinterpret_cast<float *>(ws + at); };
     int rc = TX_OK;
     auto body = [&]() -> int {
-        int *range = reinterpret_cast<int *>(ws + o_flag);
-        TX_CUDA(cudaMemsetAsync(range, 0, 2 * sizeof(int), st));
+        int *range = zeroed ? zeroed : reinterpret_cast<int *>(ws + o_range);
+        if (!zeroed) TX_CUDA(cudaMemsetAsync(range, 0, 3 * sizeof(int), st));
         txb::SplitParams sp;
-        auto seg = [&](const void *x, size_t hi, size_t lo, int64_t rows, int64_t n, int64_t n8) {
-            return txb::SplitSeg{static_cast<const float *>(x), reinterpret_cast<__half *>(ws + hi), reinterpret_cast<__half *>(ws + lo),
-                                 rows * n8 / 4, (int)(n / 4), (int)(n8 / 4)};
+        auto seg = [&](int i, const void *x, size_t hi, size_t lo, size_t factor, int64_t S, int64_t tiles, int64_t first, int64_t n, int64_t n8) {
+            sp.seg[i] = {static_cast<const float *>(x), reinterpret_cast<__half *>(ws + hi), reinterpret_cast<__half *>(ws + lo),
+                         float_at(factor), (long long)S, (int)tiles, (int)first, (int)(n / 4), (int)(n8 / 8)};
         };
-        sp.seg[0] = seg(d->q, o_qh, o_ql, rows_q, d->d_k, dk8);
-        sp.seg[1] = seg(d->k, o_kh, o_kl, rows_k, d->d_k, dk8);
-        sp.seg[2] = seg(d->v, o_vh, o_vl, rows_k, d->d_v, dv8);
+        seg(0, d->q, o_qh, o_ql, o_qf, rows_q, tiles_q, 0, d->d_k, dk8);
+        seg(1, d->k, o_kh, o_kl, o_kf, d->seq_k, tiles_k, tiles_q, d->d_k, dk8);
+        seg(2, d->v, o_vh, o_vl, o_vf, d->seq_k, tiles_k, tiles_q + slabs_k * tiles_k, d->d_v, dv8);
         sp.range = range;
-        int sms = 0;
-        if (int r = sm_count(&sms)) return r;
-        const int64_t want = (std::max({sp.seg[0].n4, sp.seg[1].n4, sp.seg[2].n4}) + 255) / 256;
-        txb::split_f32_hi_lo_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(want, 16 * sms)), 256, 0, st>>>(sp);
-        g_launches++;
-        TX_CUDA(cudaGetLastError());
+        const dim3 ctas((unsigned)(tiles_q + 2 * slabs_k * tiles_k));
+        const int64_t groups = std::max(dk8, dv8) / 8;
+        auto kernel = groups <= 4 ? txb::split_f32_hi_lo_kernel<1> : (groups <= 8 ? txb::split_f32_hi_lo_kernel<2> :
+                      (groups <= 12 ? txb::split_f32_hi_lo_kernel<3> : txb::split_f32_hi_lo_kernel<4>));
+        if (zeroed) {
+            if (int r = launch_behind(kernel, ctas, 256, 0, st, 1, sp)) return r;
+        } else {
+            kernel<<<ctas, 256, 0, st>>>(sp);                            // behind whatever the caller enqueued: a plain launch
+            g_launches++;
+            TX_CUDA(cudaGetLastError());
+        }
 
         CUtensorMap qh, ql, kh, kl, vh, vl, to;
         const int64_t sq = d->batch * d->q_heads, sk = d->batch * d->kv_heads;
@@ -831,6 +844,7 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
         p.mask = d->mask;
         p.kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
         p.range = range;
+        p.qf = float_at(o_qf); p.kf = float_at(o_kf); p.vf = float_at(o_vf);
         p.status = status;
         p.Hq = (int)d->q_heads; p.Hkv = (int)d->kv_heads; p.Sq = (int)d->seq_q; p.Sk = (int)d->seq_k;
         p.dk = (int)d->d_k; p.dv = (int)d->d_v;
@@ -857,9 +871,9 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status)
     return rc;
 }
 
-int launch_x3(const tx_sdpa_desc *d, cudaStream_t st, int *status)
+int launch_x3(const tx_sdpa_desc *d, cudaStream_t st, int *status, int *zeroed = nullptr)
 {
-    auto on = [&](auto cfg) { return launch_x3_t<decltype(cfg)>(d, st, status); };
+    auto on = [&](auto cfg) { return launch_x3_t<decltype(cfg)>(d, st, status, zeroed); };
     const bool narrow = d->d_k <= 64 && d->d_v <= 64;
     if (d->mask) return narrow ? on(txb::X3Cfg<64, 2, true>{}) : on(txb::X3Cfg<128, 2, true>{});
     return narrow ? on(txb::X3Cfg<64, 4>{}) : on(txb::X3Cfg<128, 2>{});
@@ -983,7 +997,7 @@ int mha_launch(const tx_mha_desc *d)
     const size_t o_wh = take((size_t)(4 * E * E) * 2), o_wl = take((size_t)(4 * E * E) * 2), o_wi = take((size_t)(4 * E) * 4);
     const size_t es = f16 ? 2 : 4;
     const size_t o_p[3] = {take((size_t)(Mq * E) * es), take((size_t)(Mk * E) * es), take((size_t)(Mk * E) * es)};
-    const size_t o_a = take((size_t)(Mq * E) * 4);
+    const size_t o_a = take((size_t)(Mq * E) * 4), o_range = take(3 * sizeof(int));
     // the attention result's halves go where the inputs' were (none is needed any more and Q's are as large)
     const size_t o_ah = o_xh[0], o_al = o_xl[0], o_ai = o_xi[0];
 
@@ -993,6 +1007,8 @@ int mha_launch(const tx_mha_desc *d)
     auto float_at = [&](size_t at) { return reinterpret_cast<float *>(ws + at); };
     auto body = [&]() -> int {
         txb::SplitRowsParams sp;
+        int *range = reinterpret_cast<int *>(ws + o_range);              // of the attention step
+        TX_CUDA(cudaMemsetAsync(range, 0, 3 * sizeof(int), st));
         sp.n_segs = 0; sp.rows = 0; sp.K = (int)E;
         auto add = [&](const float *src, size_t hi, size_t lo, size_t inv, int64_t rows, int64_t first_row, int heads, int64_t S) {
             txb::SplitRowsSeg &s = sp.seg[sp.n_segs++];
@@ -1026,7 +1042,12 @@ int mha_launch(const tx_mha_desc *d)
         a.seq_q = d->seq_q; a.seq_k = d->seq_k; a.d_k = a.d_v = E / d->heads;
         a.dtype = f16 ? TX_DTYPE_F16 : TX_DTYPE_F32;
         a.causal = d->causal; a.flags = d->flags & TX_SDPA_KV_LENS_HOST; a.stream = d->stream;
-        if (int rc = forward(&a)) return rc;
+        if (x3_eligible(&a) && !decode_eligible(&a)) {
+            if (int rc = validate(&a)) return rc;
+            if (int rc = with_device_lens(&a, [&](const tx_sdpa_desc *e) { return launch_x3(e, st, status, range); })) return rc;
+        } else if (int rc = forward(&a)) {
+            return rc;
+        }
 
         sp.n_segs = 0; sp.rows = 0;
         add(float_at(o_a), o_ah, o_al, o_ai, Mq, 0, (int)d->heads, d->seq_q);

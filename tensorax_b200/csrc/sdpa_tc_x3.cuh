@@ -4,9 +4,11 @@
 // accumulated in fp32 in tensor memory (the lo*lo term is below fp32's own rounding).  It stands where the
 // reference's fp32 kernels do (tensorax csrc/cuda/kernels/attn.cu:296-656 sdpa_kernel_mma and the naive / tiled /
 // flash forms before it) for head dims up to 128 (multiples of 4; d_k and d_v may differ), with or without a dense
-// additive mask, for |x| < 2^15 everywhere.
-// The split pass that writes the hi / lo copies also checks the range and raises a device flag when a value does
-// not fit; this kernel then returns at once and the exact CUDA-core kernel, launched behind it, does the work.
+// additive mask, at any magnitude: the split pass scales every row of Q and every 64-key tile of K and V by a power of two
+// that brings its largest element to [2^13, 2^14), and writes the factors.  A pair is then exact to 22 bits down to 2^-17
+// of that largest element and to 2^-39 of it below.  Q's and K's factors join the softmax scale of a (row, tile), V's the
+// accumulation; both are exact.  Where that is not enough (x3_declines) this kernel returns at once and the exact
+// CUDA-core kernel, launched behind it, does the work.
 //
 // One CTA per SM and 128-row query tile, 64 keys per tile:
 //   warp 0        TMA producer: Q hi / lo once, then K hi / lo and V hi / lo of every key tile through an NS-deep ring
@@ -36,6 +38,8 @@
 
 namespace txb {
 
+constexpr int X3_TILE = 64;      // keys per tile, each tile of K and V with a factor of its own; the split pass's CTAs
+
 template <int D_, int NS_, bool MASK_ = false>
 struct X3Cfg {
     static constexpr int D = D_, NS = NS_;                 // D: 64 or 128, at least d_k and d_v
@@ -44,7 +48,7 @@ struct X3Cfg {
     // stages and a rolled copy loop the softmax warps waited 1 480 of 3 060 cycles a tile for it (B4 H8 S512 d64: 49.6 -> 49.2 us
     // a call with four, 48.4 with the loop unrolled as well).
     static constexpr int NM = D_ == 64 ? 4 : 1;
-    static constexpr int BM = 128, BN = 64;
+    static constexpr int BM = 128, BN = X3_TILE;
     static constexpr int THREADS = 384;
     // registers: producer / MMA warpgroup, softmax warpgroup, accumulator warpgroup (128 * (56 + 192 + 248) <= 384 * 168)
     static constexpr int REGS_LIGHT = 56, REGS_SOFTMAX = 192, REGS_ACC = 248;
@@ -73,19 +77,23 @@ struct X3Cfg {
     static_assert(Q_BYTES / 4 >= 4096, "a softmax warp stages its results in its quarter of the Q buffers");
 };
 
-// range[0]: some |x| >= 2^15 or not finite.  range[1]: the bits of max |v|: a pair is exact to 2^-25 absolutely, which is
-// fp32-grade against a V of ordinary size only (errors of Q and K act on the scores absolutely, so small ones do no harm).
+// The split pass's words.  range[0]: some value is not finite, or the largest elements of the rows of one tile of V lie more
+// than 2^13 apart, so that the small rows would keep fewer than 25 bits.  range[1], range[2]: the bits of max |q| and max |k|:
+// what scaling leaves of a row or tile below 2^-39 of its maximum is worth up to 2^-39 max |q| max |k| in a score (sqrt(d)
+// such terms, times 1 / sqrt(d)), which stays below 2^-20 here.
 __device__ __forceinline__ bool x3_declines(const int *range)
 {
     const volatile int *w = range;
-    return w[0] != 0 || (w[1] != 0 && __int_as_float(w[1]) < 0.0625f);
+    return w[0] != 0 || __int_as_float(w[1]) * __int_as_float(w[2]) > 524288.f;
 }
 
 struct X3Params {
     float *out;               // [B,Hq,Sq,dv] fp32
     const float *mask;        // dense additive [B,Hq,Sq,Sk] (MASK instantiations)
     KvLens kv_lens;           // optional [B]
-    const int *range;         // the split pass's two words (see x3_declines)
+    const int *range;         // the split pass's three words (see x3_declines)
+    const float *qf;          // [B,Hq,Sq] what undoes the scale of a row of Q
+    const float *kf, *vf;     // [B,Hkv,ceil(Sk / 64)] the same of a tile of K and V
     int *status;              // device word: 0 = ok, else first failing wait's code
     int Hq, Hkv, Sq, Sk;
     int dk, dv;
@@ -363,7 +371,8 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
         const uint32_t t_s = tmem + lane_base + Cfg::COL_S;
         const uint32_t t_ph = tmem + lane_base + Cfg::COL_PH, t_pl = tmem + lane_base + Cfg::COL_PL;
         constexpr float kLog2e = 1.4426950408889634f;
-        const float scale = Cfg::MASK ? kLog2e : p.scale_log2;
+        const float row_scale = (Cfg::MASK ? p.scale : p.scale_log2) * (row < p.Sq ? p.qf[(size_t)bh * p.Sq + row] : 1.f);
+        const int f0 = kvh * ((p.Sk + BN - 1) / BN);     // factor of the head's first tile
         float m_run = Cfg::MASK ? -FLT_MAX : -1.0e30f;           // finite stand-in for "no key seen yet"
         float l = 0.f;
         bool ok = run;
@@ -374,6 +383,8 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
         };
         for (int j = 0; j < nt && ok; ++j) {
             const int kv0 = j * BN;
+            // not 0, however small the factors: -inf * 0 would make a NaN of a key that is not seen
+            const float tile_scale = fmaxf(row_scale * p.kf[f0 + j], FLT_MIN), scale = Cfg::MASK ? kLog2e : tile_scale;
             ok = ptx::mbar_wait(s_full, (uint32_t)j & 1u, abort_flag);
             if (!ok) break;
             ptx::tc_fence_after_sync();
@@ -391,10 +402,10 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                 for (int i = 0; i < BN; i += 4) {
                     uint32_t a, b2, c, d;
                     ptx::ld_shared_v4(mrow + ((uint32_t)((i >> 2) ^ (r & 7)) << 4), a, b2, c, d);
-                    sv[i] = __float_as_uint(fmaf(__uint_as_float(sv[i]), p.scale, __uint_as_float(a)));
-                    sv[i + 1] = __float_as_uint(fmaf(__uint_as_float(sv[i + 1]), p.scale, __uint_as_float(b2)));
-                    sv[i + 2] = __float_as_uint(fmaf(__uint_as_float(sv[i + 2]), p.scale, __uint_as_float(c)));
-                    sv[i + 3] = __float_as_uint(fmaf(__uint_as_float(sv[i + 3]), p.scale, __uint_as_float(d)));
+                    sv[i] = __float_as_uint(fmaf(__uint_as_float(sv[i]), tile_scale, __uint_as_float(a)));
+                    sv[i + 1] = __float_as_uint(fmaf(__uint_as_float(sv[i + 1]), tile_scale, __uint_as_float(b2)));
+                    sv[i + 2] = __float_as_uint(fmaf(__uint_as_float(sv[i + 2]), tile_scale, __uint_as_float(c)));
+                    sv[i + 3] = __float_as_uint(fmaf(__uint_as_float(sv[i + 3]), tile_scale, __uint_as_float(d)));
                 }
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(mask_empty + 8 * sm_);
@@ -477,11 +488,14 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
 #pragma unroll
         for (int i = 0; i < D; ++i) o[i] = 0.f;
         bool ok = run;
+        const int f0 = kvh * ((p.Sk + BN - 1) / BN);
         for (int j = 0; j < nt && ok; ++j) {
             const int a = j & 1;
+            const float beta = p.vf[f0 + j];             // asked for before the waits
             ok = ptx::mbar_wait(alpha_full + 8 * (j & 3), (uint32_t)(j >> 2) & 1u, abort_flag);
             if (!ok) break;
             const float alpha = alpha_s[(j & 3) * BM + r];
+            const float2 alpha2 = make_float2(alpha, alpha), beta2 = make_float2(beta, beta);
             ok = ptx::mbar_wait(pv_done + 8 * a, (uint32_t)(j >> 1) & 1u, abort_flag);
             if (!ok) break;
             ptx::tc_fence_after_sync();
@@ -494,7 +508,11 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                 ptx::tmem_wait_ld();
                 ptx::reg_fence32(t);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) o[c * 32 + i] = fmaf(o[c * 32 + i], alpha, __uint_as_float(t[i]));
+                for (int i = 0; i < 32; i += 2) {
+                    const float2 pv = __fmul2_rn(make_float2(__uint_as_float(t[i]), __uint_as_float(t[i + 1])), beta2);
+                    const float2 y = __ffma2_rn(make_float2(o[c * 32 + i], o[c * 32 + i + 1]), alpha2, pv);
+                    o[c * 32 + i] = y.x; o[c * 32 + i + 1] = y.y;
+                }
             }
             ptx::tc_fence_before_sync();
             __syncwarp();
@@ -567,85 +585,88 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
     }
 }
 
-// The split pass: hi = rn_fp16(x), lo = rn_fp16(x - hi) for up to three tensors in one launch, rows padded with zeros
-// to a multiple of 8, and the range check that decides between the tensor-core kernel above and the exact one (any
-// |x| >= 2^15, a value that is not finite, or only small values of V: x3_declines).
+// The split pass: hi = rn_fp16(2^e x), lo = rn_fp16(2^e x - hi) of Q, K and V in one launch, rows padded with zeros to a
+// multiple of 8, the factors 2^-e, and the words that decide between the tensor-core kernel above and the exact one.
+// Bound: HBM.  One CTA takes 64 rows of Q (a factor each) or a 64-key tile of K or V, all of it in registers between the
+// maximum and the scaling.  Four lanes share a row, each with every fourth group of eight elements: a row's maximum is two
+// shuffles away, and a CTA is small enough for the whole launch to be one wave (with 8, 16 or 32 lanes a row, up to eight
+// rows a thread, B2 H8 S1000 d80 took 11.5 us and B4 H16 S1024 d64 23; now 7.2 and 16.1).
 struct SplitSeg {
     const float *x;
     __half *hi, *lo;
-    long long n4;             // quads of the padded copy
-    int q4, p4;               // quads of a row: source, padded copy
+    float *factor;            // Q: [rows], K and V: [tiles]
+    long long S;              // rows of a slab, cut into `tiles` tiles (Q: all rows are one slab)
+    int tiles, first;         // `first`: CTAs of the segments before this one
+    int q4, p8;               // a row: quads of the source, groups of eight of the padded copy
 };
 struct SplitParams {
     SplitSeg seg[3];          // Q, K, V
-    int *range;
+    int *range;               // three words, zero
 };
 
-// hi and lo halves of four values
-__device__ __forceinline__ void split_quad(float4 v, uint2 &hh, uint2 &ll)
-{
-    const __half2 h01 = __floats2half2_rn(v.x, v.y), h23 = __floats2half2_rn(v.z, v.w);
-    const float2 b01 = __half22float2(h01), b23 = __half22float2(h23);
-    const __half2 l01 = __floats2half2_rn(v.x - b01.x, v.y - b01.y), l23 = __floats2half2_rn(v.z - b23.x, v.w - b23.y);
-    hh.x = *reinterpret_cast<const uint32_t *>(&h01);
-    hh.y = *reinterpret_cast<const uint32_t *>(&h23);
-    ll.x = *reinterpret_cast<const uint32_t *>(&l01);
-    ll.y = *reinterpret_cast<const uint32_t *>(&l23);
-}
-// !(|x| < 2^15) is also true for NaN
-__device__ __forceinline__ bool quad_too_large(float4 v)
-{
-    return !(fabsf(v.x) < 32768.f) || !(fabsf(v.y) < 32768.f) || !(fabsf(v.z) < 32768.f) || !(fabsf(v.w) < 32768.f);
-}
-__device__ __forceinline__ float quad_max(float4 v) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))); }
-
-__global__ void __launch_bounds__(256) split_f32_hi_lo_kernel(const SplitParams sp)
+template <int N>              // groups of eight a lane, 4 N at least p8
+__global__ void __launch_bounds__(256, N <= 2 ? 8 : 5) split_f32_hi_lo_kernel(const SplitParams sp)
 {
     ptx::grid_trigger();
-    bool bad = false;
-    float vmax = 0.f;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const long long n = max(sp.seg[0].n4, max(sp.seg[1].n4, sp.seg[2].n4));
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        // the three tensors' quads are requested together: a thread has one or two of each, and one tensor after the other
-        // waits for memory three times (B2 H8 S1000 d80: 8.6 -> 7.4 us)
-        float4 x[3];
+    constexpr int kInf = 0x7f800000;
+    __shared__ int warp_max[8], warp_min[8];
+    const int t = (int)blockIdx.x >= sp.seg[2].first ? 2 : ((int)blockIdx.x >= sp.seg[1].first ? 1 : 0);
+    const SplitSeg &s = sp.seg[t];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane & 3, row = warp * 8 + (lane >> 2);
+    const int tile = (int)blockIdx.x - s.first, slab = tile / s.tiles;
+    const long long r0 = (long long)(tile - slab * s.tiles) * X3_TILE, at = (long long)slab * s.S + r0 + row;
+    const bool in = r0 + row < s.S;
+    const float4 *src = reinterpret_cast<const float4 *>(s.x) + at * s.q4;
+    ptx::grid_wait();                                                            // where the tensors come from the launch before
+    float4 x[2 * N];
 #pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            const SplitSeg &s = sp.seg[t];
-            x[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i >= s.n4) continue;
-            if (s.q4 == s.p4) {
-                x[t] = reinterpret_cast<const float4 *>(s.x)[i];
-            } else {
-                const long long row = i / s.p4;
-                const int c = (int)(i - row * s.p4);
-                if (c < s.q4) x[t] = reinterpret_cast<const float4 *>(s.x)[row * s.q4 + c];
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            const SplitSeg &s = sp.seg[t];
-            if (i >= s.n4) continue;
-            uint2 hh, ll;
-            split_quad(x[t], hh, ll);
-            reinterpret_cast<uint2 *>(s.hi)[i] = hh;
-            reinterpret_cast<uint2 *>(s.lo)[i] = ll;
-            bad |= quad_too_large(x[t]);
-            if (t == 2) vmax = fmaxf(vmax, quad_max(x[t]));
-        }
+    for (int i = 0; i < 2 * N; ++i) {
+        const int c = ((i >> 1) * 4 + part) * 2 + (i & 1);
+        x[i] = in && c < s.q4 ? src[c] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    // one atomic per CTA and word; none for a maximum that is large enough already
-    const int wmax = __reduce_max_sync(0xffffffffu, __float_as_int(vmax));
-    __shared__ int cta_max, cta_bad;
-    if (threadIdx.x == 0) { cta_max = 0; cta_bad = 0; }
+    // the largest magnitude of the row and of the tile, as bits: integers order as the floats do, NaN above everything
+    int m = 0;
+#pragma unroll
+    for (int i = 0; i < 2 * N; ++i)
+        m = max(m, max(max(__float_as_int(fabsf(x[i].x)), __float_as_int(fabsf(x[i].y))), max(__float_as_int(fabsf(x[i].z)), __float_as_int(fabsf(x[i].w)))));
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    int most = __reduce_max_sync(0xffffffffu, m), least = __reduce_min_sync(0xffffffffu, m != 0 ? m : kInf);
+    if (lane == 0) { warp_max[warp] = most; warp_min[warp] = least; }
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) atomicMax(&cta_max, wmax);
-    if (bad) cta_bad = 1;
-    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) { most = max(most, warp_max[w]); least = min(least, warp_min[w]); }
+    // exponent that brings the maximum to [2^13, 2^14); both 2^e and 2^-e are normal floats
+    const int e = min(126, 140 - ((t == 0 ? m : most) >> 23));
+    const float scale = __int_as_float((e + 127) << 23), factor = __int_as_float((127 - e) << 23);
     if (threadIdx.x == 0) {
-        if (cta_bad) atomicOr(sp.range, 1);
-        if (cta_max > *reinterpret_cast<volatile int *>(sp.range + 1)) atomicMax(sp.range + 1, cta_max);
+        if (most >= kInf || (t == 2 && most != 0 && (most >> 23) - (least >> 23) > 13)) atomicOr(sp.range, 1);
+        if (t == 0) atomicMax(sp.range + 1, most);
+        if (t == 1) atomicMax(sp.range + 2, most);
+        if (t > 0) s.factor[tile] = factor;
+    }
+    if (!in) return;
+    if (t == 0 && part == 0) s.factor[at] = factor;
+    uint4 *hi = reinterpret_cast<uint4 *>(s.hi) + at * s.p8, *lo = reinterpret_cast<uint4 *>(s.lo) + at * s.p8;
+    auto halves = [&](float a, float b, uint32_t &h, uint32_t &l) {
+        a *= scale; b *= scale;
+        const __half2 hh = __floats2half2_rn(a, b);
+        const float2 back = __half22float2(hh);
+        const __half2 ll = __floats2half2_rn(a - back.x, b - back.y);
+        h = *reinterpret_cast<const uint32_t *>(&hh);
+        l = *reinterpret_cast<const uint32_t *>(&ll);
+    };
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int c = i * 4 + part;
+        if (c >= s.p8) continue;
+        uint4 h, l;
+        halves(x[2 * i].x, x[2 * i].y, h.x, l.x);
+        halves(x[2 * i].z, x[2 * i].w, h.y, l.y);
+        halves(x[2 * i + 1].x, x[2 * i + 1].y, h.z, l.z);
+        halves(x[2 * i + 1].z, x[2 * i + 1].w, h.w, l.w);
+        hi[c] = h;
+        lo[c] = l;
     }
 }
 
