@@ -371,10 +371,15 @@ int launch_simt_t(const txb::SimtParams &p, cudaStream_t st)
     if (p.only_if) {
         // a stand-in that nearly always has nothing to do: one wave of CTAs that walk the items if they must (a CTA
         // each took 6.7 us to find that out at 2048 items)
-        int sms = 0;
+        static std::atomic<int> fit{0};
+        int sms = 0, per_sm = fit.load(std::memory_order_relaxed);
         if (int rc = sm_count(&sms)) return rc;
-        grid.y = std::min<unsigned>(grid.y, (unsigned)sms);
-        grid.z = std::min<unsigned>(grid.z, std::max(1u, (unsigned)sms / grid.y));
+        if (per_sm == 0) {
+            TX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, txb::sdpa_simt_kernel<T, DVC, PROF>, txb::SIMT_THREADS, 0));
+            fit.store(per_sm = std::max(per_sm, 1), std::memory_order_relaxed);
+        }
+        const int64_t items = (int64_t)grid.x * grid.y * grid.z;
+        grid = dim3((unsigned)std::min<int64_t>(items, (int64_t)sms * per_sm));
         return launch_behind(txb::sdpa_simt_kernel<T, DVC, PROF>, grid, txb::SIMT_THREADS, 0, st, 1, p);
     }
     txb::sdpa_simt_kernel<T, DVC, PROF><<<grid, txb::SIMT_THREADS, 0, st>>>(p);

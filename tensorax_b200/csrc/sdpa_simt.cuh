@@ -91,13 +91,16 @@ sdpa_simt_kernel(const SimtParams p)
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    // one (batch, head) and row block per CTA, more only where the launch was given fewer CTAs than items
-    for (int64_t bh = blockIdx.z; bh < p.B * p.Hq; bh += gridDim.z)        // b*Hq + h
-    for (int64_t q0 = (int64_t)blockIdx.y * SIMT_BR; q0 < p.Sq; q0 += (int64_t)gridDim.y * SIMT_BR) {
+    // one column block, row block and (batch, head) per CTA, more only where the launch has fewer CTAs than items
+    const int64_t col_blocks = (p.dv + 32 * DVC - 1) / (32 * DVC), row_blocks = (p.Sq + SIMT_BR - 1) / SIMT_BR;
+    const int64_t n_items = col_blocks * row_blocks * p.B * p.Hq, n_ctas = (int64_t)gridDim.x * gridDim.y * gridDim.z;
+    for (int64_t item = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x; item < n_items; item += n_ctas) {
+    const int64_t bh = item / (col_blocks * row_blocks);                   // b*Hq + h
+    const int64_t q0 = item / col_blocks % row_blocks * SIMT_BR;
     const int64_t b = bh / p.Hq;
     const int64_t h = bh % p.Hq;
     const int64_t kvh = b * p.Hkv + h / (p.Hq / p.Hkv);
-    const int64_t dv0 = (int64_t)blockIdx.x * (32 * DVC);
+    const int64_t dv0 = item % col_blocks * (32 * DVC);
 
     const T *Q = static_cast<const T *>(p.q) + bh * p.Sq * p.dk;
     const T *K = static_cast<const T *>(p.k) + kvh * p.Sk * p.dk;

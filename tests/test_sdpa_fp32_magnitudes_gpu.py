@@ -1,8 +1,11 @@
 """The fp32 tensor-core path on operands of unequal magnitude.  The fp16 pairs are scaled by powers of two per row of Q and per
 64-key tile of K and V, so that (a) a power of two taken out of a tensor leaves every bit of the result alone, and (b) small
 numbers beside large ones keep fp32-grade precision; what scaling cannot hold goes to the exact kernel.  Reference: float64."""
+import ctypes
+
 import numpy as np
 import pytest
+import torch
 
 import oracle
 from conftest import assert_close_fp32, seeded
@@ -111,3 +114,33 @@ def test_factors_follow_grouped_heads_lengths_and_partial_tiles(Hq, Hkv, Sk):
     ref = oracle.sdpa_structured(q, k, v, causal=True, kv_lens=lens)
     for h in range(Hq):
         assert np.abs(got[:, h] - ref[:, h]).max() <= 1e-5 * 10.0 ** (h // (Hq // Hkv)) * 4
+
+
+@pytest.mark.parametrize("shape,causal", [((2, 16, 1600, 128), True), ((1, 3, 2400, 64), False)])
+def test_a_declined_call_costs_what_the_exact_kernel_costs(shape, causal):
+    """The stand-in behind the tensor-core kernel uses the whole chip when it has to work: at most half as much again as
+    the exact kernel by itself, split pass included (best of five each; it was four times at the first shape)."""
+    B, H, S, d = shape
+    lib = _lib.load()
+    q, k, v = (torch.randn(shape, device="cuda") for _ in range(3))
+    v[0, 0, 0] *= 1e-6
+    out = torch.zeros(shape, device="cuda")
+
+    def best(flags):
+        desc = _lib.SdpaDesc(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), mask=None, kv_lens=None, out=out.data_ptr(), batch=B,
+                             q_heads=H, kv_heads=H, seq_q=S, seq_k=S, d_k=d, d_v=d, dtype=_lib.TX_DTYPE_F32, causal=int(causal),
+                             flags=flags, stream=None, lse=None)
+        times = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            _lib.check(lib.tx_sdpa_forward(ctypes.byref(desc)))
+            b.record()
+            _lib.check(lib.tx_sdpa_finish(None))
+            times.append(a.elapsed_time(b))
+        return min(times[1:]), out.clone()
+
+    exact, ref = best(_lib.TX_SDPA_FORCE_SIMT)
+    declined, got = best(0)
+    assert torch.equal(got, ref)
+    assert declined <= 1.5 * exact, (declined, exact)
