@@ -124,14 +124,15 @@ class MultiHeadAttention:
         from ... import _C
         P = self._parameters
 
-        names = ("q", "k", "v", "out")
-        whole = _C.multi_head_attention(
-            query._c_tensor, key._c_tensor, value._c_tensor, [P[n + "_weight"]._c_tensor for n in names],
-            [P[n + "_bias"]._c_tensor if P[n + "_bias"] is not None else None for n in names], self.num_heads,
-            mask._c_tensor if mask is not None else None, causal=causal, kv_lens=kv_lens,
-            fp16_attention=self.attention_dtype == "float16")
-        if whole is not None:
-            return Tensor._wrap(whole)
+        if getattr(self.attend, "__func__", None) is _ATTEND:      # an attend of somebody else's is called, below
+            names = ("q", "k", "v", "out")
+            whole = _C.multi_head_attention(
+                query._c_tensor, key._c_tensor, value._c_tensor, [P[n + "_weight"]._c_tensor for n in names],
+                [P[n + "_bias"]._c_tensor if P[n + "_bias"] is not None else None for n in names], self.num_heads,
+                mask._c_tensor if mask is not None else None, causal=causal, kv_lens=kv_lens,
+                fp16_attention=self.attention_dtype == "float16")
+            if whole is not None:
+                return Tensor._wrap(whole)
 
         def project(x, w, b):
             return Tensor._wrap(_C.linear(x._c_tensor, P[w]._c_tensor,
@@ -156,3 +157,6 @@ class MultiHeadAttention:
     def __repr__(self) -> str:
         return (f"MultiHeadAttention(embed_dim={self.embed_dim}, num_heads={self.num_heads}, "
                 f"head_dim={self.head_dim}, dropout={self.dropout})")
+
+
+_ATTEND = MultiHeadAttention.attend

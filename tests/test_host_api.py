@@ -202,3 +202,36 @@ def test_header_is_plain_c_and_links_from_a_c_program(tmp_path):
                     "-L", libdir, "-ltensorax_b200", "-Wl,-rpath," + libdir, "-o", str(exe)], check=True)
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
     assert out == ["1", "1", "1", str(ctypes.sizeof(_lib.SdpaDesc))]
+
+
+def test_layer_calls_an_attend_that_is_not_its_own(monkeypatch):
+    """MultiHeadAttention.forward may run as one library call, but not past an `attend` that a subclass, an instance or a
+    patch of the class has put in its place."""
+    import tensorax_b200 as ts
+    from tensorax_b200 import _C
+    from tensorax_b200.nn.attention import MultiHeadAttention
+
+    whole, seen = [], []
+    x = ts.Tensor(np.zeros((1, 4, 8), np.float32))
+    monkeypatch.setattr(_C, "multi_head_attention", lambda *a, **k: whole.append(1) or x._c_tensor)
+    monkeypatch.setattr(_C, "linear", lambda t, *a, **k: t)
+
+    def attend(self, q, k, v, mask=None, causal=False, kv_lens=None):
+        seen.append(causal)
+        return q
+
+    class Mine(MultiHeadAttention):
+        pass
+
+    Mine(8, 2)(x, x, x)
+    assert len(whole) == 1 and not seen
+    Mine.attend = attend
+    Mine(8, 2)(x, x, x, causal=True)
+    assert len(whole) == 1 and seen == [True]
+    one = MultiHeadAttention(8, 2)
+    one.attend = attend.__get__(one)
+    one(x, x, x)
+    assert len(whole) == 1 and len(seen) == 2
+    monkeypatch.setattr(MultiHeadAttention, "attend", attend)
+    MultiHeadAttention(8, 2)(x, x, x)
+    assert len(whole) == 1 and len(seen) == 3
