@@ -757,7 +757,7 @@ int forward_f32_via_f16(const tx_sdpa_desc *d, cudaStream_t st)
         h.dtype = TX_DTYPE_F16;
         int *status = nullptr;
         rc = status_word(&status);
-        if (rc == TX_OK) rc = launch_tc(&h, st, status);
+        if (rc == TX_OK) rc = launch_f16(&h, st, status);
     }
     pool_free(ws, st);
     return rc;
@@ -887,15 +887,15 @@ int launch_x3(const tx_sdpa_desc *d, cudaStream_t st, int *status, int *zeroed =
 int forward_launch(const tx_sdpa_desc *d)
 {
     cudaStream_t st = static_cast<cudaStream_t>(d->stream);
+    if (d->dtype == TX_DTYPE_F32 && (d->flags & TX_SDPA_F32_VIA_F16)) {
+        tx_sdpa_desc probe = *d;
+        probe.dtype = TX_DTYPE_F16;                 // does the fp16 path take this call?
+        if (tc_eligible(&probe)) return forward_f32_via_f16(d, st);
+    }
     if (decode_eligible(d)) {
         int *status = nullptr;
         if (int rc = status_word(&status)) return rc;
         return d->dtype == TX_DTYPE_F16 ? launch_decode<__half>(d, st, status) : launch_decode<float>(d, st, status);
-    }
-    if (d->dtype == TX_DTYPE_F32 && (d->flags & TX_SDPA_F32_VIA_F16)) {
-        tx_sdpa_desc probe = *d;
-        probe.dtype = TX_DTYPE_F16;                 // would the fp16 form of this call run on the tensor cores?
-        if (tc_eligible(&probe)) return forward_f32_via_f16(d, st);
     }
     if (tc_eligible(d)) {
         int *status = nullptr;

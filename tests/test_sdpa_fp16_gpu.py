@@ -350,3 +350,12 @@ def test_fp32_tensors_on_the_tensor_cores_by_request():
     q2, k2, v2 = (seeded(i, 1, 2, 50, 40) for i in (133, 134, 135))
     got, _ = sdpa_device(q2, k2, v2, flags=_lib.TX_SDPA_F32_VIA_F16)
     assert_close_fp32(got, oracle.sdpa_f32(q2, k2, v2))
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk", [(2, 4, 2, 1, 300), (1, 8, 1, 2, 700), (1, 2, 2, 128, 128), (1, 1, 1, 20, 40)])
+def test_fp32_tensors_by_request_with_few_rows(B, Hq, Hkv, Sq, Sk):
+    """The same equality for calls that without the flag go to the decoding kernel in fp32."""
+    q, k, v = seeded(140, B, Hq, Sq, 64), seeded(141, B, Hkv, Sk, 64), seeded(142, B, Hkv, Sk, 64)
+    via, _ = sdpa_device(q, k, v, flags=_lib.TX_SDPA_F32_VIA_F16)
+    direct, _ = sdpa_device(*(x.astype(np.float16) for x in (q, k, v)))
+    assert np.array_equal(via.view(np.uint32), direct.view(np.uint32))
