@@ -205,11 +205,10 @@ TX_API int tx_sdpa_forward(const tx_sdpa_desc *desc);
  * per device and stays set until a tx_sdpa_finish call on that device reports and clears it; launches issued in
  * between return at once and write NaN. */
 TX_API int tx_sdpa_finish(void *stream);
-/* 1 if tx_sdpa_forward would run `desc` on a tcgen05 kernel (fp16, or fp32 as hi/lo fp16 pairs), 0 if on CUDA cores.
- * (For fp32 the answer is about the shape: a value outside the pairs' range still sends the call to CUDA cores; and it is 1
- * for the unmasked head dims 64 and 128 only, although masked calls and the head dims between run on the same kernel.)
- * Likewise calls with few query rows per K/V head -- decoding steps, up to 16 rows in fp16 and 32 in fp32 -- and small fp32
- * calls run on a kernel of their own, on fp32 FMAs, whatever the answer for their shape. */
+/* 1 if tx_sdpa_forward runs `desc` on a tcgen05 kernel (fp16, or fp32 as hi/lo fp16 pairs), 0 if on CUDA cores: calls
+ * with few query rows per K/V head -- decoding steps, up to 16 rows in fp16 and 32 in fp32 -- and small fp32 calls, which the
+ * decoding kernel takes, and what only the exact kernel takes.  (For fp32 the answer is about the shape: values that pairs
+ * cannot carry still send the call to CUDA cores.) */
 TX_API int tx_sdpa_uses_tensor_cores(const tx_sdpa_desc *desc);
 /* How many kernels of this library have been launched by this process so far. */
 TX_API int64_t tx_kernel_launch_count(void);

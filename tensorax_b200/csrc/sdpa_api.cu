@@ -569,7 +569,8 @@ int launch_tc(const tx_sdpa_desc *d, cudaStream_t st, int *status, long long *pr
 // because the tensor-core form first writes and reads back hi / lo copies of the whole cache.
 // Small fp32 calls go there too: one launch without a workspace against three and a memset.  Up to 2^23 products (B1 H2
 // S128 d64 44 -> 31 us a call, B1 H8 S128 d64 38 -> 28, B4 H8 S64 d64 37 -> 33; at 2^24 products and 1024 row groups it
-// was 37 against 43) or up to two query rows per SM in all (B1 H4 Sq64 Sk2048 d128 84 -> 42: four CTAs' work otherwise).
+// was 37 against 43) or up to two query rows per SM in all (B1 H4 Sq64 Sk2048 d128 84 -> 42: four CTAs' work otherwise;
+// 148 SMs where there is no device to ask).
 bool decode_eligible(const tx_sdpa_desc *d)
 {
     if (d->flags & (TX_SDPA_FORCE_SIMT | TX_SDPA_P_IN_SMEM)) return false;
@@ -578,8 +579,10 @@ bool decode_eligible(const tx_sdpa_desc *d)
     if (!al(d->q) || !al(d->k) || !al(d->v)) return false;
     const int64_t rows = d->q_heads / d->kv_heads * d->seq_q;
     if (d->dtype == TX_DTYPE_F16) return rows <= 16 && d->seq_k >= 128;
+    int sms = 0;
+    if (sm_count(&sms) != TX_OK) sms = 148;
     const double all_rows = (double)(d->batch * d->kv_heads * rows);
-    return rows <= 32 || all_rows <= 296 || all_rows * (double)d->seq_k * (double)d->d_k <= 8388608.0;
+    return rows <= 32 || all_rows <= 2.0 * sms || all_rows * (double)d->seq_k * (double)d->d_k <= 8388608.0;
 }
 
 template <class Cfg>
@@ -884,32 +887,39 @@ int launch_x3(const tx_sdpa_desc *d, cudaStream_t st, int *status, int *zeroed =
     return narrow ? on(txb::X3Cfg<64, 4>{}) : on(txb::X3Cfg<128, 2>{});
 }
 
+// Which kernel takes a (valid) call.
+enum class Route { Decode, TensorCores, Pairs, CudaCores };
+Route route_of(const tx_sdpa_desc *d)
+{
+    if (decode_eligible(d)) return Route::Decode;
+    if (tc_eligible(d)) return Route::TensorCores;
+    return x3_eligible(d) ? Route::Pairs : Route::CudaCores;
+}
+
+// fp32 tensors to be rounded to fp16 first: the call as the fp16 path gets it, if it takes it
+bool via_f16(const tx_sdpa_desc *d, tx_sdpa_desc *h)
+{
+    if (d->dtype != TX_DTYPE_F32 || !(d->flags & TX_SDPA_F32_VIA_F16)) return false;
+    *h = *d;
+    h->dtype = TX_DTYPE_F16;
+    return tc_eligible(h);
+}
+
 int forward_launch(const tx_sdpa_desc *d)
 {
     cudaStream_t st = static_cast<cudaStream_t>(d->stream);
-    if (d->dtype == TX_DTYPE_F32 && (d->flags & TX_SDPA_F32_VIA_F16)) {
-        tx_sdpa_desc probe = *d;
-        probe.dtype = TX_DTYPE_F16;                 // does the fp16 path take this call?
-        if (tc_eligible(&probe)) return forward_f32_via_f16(d, st);
+    tx_sdpa_desc h;
+    if (via_f16(d, &h)) return forward_f32_via_f16(d, st);
+    const Route route = route_of(d);
+    if (route == Route::CudaCores) {
+        txb::SimtParams p;
+        fill_simt_params(&p, d);
+        return d->dtype == TX_DTYPE_F16 ? launch_simt<__half>(p, st) : launch_simt<float>(p, st);
     }
-    if (decode_eligible(d)) {
-        int *status = nullptr;
-        if (int rc = status_word(&status)) return rc;
-        return d->dtype == TX_DTYPE_F16 ? launch_decode<__half>(d, st, status) : launch_decode<float>(d, st, status);
-    }
-    if (tc_eligible(d)) {
-        int *status = nullptr;
-        if (int rc = status_word(&status)) return rc;
-        return launch_tc(d, st, status);
-    }
-    if (x3_eligible(d)) {
-        int *status = nullptr;
-        if (int rc = status_word(&status)) return rc;
-        return launch_x3(d, st, status);
-    }
-    txb::SimtParams p;
-    fill_simt_params(&p, d);
-    return d->dtype == TX_DTYPE_F16 ? launch_simt<__half>(p, st) : launch_simt<float>(p, st);
+    int *status = nullptr;
+    if (int rc = status_word(&status)) return rc;
+    if (route == Route::Decode) return d->dtype == TX_DTYPE_F16 ? launch_decode<__half>(d, st, status) : launch_decode<float>(d, st, status);
+    return route == Route::TensorCores ? launch_tc(d, st, status) : launch_x3(d, st, status);
 }
 
 int forward(const tx_sdpa_desc *d)
@@ -1744,14 +1754,9 @@ int tx_sdpa_finish(void *stream) { return finish(static_cast<cudaStream_t>(strea
 int tx_sdpa_uses_tensor_cores(const tx_sdpa_desc *desc)
 {
     if (validate(desc) != TX_OK) return 0;
-    if (desc->dtype == TX_DTYPE_F32 && (desc->flags & TX_SDPA_F32_VIA_F16)) {
-        tx_sdpa_desc probe = *desc;
-        probe.dtype = TX_DTYPE_F16;
-        return tc_eligible(&probe) ? 1 : 0;
-    }
-    if (tc_eligible(desc)) return 1;
-    const bool plain = !desc->mask && desc->d_k == desc->d_v && (desc->d_k == 64 || desc->d_k == 128);
-    return (plain && x3_eligible(desc)) ? 1 : 0;
+    tx_sdpa_desc h;
+    const Route route = route_of(via_f16(desc, &h) ? &h : desc);
+    return route == Route::TensorCores || route == Route::Pairs ? 1 : 0;
 }
 
 int64_t tx_kernel_launch_count(void) { return g_launches.load(); }

@@ -46,7 +46,7 @@ def test_config1_every_fp32_entry_point(golden, name):
 def test_hand_written_cases(golden, case):
     q, k, v = (golden[f"hand_{case}_{t}"] for t in "qkv")
     got, tc = sdpa_device(q, k, v)
-    assert not tc
+    assert tc == (q.shape[3] % 4 == 0 and v.shape[3] % 4 == 0)      # as fp16 pairs, or on CUDA cores
     assert_close_fp32(got, golden[f"hand_{case}_out"])
 
 

@@ -18,11 +18,11 @@ CASES = [
     # B, Hq, Hkv, Sq, Sk, causal, kv_lens
     (1, 2, 2, 300, 300, True, None),
     (2, 4, 2, 320, 320, True, [320, 133]),
-    (1, 1, 1, 128, 128, False, None),
-    (1, 1, 1, 129, 129, True, None),
+    (3, 3, 3, 128, 128, False, None),              # one tile; as many heads as keep it off the decoding kernel
+    (3, 3, 3, 129, 129, True, None),
     (1, 2, 1, 200, 700, False, None),
     (2, 2, 2, 256, 256, False, [0, 256]),          # batch 0 sees no key: NaN rows, as the reference
-    (1, 1, 1, 100, 900, True, None),
+    (2, 2, 2, 100, 900, True, None),
     (2, 100, 100, 257, 257, False, [257, 77]),     # more work items than SMs
 ]
 
@@ -95,10 +95,15 @@ def test_launches_and_shape_rule():
     assert tc and lib.tx_kernel_launch_count() - n0 == 3            # split pass, tensor-core kernel, stand-in
     m = np.zeros((1, 2, 256, 256), np.float32)
     _, tc_mask = sdpa_device(q, k, v, mask=m)
-    assert not tc_mask                                              # dense masks stay on the exact kernel
+    assert tc_mask and lib.tx_kernel_launch_count() - n0 == 6       # dense masks take the same three
     q32 = seeded(24, 1, 2, 256, 32)
     _, tc_small = sdpa_device(q32, q32, q32)
-    assert not tc_small
+    assert tc_small                                                 # and so does every head dim up to 128 in steps of 4
+    for q, k in ((seeded(25, 1, 2, 256, 132), seeded(26, 1, 2, 256, 132)), (seeded(25, 1, 2, 256, 30), seeded(26, 1, 2, 256, 30)),
+                 (seeded(25, 2, 4, 1, 64), seeded(26, 2, 4, 700, 64)), (seeded(25, 1, 2, 128, 64), seeded(26, 1, 2, 128, 64))):
+        n0 = lib.tx_kernel_launch_count()
+        _, tc = sdpa_device(q, k, k)                                # other head dims: exact kernel; few rows, small calls: decoding
+        assert not tc and lib.tx_kernel_launch_count() - n0 == 1
 
 
 def test_five_reference_names_share_the_path():

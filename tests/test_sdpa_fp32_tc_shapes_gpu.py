@@ -16,7 +16,8 @@ def test_partly_filled_panels(dk, dv, Sq, Sk, causal):
     B, Hq, Hkv = 2, 4, 2
     q, k, v = seeded(1, B, Hq, Sq, dk), seeded(2, B, Hkv, Sk, dk), seeded(3, B, Hkv, Sk, dv)
     lens = [Sk, Sk - 70]
-    outs, _ = sdpa_device(q, k, v, causal=causal, kv_lens=lens, repeats=2)
+    outs, tc = sdpa_device(q, k, v, causal=causal, kv_lens=lens, repeats=2)
+    assert tc
     assert np.array_equal(outs[0], outs[1])
     assert_close_fp32(outs[0], oracle.sdpa_structured(q, k, v, causal=causal, kv_lens=lens))
 
@@ -25,7 +26,7 @@ def test_partly_filled_panels(dk, dv, Sq, Sk, causal):
 @pytest.mark.parametrize("Sq,Sk", [(128, 64), (130, 260), (257, 323), (64, 1001)])     # rows of the mask 16-byte aligned and not
 @pytest.mark.parametrize("kind", ["causal", "random", "rows"])
 def test_dense_masks(d, Sq, Sk, kind):
-    B, H = 2, 3
+    B, H = 4, 6                                          # enough rows for none to go to the decoding kernel
     q, k, v = seeded(11, B, H, Sq, d), seeded(12, B, H, Sk, d), seeded(13, B, H, Sk, d)
     if kind == "causal":
         m = np.where(np.arange(Sk)[None, :] <= np.arange(Sq)[:, None], 0.0, -np.inf)
@@ -37,7 +38,8 @@ def test_dense_masks(d, Sq, Sk, kind):
             m[:, 1, Sq - 1] = np.finfo(np.float32).min   # uniform average
             m[0, 0, 5, : Sk // 2] = -1e9
     m = np.ascontiguousarray(m, dtype=np.float32)
-    got, _ = sdpa_device(q, k, v, mask=m)
+    got, tc = sdpa_device(q, k, v, mask=m)
+    assert tc
     with np.errstate(all="ignore"):
         ref = oracle.sdpa_f32(q, k, v, m)
     assert_close_fp32(got, ref)
