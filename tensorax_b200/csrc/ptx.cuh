@@ -11,6 +11,7 @@
 #include "kv_lens.cuh"
 
 #include "bounded_wait.h"
+#include "status_report.h"
 
 namespace txb {
 namespace ptx {
@@ -96,18 +97,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
                         [] { return global_timer_ns(); }, abort_flag, limit_ns);
 }
 
-// Record that a wait ran out: the first code stays in the device status word (asked by the launch's later CTAs), and
-// whoever set it also writes it to the host's mirror, whose device address is kept 8 bytes behind the word (null: none).
-// The mirror is what lets the host learn of a failure after a synchronise without a copy from the device.
+// Record that a wait ran out (status_report.h).  The device address of the host's mirror is kept 8 bytes behind the status
+// word (null: none); with it the host learns of a failure after a synchronise without a copy from the device.
 __device__ __forceinline__ void report(int *status, int code)
 {
-    if (atomicCAS(status, 0, code) == 0) {
-        volatile int *mirror = *reinterpret_cast<volatile int *volatile *>(status + 2);
-        if (mirror) {
-            *mirror = code;
-            __threadfence_system();
-        }
-    }
+    make_report([&](int c) { return atomicCAS(status, 0, c); },
+                [&](int c) {
+                    volatile int *mirror = *reinterpret_cast<volatile int *volatile *>(status + 2);
+                    if (mirror) {
+                        *mirror = c;
+                        __threadfence_system();
+                    }
+                },
+                code);
 }
 
 // ---------------------------------------------------------------- fences

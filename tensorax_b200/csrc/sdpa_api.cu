@@ -934,12 +934,14 @@ int finish(cudaStream_t st)
     TX_CUDA(cudaStreamSynchronize(st));
     int dev = 0;
     if (int rc = current_device(&dev)) return rc;
-    if (g_status_ready[dev].load(std::memory_order_acquire) && *g_status[dev].mirror != 0) {
-        const int code = *g_status[dev].mirror;
-        (void)cudaMemset(g_status[dev].word, 0, sizeof code);      // the word only: the mirror's address stays
-        *g_status[dev].mirror = 0;
+    if (!g_status_ready[dev].load(std::memory_order_acquire) || *g_status[dev].mirror == 0) return TX_OK;
+    std::lock_guard<std::mutex> lk(g_status_mu);
+    const int code = txb::take_report(
+        [&](int v) { return __atomic_exchange_n(const_cast<int *>(g_status[dev].mirror), v, __ATOMIC_SEQ_CST); },
+        // the word only: the mirror's address stays behind it
+        [&] { return cudaMemset(g_status[dev].word, 0, sizeof(int)) == cudaSuccess && cudaStreamSynchronize(nullptr) == cudaSuccess; });
+    if (code != 0)
         return fail(TX_ERR_KERNEL, "SDPA kernel gave up on a bounded wait (stage code %d); output is not valid", code);
-    }
     return TX_OK;
 }
 
