@@ -282,7 +282,11 @@ gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ 
             const GemmX3Problem &pr = p.prob[problem_of(tile)];
             const int local = tile - pr.first_tile;
             const int row0 = local / pr.tiles_n * BM + quarter * 32, col0 = local % pr.tiles_n * BN + half * HALF;
-            const float inv = row0 + lane < pr.M ? pr.inv_x[row0 + lane] : 0.f;
+            // The result is sum * inv_x * inv_w + bias; the factor below 1 comes first where the other one is above, so that
+            // the product in between is in range whenever the result is (x of 1e36 and weights of 1e-30: sum * inv_x alone
+            // overflowed).  Rows that need inv_x last are rare: a warp without one does nothing more.
+            const float inv_x = row0 + lane < pr.M ? pr.inv_x[row0 + lane] : 0.f, inv = fminf(inv_x, 1.f), inv_last = fmaxf(inv_x, 1.f);
+            const bool any_last = __any_sync(0xffffffffu, inv_x > 1.f);
             const int dh = pr.heads > 0 ? p.N / pr.heads : p.N;
 #pragma unroll
             for (int q = 0; q < HALF / 32; ++q) {
@@ -294,6 +298,10 @@ gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ 
                                       __float_as_uint(sum[q * 32 + i + 2] * inv), __float_as_uint(sum[q * 32 + i + 3] * inv));
                 __syncwarp();
                 const int n = col0 + q * 32 + (lane & 7) * 4;
+                float last[8];                                            // of the rows this lane stores
+                if (any_last)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) last[i] = __shfl_sync(0xffffffffu, inv_last, i * 4 + (lane >> 3));
                 if (n < p.N) {
                     const float4 iw = *reinterpret_cast<const float4 *>(pr.inv_w + n);
                     const float4 bb = pr.bias ? __ldg(reinterpret_cast<const float4 *>(pr.bias + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -304,8 +312,13 @@ gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ 
                         if (m >= pr.M) break;
                         uint32_t x, y, z, w;
                         ptx::ld_shared_v4(turn + (uint32_t)r * 128 + ((uint32_t)((lane & 7) ^ (r & 7)) << 4), x, y, z, w);
-                        const float4 f = make_float4(fmaf(__uint_as_float(x), iw.x, bb.x), fmaf(__uint_as_float(y), iw.y, bb.y),
-                                                     fmaf(__uint_as_float(z), iw.z, bb.z), fmaf(__uint_as_float(w), iw.w, bb.w));
+                        float4 f = make_float4(fmaf(__uint_as_float(x), iw.x, bb.x), fmaf(__uint_as_float(y), iw.y, bb.y),
+                                               fmaf(__uint_as_float(z), iw.z, bb.z), fmaf(__uint_as_float(w), iw.w, bb.w));
+                        if (any_last) {
+                            const float a = last[r4 / 4];
+                            f = make_float4(fmaf(__uint_as_float(x) * iw.x, a, bb.x), fmaf(__uint_as_float(y) * iw.y, a, bb.y),
+                                            fmaf(__uint_as_float(z) * iw.z, a, bb.z), fmaf(__uint_as_float(w) * iw.w, a, bb.w));
+                        }
                         const size_t at = pr.heads > 0 ? (((size_t)(m / pr.S) * pr.heads + h) * pr.S + m % pr.S) * dh + cc
                                                        : (size_t)m * p.N + n;
                         if (p.out_f16) {

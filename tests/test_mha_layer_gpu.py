@@ -83,3 +83,16 @@ def test_halves_written_by_the_projections(E, H, scale):
     got = mha(*(ts.Tensor(t, device="cuda") for t in (x, k, y))).numpy()
     ref = oracle.mha_forward_f32(x, k, y, params, H, None)
     assert np.linalg.norm(got - ref) <= 2e-5 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("a,b", [(36, -30), (-36, 30), (34, -8)])
+def test_products_in_range_of_operands_near_its_ends(a, b):
+    """Inputs of 1e36 and value weights of 1e-30, or the other way round: the projections' results are ordinary numbers."""
+    E, H = 64, 2
+    mha, params = layer(E, H, False)
+    w = (params["v_weight"] * np.float32(10.0) ** b).astype(np.float32)
+    mha._parameters["v_weight"] = ts.Tensor(w, device="cuda")
+    q, x = seeded(12, 2, 5, E), (seeded(13, 2, 1, E) * 10.0 ** a / 8).astype(np.float32)
+    got = mha(ts.Tensor(q, device="cuda"), ts.Tensor(q[:, :1].copy(), device="cuda"), ts.Tensor(x, device="cuda")).numpy()
+    ref = x.astype(np.float64) @ w.astype(np.float64).T @ params["out_weight"].astype(np.float64).T
+    assert np.linalg.norm(got - ref) <= 2e-6 * np.linalg.norm(np.broadcast_to(ref, got.shape))
