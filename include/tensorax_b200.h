@@ -160,7 +160,9 @@ TX_API int tx_linear_set_cuda_cores_only(int on);
 /* ---- multi-head attention layer: the whole of MultiHeadAttention.forward (tensorax/nn/attention/layers.py:105-128) in
  *      fp32 -- x W^T + b for queries, keys and values, attention per head, output projection -- as one stream-ordered
  *      sequence without synchronisation.  Projections run on the fp16 tensor cores with operands as row-scaled hi + lo
- *      pairs and fp32 sums (fp32-grade accuracy at any magnitude); embed must be a multiple of 8, the head dim of 4, pointers
+ *      pairs and fp32 sums: an element keeps 22 bits down to 2^-17 of its row's largest, whatever that is, and 2^-39 of
+ *      it below.  A row of the inputs, weights or attention result in which more than one element in 16 lies below 2^-17
+ *      sends the projections to exact fp32 products on CUDA cores (decided on the device).  embed must be a multiple of 8, the head dim of 4, pointers
  *      16-byte aligned (else TX_ERR_UNSUPPORTED).  Does not synchronise; tx_sdpa_finish reports failures. */
 enum { TX_MHA_F16_ATTENTION = 32 };  /* flag: heads rounded to fp16 for the attention step (as cast_f32_to_f16 of them) */
 typedef struct tx_mha_desc {

@@ -9,7 +9,8 @@
 //
 //   split_rows_kernel   one warp per row of x or W: the row is scaled by a power of two that brings its largest element
 //                       to [2^13, 2^14), then hi = rn16(x), lo = rn16(x - hi).  With the scale a pair is exact to 2^-39
-//                       of the row's maximum and to 22 bits down to 2^-17 of it, whatever the row's magnitude.
+//                       of the row's maximum and to 22 bits down to 2^-17 of it, whatever the row's magnitude.  A row in
+//                       which more than one element in 16 lies below that (an outlier and little else) raises a flag.
 //   gemm_x3_kernel      persistent, one CTA per SM, 128 x BN tiles.  The tensor core's fp32 accumulation truncates, so a
 //                       tensor-memory accumulator takes two stages (K = 128) only, a stage's small products first, so
 //                       that few of its 24 MMAs add at full magnitude; two accumulators ping-pong and two warpgroups
@@ -17,11 +18,13 @@
 //                       warp 0 TMA producer, warp 1 MMA issuer, warps 4-7 / 8-11 sums and results of the left / right
 //                       half of a tile's columns (thread = row); results are turned through shared memory so that a
 //                       warp stores whole 128-byte pieces of rows, head-split, fp32 or fp16.
+//                       With the flag raised the CTA computes its tiles from the fp32 operands on CUDA cores instead.
 // Bound: L2 -> SM traffic (a 128 x 256 tile brings 96 KB per 64 k, 128 FLOP per byte) next to the tensor pipe.  Measured, B4
 // S1024 E1024 (three projections, then the output's): 94 us together = 1.1 PFLOP/s of fp16 MMAs; folding after every stage
 // 103 us, after four 93; CTA pairs on 256 x 256 tiles (cta_group::2, 64 KB per 64 k and SM) 95 us, 128 x 128 tiles 99 us.
 // Every mbarrier wait is bounded.
 #pragma once
+#include "linear_simt.cuh"
 #include "ptx.cuh"
 
 namespace txb {
@@ -40,6 +43,7 @@ constexpr int kSplitRowsSegs = 7;          // q, k, v inputs and four weights
 struct SplitRowsParams {
     SplitRowsSeg seg[kSplitRowsSegs];
     int n_segs, rows, K;      // rows: of all segments
+    int *outliers;            // set where some row is not carried well
 };
 
 __global__ void __launch_bounds__(256) split_rows_kernel(const SplitRowsParams p)
@@ -78,8 +82,11 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const SplitRowsParams p
     const int e = mx == 0 ? 0 : min(126, max(-126, 13 - ((mx >> 23) - 127)));
     const float scale = __int_as_float((e + 127) << 23);
     if (lane == 0) s.inv[row] = __int_as_float((127 - e) << 23);
+    int small = 0;                                // elements that keep fewer than 22 bits
+    auto is_small = [](float v) { return v != 0.f && fabsf(v) < 0.125f; };
     auto put = [&](int k, float4 v) {
         v.x *= scale; v.y *= scale; v.z *= scale; v.w *= scale;
+        small += (int)is_small(v.x) + (int)is_small(v.y) + (int)is_small(v.z) + (int)is_small(v.w);
         const __half2 h01 = __floats2half2_rn(v.x, v.y), h23 = __floats2half2_rn(v.z, v.w);
         const float2 b01 = __half22float2(h01), b23 = __half22float2(h23);
         const __half2 l01 = __floats2half2_rn(v.x - b01.x, v.y - b01.y), l23 = __floats2half2_rn(v.z - b23.x, v.w - b23.y);
@@ -95,6 +102,8 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const SplitRowsParams p
         if (k < p.K) put(k, keep[i]);
     }
     for (int k = 1024 + lane * 4; k < p.K; k += 128) put(k, load(k));
+    small = __reduce_add_sync(0xffffffffu, small);
+    if (lane == 0 && small > p.K / 16) atomicOr(p.outliers, 1);
 }
 
 // ------------------------------------------------------------------ GEMM
@@ -103,6 +112,8 @@ struct GemmX3Problem {
     const float *bias;                     // optional [N]
     void *out;                             // [M, N], or [M / S, heads, S, N / heads] when heads > 0
     int M, S, heads;
+    const float *x, *w;                    // the operands as they were: [M, K] or [M / S, x_heads, S, K / x_heads], [N, K]
+    int x_heads;
     int w_row;                             // first row of this problem's W inside the W map
     int first_tile, tiles_n;
 };
@@ -110,8 +121,18 @@ struct GemmX3Params {
     GemmX3Problem prob[3];
     int n_probs, n_tiles, N, K;
     int out_f16;
+    const int *outliers;                   // the split passes' flag
     int *status;
 };
+// Which of the products a tile belongs to
+__device__ __forceinline__ int problem_of(const GemmX3Params &p, int tile)
+{
+    int i = 0;
+    if (p.n_probs > 1 && tile >= p.prob[1].first_tile) i = 1;
+    if (p.n_probs > 2 && tile >= p.prob[2].first_tile) i = 2;
+    return i;
+}
+
 struct GemmX3Maps {
     CUtensorMap xh[3], xl[3], wh, wl;
 };
@@ -132,6 +153,30 @@ struct GemmX3Cfg {
     static_assert(SMEM_BYTES <= 232448, "more than the 227 KB a CTA may have");
 };
 
+// This CTA's tiles from the fp32 operands, where some row's halves would not do.  A function of its own: inside the kernel
+// its code cost the ordinary path 13 us a launch (B4 S1024 E1024: 78 -> 92 and 29 -> 44 us).
+template <class Cfg>
+__device__ __noinline__ void gemm_exact_tiles(const GemmX3Params &p, uint8_t *smem)
+{
+    auto a_s = reinterpret_cast<float (*)[LIN_BM + 4]>(smem);
+    auto w_s = reinterpret_cast<float (*)[LIN_BN + 4]>(smem + LIN_BK * (LIN_BM + 4) * sizeof(float));
+    for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
+        const GemmX3Problem &pr = p.prob[problem_of(p, tile)];
+        const int local = tile - pr.first_tile;
+        LinearParams lp;
+        lp.x = pr.x; lp.w = pr.w; lp.bias = pr.bias; lp.out = nullptr;
+        lp.B = pr.M / pr.S; lp.S = pr.S; lp.K = p.K; lp.N = p.N; lp.heads_in = pr.x_heads; lp.heads_out = pr.heads;
+        for (int m = 0; m < Cfg::BM; m += LIN_BM)
+            for (int n = 0; n < Cfg::BN; n += LIN_BN)
+                linear_simt_tile(lp, local / pr.tiles_n * Cfg::BM + m, local % pr.tiles_n * Cfg::BN + n, threadIdx.x, a_s, w_s,
+                                 [&](int64_t row, int64_t col, float v) {
+                                     const int64_t at = lin_index(row, col, lp.S, lp.N, lp.heads_out);
+                                     if (p.out_f16) static_cast<__half *>(pr.out)[at] = __float2half_rn(v);
+                                     else static_cast<float *>(pr.out)[at] = v;
+                                 });
+    }
+}
+
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
 gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ GemmX3Params p)
@@ -144,13 +189,6 @@ gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ 
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + Cfg::OFF_ABORT);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int k_stages = (p.K + BK - 1) / BK, chunks = (k_stages + Cfg::CHUNK - 1) / Cfg::CHUNK;
-
-    auto problem_of = [&](int tile) {
-        int i = 0;
-        if (p.n_probs > 1 && tile >= p.prob[1].first_tile) i = 1;
-        if (p.n_probs > 2 && tile >= p.prob[2].first_tile) i = 2;
-        return i;
-    };
 
     if (tid == 0) {
         *abort_flag = 0;
@@ -177,6 +215,16 @@ gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ 
     const bool run = *abort_flag == 0;
     ptx::grid_trigger();
     ptx::grid_wait();                                                     // the split pass; the start above ran under its end
+    if (*reinterpret_cast<const volatile int *>(p.outliers) != 0) {
+        gemm_exact_tiles<Cfg>(p, smem);
+        ptx::tc_fence_before_sync();
+        __syncthreads();
+        if (warp == 1) {
+            ptx::tc_fence_after_sync();
+            ptx::tmem_dealloc(tmem, Cfg::TMEM_COLS);
+        }
+        return;
+    }
 
     if (warp < 4) {
     ptx::setmaxnreg_dec<Cfg::REGS_LIGHT>();
@@ -186,7 +234,7 @@ gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ 
             bool ok = true;
             int n = 0;                                                    // stages so far, over all tiles
             for (int tile = blockIdx.x; tile < p.n_tiles && ok; tile += gridDim.x) {
-                const int i = problem_of(tile), local = tile - p.prob[i].first_tile;
+                const int i = problem_of(p, tile), local = tile - p.prob[i].first_tile;
                 const int m0 = local / p.prob[i].tiles_n * BM, n0 = p.prob[i].w_row + local % p.prob[i].tiles_n * BN;
                 for (int j = 0; j < k_stages && ok; ++j, ++n) {
                     const int s = n % NS;
@@ -279,7 +327,7 @@ gemm_x3_kernel(const __grid_constant__ GemmX3Maps maps, const __grid_constant__ 
             if (!ok) break;
             // result: 32 rows x 32 columns at a time through shared memory (16-byte pieces at piece ^ (row & 7)), then
             // eight lanes store 128 bytes of one row
-            const GemmX3Problem &pr = p.prob[problem_of(tile)];
+            const GemmX3Problem &pr = p.prob[problem_of(p, tile)];
             const int local = tile - pr.first_tile;
             const int row0 = local / pr.tiles_n * BM + quarter * 32, col0 = local % pr.tiles_n * BN + half * HALF;
             // The result is sum * inv_x * inv_w + bias; the factor below 1 comes first where the other one is above, so that

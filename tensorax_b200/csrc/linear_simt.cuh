@@ -35,37 +35,43 @@ __device__ __forceinline__ int64_t lin_index(int64_t m, int64_t c, int64_t S, in
     return ((b * heads + c / dh) * S + s) * dh + c % dh;
 }
 
-__global__ void __launch_bounds__(LIN_THREADS) linear_simt_kernel(const LinearParams p)
+// One 64 x 64 tile of x W^T: `store(m, n, value)` for every element inside.  All threads of the CTA call it, the first
+// LIN_THREADS of them work.
+template <class Store>
+__device__ __forceinline__ void linear_simt_tile(const LinearParams &p, int64_t m0, int64_t n0, int tid, float (*a_s)[LIN_BM + 4],
+                                                 float (*w_s)[LIN_BN + 4], Store store)
 {
-    __shared__ float a_s[LIN_BK][LIN_BM + 4];
-    __shared__ float w_s[LIN_BK][LIN_BN + 4];
-    const int tid = threadIdx.x;
     const int64_t M = p.B * p.S;
-    const int64_t m0 = (int64_t)blockIdx.y * LIN_BM, n0 = (int64_t)blockIdx.x * LIN_BN;
+    const bool works = tid < LIN_THREADS;
     const int tx = tid & 15, ty = tid >> 4;          // 16 x 16 threads, 4 x 4 outputs each
     float acc[4][4] = {};
     for (int64_t k0 = 0; k0 < p.K; k0 += LIN_BK) {
         // tile loads: thread -> (row = tid / 4, four consecutive k)
+        if (works) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int row = tid >> 2, kk = (tid & 3) * 4 + i;
-            const int64_t m = m0 + row, n = n0 + row, k = k0 + kk;
-            a_s[kk][row] = (m < M && k < p.K) ? __ldg(p.x + lin_index(m, k, p.S, p.K, p.heads_in)) : 0.f;
-            w_s[kk][row] = (n < p.N && k < p.K) ? __ldg(p.w + n * p.K + k) : 0.f;
+            for (int i = 0; i < 4; ++i) {
+                const int row = tid >> 2, kk = (tid & 3) * 4 + i;
+                const int64_t m = m0 + row, n = n0 + row, k = k0 + kk;
+                a_s[kk][row] = (m < M && k < p.K) ? p.x[lin_index(m, k, p.S, p.K, p.heads_in)] : 0.f;
+                w_s[kk][row] = (n < p.N && k < p.K) ? __ldg(p.w + n * p.K + k) : 0.f;
+            }
         }
         __syncthreads();
+        if (works) {
 #pragma unroll
-        for (int kk = 0; kk < LIN_BK; ++kk) {
-            float a[4], b[4];
+            for (int kk = 0; kk < LIN_BK; ++kk) {
+                float a[4], b[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { a[i] = a_s[kk][ty * 4 + i]; b[i] = w_s[kk][tx * 4 + i]; }
+                for (int i = 0; i < 4; ++i) { a[i] = a_s[kk][ty * 4 + i]; b[i] = w_s[kk][tx * 4 + i]; }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+                for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+            }
         }
         __syncthreads();
     }
+    if (!works) return;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int64_t m = m0 + ty * 4 + i;
@@ -73,11 +79,17 @@ __global__ void __launch_bounds__(LIN_THREADS) linear_simt_kernel(const LinearPa
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int64_t n = n0 + tx * 4 + j;
-            if (n >= p.N) continue;
-            const float v = p.bias ? acc[i][j] + __ldg(p.bias + n) : acc[i][j];
-            p.out[lin_index(m, n, p.S, p.N, p.heads_out)] = v;
+            if (n < p.N) store(m, n, p.bias ? acc[i][j] + __ldg(p.bias + n) : acc[i][j]);
         }
     }
+}
+
+__global__ void __launch_bounds__(LIN_THREADS) linear_simt_kernel(const LinearParams p)
+{
+    __shared__ float a_s[LIN_BK][LIN_BM + 4];
+    __shared__ float w_s[LIN_BK][LIN_BN + 4];
+    linear_simt_tile(p, (int64_t)blockIdx.y * LIN_BM, (int64_t)blockIdx.x * LIN_BN, threadIdx.x, a_s, w_s,
+                     [&](int64_t m, int64_t n, float v) { p.out[lin_index(m, n, p.S, p.N, p.heads_out)] = v; });
 }
 
 }  // namespace txb

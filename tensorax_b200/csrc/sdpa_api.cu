@@ -1014,7 +1014,7 @@ int mha_launch(const tx_mha_desc *d)
     const size_t o_wh = take((size_t)(4 * E * E) * 2), o_wl = take((size_t)(4 * E * E) * 2), o_wi = take((size_t)(4 * E) * 4);
     const size_t es = f16 ? 2 : 4;
     const size_t o_p[3] = {take((size_t)(Mq * E) * es), take((size_t)(Mk * E) * es), take((size_t)(Mk * E) * es)};
-    const size_t o_a = take((size_t)(Mq * E) * 4), o_range = take(3 * sizeof(int));
+    const size_t o_a = take((size_t)(Mq * E) * 4), o_range = take(4 * sizeof(int));
     // the attention result's halves go where the inputs' were (none is needed any more and Q's are as large)
     const size_t o_ah = o_xh[0], o_al = o_xl[0], o_ai = o_xi[0];
 
@@ -1024,9 +1024,9 @@ int mha_launch(const tx_mha_desc *d)
     auto float_at = [&](size_t at) { return reinterpret_cast<float *>(ws + at); };
     auto body = [&]() -> int {
         txb::SplitRowsParams sp;
-        int *range = reinterpret_cast<int *>(ws + o_range);              // of the attention step
-        TX_CUDA(cudaMemsetAsync(range, 0, 3 * sizeof(int), st));
-        sp.n_segs = 0; sp.rows = 0; sp.K = (int)E;
+        int *range = reinterpret_cast<int *>(ws + o_range), *outliers = range + 3;     // of the attention step, of the projections
+        TX_CUDA(cudaMemsetAsync(range, 0, 4 * sizeof(int), st));
+        sp.n_segs = 0; sp.rows = 0; sp.K = (int)E; sp.outliers = outliers;
         auto add = [&](const float *src, size_t hi, size_t lo, size_t inv, int64_t rows, int64_t first_row, int heads, int64_t S) {
             txb::SplitRowsSeg &s = sp.seg[sp.n_segs++];
             s.x = src; s.hi = half_at(hi) + first_row * E; s.lo = half_at(lo) + first_row * E; s.inv = float_at(inv) + first_row;
@@ -1042,12 +1042,12 @@ int mha_launch(const tx_mha_desc *d)
         TX_CUDA(cudaGetLastError());
 
         txb::GemmX3Params g;
-        g.N = g.K = (int)E; g.status = status; g.out_f16 = f16 ? 1 : 0; g.n_probs = 3;
+        g.N = g.K = (int)E; g.status = status; g.out_f16 = f16 ? 1 : 0; g.n_probs = 3; g.outliers = outliers;
         const __half *xh[3], *xl[3];
         for (int i = 0; i < 3; ++i) {
             xh[i] = half_at(o_xh[i]); xl[i] = half_at(o_xl[i]);
             g.prob[i] = {float_at(o_xi[i]), float_at(o_wi) + i * E, bias[i], ws + o_p[i], (int)M[i], (int)seq[i], (int)d->heads,
-                         (int)(i * E), 0, 0};
+                         x[i], w[i], 0, (int)(i * E), 0, 0};
         }
         if (int rc = launch_gemm_x3(g, xh, xl, half_at(o_wh), half_at(o_wl), 3 * E, st)) return rc;
 
@@ -1071,7 +1071,7 @@ int mha_launch(const tx_mha_desc *d)
         if (int rc = launch_behind(txb::split_rows_kernel, split_grid(), 256, 0, st, 1, sp)) return rc;
         g.n_probs = 1; g.out_f16 = 0;
         g.prob[0] = {float_at(o_ai), float_at(o_wi) + 3 * E, d->bo, d->out, (int)Mq, (int)d->seq_q, 0,
-                     0, 0, 0};
+                     float_at(o_a), d->wo, (int)d->heads, 0, 0, 0};
         xh[0] = half_at(o_ah); xl[0] = half_at(o_al);
         return launch_gemm_x3(g, xh, xl, half_at(o_wh) + 3 * E * E, half_at(o_wl) + 3 * E * E, E, st);
     };

@@ -96,3 +96,42 @@ def test_products_in_range_of_operands_near_its_ends(a, b):
     got = mha(ts.Tensor(q, device="cuda"), ts.Tensor(q[:, :1].copy(), device="cuda"), ts.Tensor(x, device="cuda")).numpy()
     ref = x.astype(np.float64) @ w.astype(np.float64).T @ params["out_weight"].astype(np.float64).T
     assert np.linalg.norm(got - ref) <= 2e-6 * np.linalg.norm(np.broadcast_to(ref, got.shape))
+
+
+@pytest.mark.parametrize("E,H,Sq,Sk", [(72, 3, 70, 70), (256, 4, 130, 65), (1088, 17, 33, 40)])
+def test_outliers_inside_a_row(E, H, Sq, Sk):
+    """Elements far below their row's largest, which the weights leave out: the projections see the small ones alone.  Float64
+    reference of the layer with one key per query row's batch element left visible; bound: fp32 sums over E, twice."""
+    mha, params = layer(E, H, True)
+    w = params["v_weight"].copy()
+    w[:, 0] = 0
+    mha._parameters["v_weight"] = ts.Tensor(w, device="cuda")
+    x, y, z = seeded(9, 2, Sq, E), seeded(10, 2, Sk, E), seeded(11, 2, Sk, E)
+    z[..., 0] = 1e9
+    got = mha(*(ts.Tensor(t, device="cuda") for t in (x, y, z)), kv_lens=[1, 1]).numpy()
+    v0 = z[:, :1].astype(np.float64) @ w.astype(np.float64).T + params["v_bias"]
+    ref = np.broadcast_to(v0 @ params["out_weight"].astype(np.float64).T + params["out_bias"], got.shape)
+    assert np.linalg.norm(got - ref) <= 5e-6 * np.linalg.norm(ref)
+
+
+def test_outliers_in_the_weights_and_in_the_attention_result():
+    """Whole weight rows of small numbers beside one large one that the input leaves out, and a head of the attention result
+    far above all others that the output weights leave out (fp32 and fp16 attention results of the layer alike)."""
+    E, H, S = 128, 4, 60
+    mha, params = layer(E, H, False)
+    x = seeded(14, 2, S, E)
+    x[..., 5] = 0
+    w = params["v_weight"].copy()
+    w[:, 5] = 1e9
+    mha._parameters["v_weight"] = ts.Tensor(w, device="cuda")
+    got = mha(*(ts.Tensor(x, device="cuda"),) * 3).numpy()
+    ref = oracle.mha_forward_f32(x, x, x, dict(params, v_weight=w), H, None)
+    assert np.linalg.norm(got - ref) <= 1e-5 * np.linalg.norm(ref)
+    mha, params = layer(E, H, False)
+    w, o = params["v_weight"].copy(), params["out_weight"].copy()
+    w[:32] *= np.float32(1e9)
+    o[:, :32] = 0
+    mha._parameters["v_weight"], mha._parameters["out_weight"] = ts.Tensor(w, device="cuda"), ts.Tensor(o, device="cuda")
+    got = mha(*(ts.Tensor(x, device="cuda"),) * 3).numpy()
+    ref = oracle.mha_forward_f32(x, x, x, dict(params, v_weight=w, out_weight=o), H, None)
+    assert np.linalg.norm(got - ref) <= 1e-5 * np.linalg.norm(ref)
