@@ -66,7 +66,10 @@ struct DecodeCfg {
     static constexpr uint32_t OFF_ABORT = OFF_BAR + 2 * NS * 8;
     static constexpr uint32_t OFF_ML = OFF_ABORT + 16;                   // float [WARPS + 1][R][2]: warps, then the CTA
     static constexpr uint32_t SMEM = OFF_ML + (WARPS + 1) * R * 8;
-    static constexpr int THREADS = (WARPS + 1) * 32, CTAS_PER_SM = 2, MAX_SPLITS = 16;
+    static constexpr int THREADS = (WARPS + 1) * 32, MAX_SPLITS = 16;
+    // CTAs an SM holds (228 KB, 1 KB of it per CTA taken): one in fp32 at d = 128 and 256 with up to two rows.  Counting on two
+    // there cut the keys into two waves of clusters: B4 Hkv8 Sk1000 d128 24.6 us, 16.4 with one; B9 Hkv8 Sk4096 75.8 and 66.7.
+    static constexpr int CTAS_PER_SM = 2 * (SMEM + 1024) <= 233472 ? 2 : 1;
     static_assert(R == 1 || R == 2 || R == 4, "more rows are shared out over CTAs (eight in one: slower at every size)");
     static_assert(LPK >= 8 && LPK <= 32 && NV >= 1 && NV * VEC == EPL, "lane layout");
     static_assert(MERGE <= RING, "partial results are merged in the drained ring");
@@ -96,7 +99,7 @@ __device__ __forceinline__ constexpr int dec_reverse(int x)
 }
 
 template <class Cfg>
-__global__ void __launch_bounds__(Cfg::THREADS, Cfg::CTAS_PER_SM)
+__global__ void __launch_bounds__(Cfg::THREADS, 2)
 sdpa_decode_kernel(const DecodeParams p)
 {
     using T = typename Cfg::T;
