@@ -590,7 +590,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
 // Bound: HBM.  One CTA takes 64 rows of Q (a factor each) or a 64-key tile of K or V, all of it in registers between the
 // maximum and the scaling.  Four lanes share a row, each with every fourth group of eight elements: a row's maximum is two
 // shuffles away, and a CTA is small enough for the whole launch to be one wave (with 8, 16 or 32 lanes a row, up to eight
-// rows a thread, B2 H8 S1000 d80 took 11.5 us and B4 H16 S1024 d64 23; now 7.2 and 16.1).
+// rows a thread, B2 H8 S1000 d80 took 11.5 us and B4 H16 S1024 d64 23; now 7.2 and 14.7; eight CTAs an SM at d = 64 spill: 15.9).
 struct SplitSeg {
     const float *x;
     __half *hi, *lo;
@@ -605,7 +605,7 @@ struct SplitParams {
 };
 
 template <int N>              // groups of eight a lane, 4 N at least p8
-__global__ void __launch_bounds__(256, N <= 2 ? 8 : 5) split_f32_hi_lo_kernel(const SplitParams sp)
+__global__ void __launch_bounds__(256, N == 1 ? 8 : N == 2 ? 6 : 5) split_f32_hi_lo_kernel(const SplitParams sp)
 {
     ptx::grid_trigger();
     constexpr int kInf = 0x7f800000;
