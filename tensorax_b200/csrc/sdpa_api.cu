@@ -646,23 +646,38 @@ int launch_f16(const tx_sdpa_desc *d, cudaStream_t st, int *status)
     return decode_eligible(d) ? launch_decode<__half>(d, st, status) : launch_tc(d, st, status);
 }
 
-// CTAs per work item of a backward kernel: `items` items, the longest of `longest` tiles and `mean` on average, on `sms`
-// multiprocessors of `per_sm` CTAs (two on one get through half as much again as one does).  Time in tiles, a CTA's start
-// and end counting as three, five with the sum over the cluster: the longest CTA, or all of them spread over the places, in
-// whole waves where the items are equal.  An item is cut (in two, four or eight, a cluster) where that shortens the launch
-// by a fifth or more; a CTA keeps two tiles at least.  B2 Hq12 Hkv4 S921 d64 causal: the dK/dV kernel 79 us uncut, 28 us
-// in four, 36 us in eight; the dQ kernel 19 us uncut, 22 us in two.
-int bwd_split(double items, double longest, double mean, int sms, int per_sm)
+// One kernel of the backward as its launch sees it: items, tiles of the longest and of the mean one, the time of a tile.
+struct BwdWork {
+    double items, longest, mean, tile;
+};
+
+// CTAs per work item of a backward kernel on `sms` multiprocessors of `per_sm` CTAs (two on one get through half as much
+// again as one does).  Time in tiles, a CTA's start and end counting as three, five with the sum over the cluster: the longest
+// CTA, or all of them spread over the places, in whole waves where the items are equal.  An item is cut (in two, four or
+// eight, a cluster) where that shortens the launch by a fifth or more; a CTA keeps two tiles at least.  B2 Hq12 Hkv4 S921
+// d64 causal: the dK/dV kernel 67 us uncut, 42 us in two, 28 us in four, 35 us in eight; the dQ kernel 20 us uncut, 22 in two.
+int bwd_split(const BwdWork &w, int sms, int per_sm)
 {
     const double places = per_sm == 2 ? 1.5 * sms : (double)sms;
     auto cost = [&](int z) {
-        const double fixed = z > 1 ? 5.0 : 3.0, one = std::ceil(longest / z) + fixed, waves = items * z / places;
-        return std::max(one, mean < longest ? waves * (mean / z + fixed) : std::ceil(waves) * one);
+        const double fixed = z > 1 ? 5.0 : 3.0, one = std::ceil(w.longest / z) + fixed, waves = w.items * z / places;
+        return std::max(one, w.mean < w.longest ? waves * (w.mean / z + fixed) : std::ceil(waves) * one);
     };
     int best = 1;
-    for (int z = 2; z <= 8 && longest >= 2.0 * z; z *= 2)
+    for (int z = 2; z <= 8 && w.longest >= 2.0 * z; z *= 2)
         if (cost(z) < 0.8 * cost(best)) best = z;
     return best;
+}
+
+// Both kernels as they run, the dK/dV kernel beside the dQ kernel's CTAs wherever those leave an SM free (one CTA each):
+// all the work spread over the SMs, or the longest dK/dV CTA behind the dQ CTAs that go before it, or the longest dQ CTA.
+double bwd_together(const BwdWork &q, int zq, const BwdWork &k, int zk, int sms)
+{
+    auto share = [](const BwdWork &w, int z, double tiles) { return (tiles / z + (z > 1 ? 5.0 : 2.0)) * w.tile; };
+    auto chain = [&](const BwdWork &w, int z) { return share(w, z, z * std::ceil(w.longest / z)); };
+    const double q1 = share(q, zq, q.mean), k1 = share(k, zk, k.mean);
+    const double work = (q.items * zq * q1 + k.items * zk * k1) / sms, behind = std::max(0.0, q.items * zq / sms - 1.0) * q1;
+    return std::max({work, behind + chain(k, zk), chain(q, zq)});
 }
 
 template <int D, class DqCfg, class DkvCfg>
@@ -682,6 +697,22 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
     int sms = 0;
     if (int rc = sm_count(&sms)) return rc;
     {
+        auto up = [](int64_t n, int64_t by) { return (double)((n + by - 1) / by); };
+        const double ratio = (double)(d->q_heads / d->kv_heads), tq = up(d->seq_k, DqCfg::BN), tk = up(d->seq_q, DkvCfg::BQ) * ratio;
+        // a dK/dV tile against a dQ tile, one CTA per SM: 1.2 and 1.7 us at d = 128, 1.8 and 2.2 at d = 256
+        const BwdWork q = {up(d->seq_q, DqCfg::BM) * (double)(d->batch * d->q_heads), tq, d->causal ? 0.5 * (tq + 1) : tq, 1.0};
+        const BwdWork k = {up(d->seq_k, DkvCfg::BMK) * (double)(d->batch * d->kv_heads * DkvCfg::ZS), tk, d->causal ? 0.5 * (tk + ratio) : tk,
+                           D == 128 ? 0.7 : 0.82};
+        p.split_q = bwd_split(q, sms, DqCfg::CTAS_PER_SM);
+        p.split_k = bwd_split(k, sms, DkvCfg::CTAS_PER_SM);
+        // Each kernel alone gains by that; together, uncut, they may fill the chip as it is.  B1 H8 S1000 d256 causal: kernels
+        // of 41 + 59 us uncut and 29 + 51 in two, the call 72 and 78; B1 H4 S2048 d128 32 + 42 and 22 + 30, the call 51.5 and
+        // 55.6.  (58 shapes measured with every pair of cuts: none slower than uncut by this, four by up to 9 % without it.)
+        if (DqCfg::CTAS_PER_SM == 1 && p.split_q * p.split_k > 1 &&
+            bwd_together(q, p.split_q, k, p.split_k, sms) >= 0.9 * bwd_together(q, 1, k, 1, sms))
+            p.split_q = p.split_k = 1;
+    }
+    {
         CUtensorMap tq, tdo, tk, tv;
         if (int rc = make_map(&tq, d->q, d->batch * d->q_heads, d->seq_q, D, DqCfg::BM)) return rc;
         if (int rc = make_map(&tdo, dout_h, d->batch * d->q_heads, d->seq_q, D, DqCfg::BM)) return rc;
@@ -696,8 +727,6 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
         if (int rc = launch_group(d->causal != 0, slabs, items, 4.0 * (double)d->seq_k * (double)D / (double)ratio, ratio, &group, 32))
             return rc;
         p.group_q = (int)group; p.items_q = (int)items; p.slabs_q = (int)slabs;
-        const double tiles = (double)((d->seq_k + DqCfg::BN - 1) / DqCfg::BN);
-        p.split_q = bwd_split((double)(items * slabs), tiles, d->causal ? 0.5 * (tiles + 1) : tiles, sms, DqCfg::CTAS_PER_SM);
         if (items * slabs * p.split_q > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA backward: more than 2^31 work items");
         if (int rc = launch_behind(txb::sdpa_bwd_dq_kernel<DqCfg>, dim3((unsigned)(items * slabs * p.split_q)), DqCfg::THREADS,
                                    DqCfg::SMEM_BYTES, st, p.split_q, tq, tdo, tk, tv, p))
@@ -718,9 +747,6 @@ int launch_bwd(const tx_sdpa_bwd_desc *d, cudaStream_t st, int *status, const __
         if (int rc = launch_group(d->causal != 0, slabs, items * DkvCfg::ZS, 4.0 * (double)ratio * (double)d->seq_q * (double)D, 1, &group, 32))
             return rc;
         p.group_k = (int)group; p.items_k = (int)items; p.slabs_k = (int)slabs;
-        const double tiles = (double)((d->seq_q + DkvCfg::BQ - 1) / DkvCfg::BQ * ratio);
-        p.split_k = bwd_split((double)(items * slabs * DkvCfg::ZS), tiles, d->causal ? 0.5 * (tiles + ratio) : tiles,
-                              sms, DkvCfg::CTAS_PER_SM);
         const int64_t ctas = items * slabs * DkvCfg::ZS * p.split_k;
         if (ctas > 0x7fffffffLL) return fail(TX_ERR_UNSUPPORTED, "SDPA backward: more than 2^31 work items");
         if (int rc = launch_behind(txb::sdpa_bwd_dkv_kernel<DkvCfg>, dim3((unsigned)ctas), DkvCfg::THREADS, DkvCfg::SMEM_BYTES, st,
