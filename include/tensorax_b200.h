@@ -76,6 +76,8 @@ TX_API int tx_cuda_set_device(int device);
  * cached in the pool (the reference pays a cudaMalloc/cudaFree pair per output tensor) */
 TX_API void *tx_cuda_malloc(size_t bytes);            /* NULL on failure */
 TX_API int tx_cuda_free(void *ptr);
+/* Blocks come from the device's stream-ordered pool.  Of what has been freed it keeps up to 4 GiB (5 with rounding) beyond what
+ * the program holds; the rest goes back to the driver at the next synchronise, all of it with tx_cuda_pool_trim. */
 /* tx_cuda_malloc / tx_cuda_free are ordered on the legacy default stream: safe with work on stream NULL and on
  * ordinary (blocking) streams, which synchronise with it.  A buffer last used by a kernel on a cudaStreamNonBlocking
  * stream must be freed with tx_cuda_free_on(ptr, that_stream) (or after synchronising that stream): the block then

@@ -65,7 +65,7 @@ def test_the_kernels_use_that_rule():
     """Every mbarrier wait goes through ptx::mbar_wait, which is bounded_wait with the PTX probes."""
     ptx = open(os.path.join(ROOT, "tensorax_b200", "csrc", "ptx.cuh")).read()
     assert '#include "bounded_wait.h"' in ptx and "return bounded_wait(" in ptx
-    for name in ("sdpa_tc.cuh", "sdpa_tc_pair.cuh", "sdpa_bwd.cuh", "linear_tc.cuh"):
+    for name in ("sdpa_tc.cuh", "sdpa_tc_pair.cuh", "sdpa_tc_x3.cuh", "sdpa_decode.cuh", "sdpa_bwd.cuh", "linear_tc.cuh", "gemm_x3.cuh"):
         text = open(os.path.join(ROOT, "tensorax_b200", "csrc", name)).read()
         assert "mbar_wait(" in text
         assert "__trap" not in text and "assert(" not in text.replace("static_assert(", "")

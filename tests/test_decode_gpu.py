@@ -18,7 +18,7 @@ CASES = [
     (1, 9, 1, 1, 4097, False, None, False),               # one row more than a row group
     (2, 4, 4, 1, 300, False, None, True),                 # the reference's padding-mask form
     (1, 2, 1, 3, 200, True, None, False),                 # several rows per head, causal
-    (40, 8, 4, 1, 333, False, "ramp", False),             # more lengths than travel with a launch
+    (40, 8, 4, 1, 333, False, "ramp", False),             # lengths on the device; from the host: test_kv_lens_host_gpu.py
 ]
 
 
