@@ -104,7 +104,7 @@ TX_API int tx_host_free_pinned(void *ptr);
  *      the reference's sdpa_cpu on unit-variance inputs, the figure of the exact kernel; 3e-5 at scores of +-100, where the
  *      exact kernel itself is at 1e-5).  Rows of Q and 64-key tiles of K and V are scaled by powers of two first, so magnitudes
  *      do not matter.  A device-side check sends a call to the exact CUDA-core kernel, which also takes every other shape,
- *      where scaling does not help: a value that is not finite, max |Q| * max |K| above 2^19, or a tile of V whose keys'
+ *      where scaling does not help: a value that is not finite, max |Q| * max |K| above 2^19, or keys of one head's V whose
  *      largest elements are more than 2^13 apart.  Calls with few query rows per K/V head take
  *      the decoding kernel (exact fp32 products). */
 TX_API int tx_sdpa_naive_cuda(const float *Q, const float *K, const float *V, const float *mask,

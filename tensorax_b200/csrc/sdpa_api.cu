@@ -835,7 +835,7 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status, int *zeroed
     auto take = [&](int64_t bytes) { const size_t at = total; total += align_up((size_t)bytes, 256); return at; };
     const size_t o_qh = take(rows_q * dk8 * 2), o_ql = take(rows_q * dk8 * 2), o_kh = take(rows_k * dk8 * 2), o_kl = take(rows_k * dk8 * 2),
                  o_vh = take(rows_k * dv8 * 2), o_vl = take(rows_k * dv8 * 2);
-    const size_t o_qf = take(rows_q * 4), o_kf = take(slabs_k * tiles_k * 4), o_vf = take(slabs_k * tiles_k * 4), o_range = take(3 * sizeof(int));
+    const size_t o_qf = take(rows_q * 4), o_kf = take(slabs_k * tiles_k * 4), o_vf = take(slabs_k * tiles_k * 4), o_vr = take(slabs_k * tiles_k * 4), o_range = take(3 * sizeof(int));
     char *ws = nullptr;
     if (int rc = pool_alloc(&ws, total, st)) return rc;
     auto float_at = [&](size_t at) { return reinterpret_cast<float *>(ws + at); };
@@ -846,7 +846,7 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status, int *zeroed
         txb::SplitParams sp;
         auto seg = [&](int i, const void *x, size_t hi, size_t lo, size_t factor, int64_t S, int64_t tiles, int64_t first, int64_t n, int64_t n8) {
             sp.seg[i] = {static_cast<const float *>(x), reinterpret_cast<__half *>(ws + hi), reinterpret_cast<__half *>(ws + lo),
-                         float_at(factor), (long long)S, (int)tiles, (int)first, (int)(n / 4), (int)(n8 / 8)};
+                         float_at(factor), i == 2 ? reinterpret_cast<int *>(ws + o_vr) : nullptr, (long long)S, (int)tiles, (int)first, (int)(n / 4), (int)(n8 / 8)};
         };
         seg(0, d->q, o_qh, o_ql, o_qf, rows_q, tiles_q, 0, d->d_k, dk8);
         seg(1, d->k, o_kh, o_kl, o_kf, d->seq_k, tiles_k, tiles_q, d->d_k, dk8);
@@ -878,7 +878,7 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status, int *zeroed
         p.mask = d->mask;
         p.kv_lens = lens_of(d->kv_lens, d->flags, d->batch);
         p.range = range;
-        p.qf = float_at(o_qf); p.kf = float_at(o_kf); p.vf = float_at(o_vf);
+        p.qf = float_at(o_qf); p.kf = float_at(o_kf); p.vf = float_at(o_vf); p.vr = reinterpret_cast<const int *>(ws + o_vr);
         p.status = status;
         p.Hq = (int)d->q_heads; p.Hkv = (int)d->kv_heads; p.Sq = (int)d->seq_q; p.Sk = (int)d->seq_k;
         p.dk = (int)d->d_k; p.dv = (int)d->d_v;
@@ -894,7 +894,7 @@ int launch_x3_t(const tx_sdpa_desc *d, cudaStream_t st, int *status, int *zeroed
         if (int r = launch_behind(txb::sdpa_tc_x3_kernel<Cfg>, dim3((unsigned)(n_tiles * sq)), Cfg::THREADS, Cfg::SMEM_BYTES, st, 1,
                                   qh, ql, kh, kl, vh, vl, to, p))
             return r;
-        // the exact kernel behind it: works only when the split pass found a value the fp16 pairs cannot carry
+        // the exact kernel behind it: works only where the fp16 pairs would not do
         txb::SimtParams sp2;
         fill_simt_params(&sp2, d);
         sp2.only_if = range;

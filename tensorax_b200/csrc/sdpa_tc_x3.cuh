@@ -15,7 +15,7 @@
 //   warp 1        issues the MMAs: QK^T of tile j+1 as soon as the softmax warps have S_j in registers, then PV of tile j
 //   warps 2-3     idle, or bring the dense mask's [128 rows][64 keys] tile to shared memory (cp.async: any row length)
 //   warps 4-7     softmax, thread = row = tensor-memory lane: fp32 online softmax with the exact running max
-//                 (full-precision `ex2.approx`, no polynomial), P split into hi / lo in registers and stored to
+//                 (full-precision `ex2.approx`, no polynomial), 2^14 P split into hi / lo in registers and stored to
 //                 tensor memory as two fp16 operands; the row's rescale factor of the tile goes to shared memory
 //   warps 8-11    accumulators, thread = row: O lives in REGISTERS.  Each tile's P V is a fresh tensor-memory
 //                 accumulator (12 MMAs) that these warps fold in with O = O * alpha + PV, rounded to nearest.  The
@@ -77,10 +77,15 @@ struct X3Cfg {
     static_assert(Q_BYTES / 4 >= 4096, "a softmax warp stages its results in its quarter of the Q buffers");
 };
 
-// The split pass's words.  range[0]: some value is not finite, or the largest elements of the rows of one tile of V lie more
-// than 2^13 apart, so that the small rows would keep fewer than 25 bits.  range[1], range[2]: the bits of max |q| and max |k|:
-// what scaling leaves of a row or tile below 2^-39 of its maximum is worth up to 2^-39 max |q| max |k| in a score (sqrt(d)
-// such terms, times 1 / sqrt(d)), which stays below 2^-20 here.
+// P is carried as 2^14 p (p <= 1), so that its pairs too are exact to 2^-39 absolutely and not to 2^-25: keys of small weight
+// and large V count.  The split pass takes the factor out of V's (X3Params::vf).
+constexpr float X3_P_SCALE = 16384.f;
+
+// range[0]: some value is not finite (the split pass), or the largest elements of two keys of a head's V lie more than 2^13
+// apart (this kernel, on its way; the exact kernel then does the whole call once more), so that the rounding of P and V at
+// the large ones would show beside the small ones.  range[1], range[2]: the bits of max |q| and max |k|: what scaling leaves
+// of a row or tile below 2^-39 of its maximum is worth up to 2^-39 max |q| max |k| in a score (sqrt(d) such terms, times
+// 1 / sqrt(d)), which stays below 2^-20 here.
 __device__ __forceinline__ bool x3_declines(const int *range)
 {
     const volatile int *w = range;
@@ -91,9 +96,10 @@ struct X3Params {
     float *out;               // [B,Hq,Sq,dv] fp32
     const float *mask;        // dense additive [B,Hq,Sq,Sk] (MASK instantiations)
     KvLens kv_lens;           // optional [B]
-    const int *range;         // the split pass's three words (see x3_declines)
+    int *range;               // three words (see x3_declines)
     const float *qf;          // [B,Hq,Sq] what undoes the scale of a row of Q
-    const float *kf, *vf;     // [B,Hkv,ceil(Sk / 64)] the same of a tile of K and V
+    const float *kf, *vf;     // [B,Hkv,ceil(Sk / 64)] the same of a tile of K and V (V: and of P)
+    const int *vr;            // [B,Hkv,ceil(Sk / 64)] exponent fields of the largest and the smallest key of a tile of V: max | min << 8
     int *status;              // device word: 0 = ok, else first failing wait's code
     int Hq, Hkv, Sq, Sk;
     int dk, dv;
@@ -376,6 +382,17 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
         float m_run = Cfg::MASK ? -FLT_MAX : -1.0e30f;           // finite stand-in for "no key seen yet"
         float l = 0.f;
         bool ok = run;
+        if (run && warp == 4) {                          // how far V's keys lie apart, while the first tiles are on their way
+            int most = 0, least = 255;
+            for (int j = lane; j < nt; j += 32) {
+                const int f = p.vr[f0 + j];
+                most = max(most, f & 255);
+                least = min(least, f >> 8);
+            }
+            most = __reduce_max_sync(0xffffffffu, most);
+            least = __reduce_min_sync(0xffffffffu, least);
+            if (lane == 0 && most - least > 13) atomicOr(p.range, 1);
+        }
         auto arrive_warp = [&](uint32_t bar) {
             ptx::tc_fence_before_sync();
             __syncwarp();
@@ -434,6 +451,7 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
             if (lane == 0) ptx::mbar_arrive(alpha_full + 8 * (j & 3));
             // p = 2^(s*scale - m): a masked score is -inf and gives exactly 0
             const float2 scale2 = make_float2(scale, scale), negm2 = make_float2(-m_next, -m_next);
+            const float2 p_scale2 = make_float2(X3_P_SCALE, X3_P_SCALE);
             float2 sum_a = make_float2(0.f, 0.f), sum_b = make_float2(0.f, 0.f);
             uint32_t pkh[BN / 2], pkl[BN / 2];
 #pragma unroll
@@ -447,9 +465,10 @@ sdpa_tc_x3_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_consta
                 const float2 eb = make_float2(ptx::ex2_approx(xb.x), ptx::ex2_approx(xb.y));
                 sum_a = __fadd2_rn(sum_a, ea);
                 sum_b = __fadd2_rn(sum_b, eb);
-                const __half2 ha = __floats2half2_rn(ea.x, ea.y), hb = __floats2half2_rn(eb.x, eb.y);
+                const float2 pa = __fmul2_rn(ea, p_scale2), pb = __fmul2_rn(eb, p_scale2);
+                const __half2 ha = __floats2half2_rn(pa.x, pa.y), hb = __floats2half2_rn(pb.x, pb.y);
                 const float2 ba = __half22float2(ha), bb = __half22float2(hb);
-                const __half2 la = __floats2half2_rn(ea.x - ba.x, ea.y - ba.y), lb = __floats2half2_rn(eb.x - bb.x, eb.y - bb.y);
+                const __half2 la = __floats2half2_rn(pa.x - ba.x, pa.y - ba.y), lb = __floats2half2_rn(pb.x - bb.x, pb.y - bb.y);
                 pkh[i / 2] = *reinterpret_cast<const uint32_t *>(&ha);
                 pkh[i / 2 + 1] = *reinterpret_cast<const uint32_t *>(&hb);
                 pkl[i / 2] = *reinterpret_cast<const uint32_t *>(&la);
@@ -595,6 +614,7 @@ struct SplitSeg {
     const float *x;
     __half *hi, *lo;
     float *factor;            // Q: [rows], K and V: [tiles]
+    int *fields;              // V: [tiles], see X3Params::vr
     long long S;              // rows of a slab, cut into `tiles` tiles (Q: all rows are one slab)
     int tiles, first;         // `first`: CTAs of the segments before this one
     int q4, p8;               // a row: quads of the source, groups of eight of the padded copy
@@ -640,10 +660,11 @@ __global__ void __launch_bounds__(256, N == 1 ? 8 : N == 2 ? 6 : 5) split_f32_hi
     const int e = min(126, 140 - ((t == 0 ? m : most) >> 23));
     const float scale = __int_as_float((e + 127) << 23), factor = __int_as_float((127 - e) << 23);
     if (threadIdx.x == 0) {
-        if (most >= kInf || (t == 2 && most != 0 && (most >> 23) - (least >> 23) > 13)) atomicOr(sp.range, 1);
+        if (most >= kInf) atomicOr(sp.range, 1);
         if (t == 0) atomicMax(sp.range + 1, most);
         if (t == 1) atomicMax(sp.range + 2, most);
-        if (t > 0) s.factor[tile] = factor;
+        if (t == 1) s.factor[tile] = factor;
+        if (t == 2) { s.factor[tile] = factor / X3_P_SCALE; s.fields[tile] = most >> 23 | (least >> 23) << 8; }
     }
     if (!in) return;
     if (t == 0 && part == 0) s.factor[at] = factor;

@@ -76,6 +76,26 @@ def test_small_head_and_small_tiles_of_v_beside_large_ones(d):
             assert np.linalg.norm(got[b, h] - ref[b, h]) <= 2e-6 * np.sqrt(S) * np.linalg.norm(ref[b, h])
 
 
+@pytest.mark.parametrize("d", [64, 80, 128])
+@pytest.mark.parametrize("f", [30.0, 1500.0, 1e6, 1e15])
+def test_keys_of_small_weight_and_large_values(d, f):
+    """One key of weight 1 and a tile of others whose weights times values still count: 1e-8 * 1500 and the like."""
+    q, k, v = inputs(d, d, 50)
+    q *= np.float32(0.1)
+    v[:, :, 64:128] = np.float32(f) * (2 + v[:, :, 64:128].clip(-1, 1))
+    m = np.full((B, H, S, S), -np.inf, np.float32)
+    m[..., 5] = 0
+    m[..., 64:128] = np.float32(np.log(1e-5 / f))
+    ref = exact64(q, k, v, m)
+    for e in (1.0, 2.0 ** -20):
+        got = sdpa_device(q, k, v * np.float32(e), mask=m)[0]
+        if f < 1e4:
+            assert np.abs(got - ref * e).max() <= 2e-6 * e
+        else:                                                 # too far apart: the exact kernel, with its own bound
+            exact, _ = sdpa_device(q, k, v * np.float32(e), mask=m, flags=_lib.TX_SDPA_FORCE_SIMT)
+            assert np.array_equal(got, exact) and np.abs(got - ref * e).max() <= 1e-5 * e
+
+
 def test_garbage_behind_a_mask_and_mismatched_outliers():
     q, k, v = inputs(80, 80, 30)
     m = np.zeros((B, H, S, S), np.float32)
